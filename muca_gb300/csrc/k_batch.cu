@@ -15,7 +15,7 @@
 // shared memory of the u32 bins for more blocks per SM.  Work is fetched by
 // an atomic counter over items sorted by decreasing cost, so the large
 // lattices start first and the small ones fill the tail.
-#include "sweep_core.cuh"
+#include "window.cuh"
 
 namespace muca {
 
@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(256, 1) k_batch_sweep(const BatchInst *__restr
 {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint32_t s_item;
-    __shared__ float s_btab[17];
+    __shared__ float s_btab[kBetaTab];
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(next_item, 1u);
         __syncthreads();
@@ -53,7 +53,9 @@ __global__ void __launch_bounds__(256, 1) k_batch_sweep(const BatchInst *__restr
         uint32_t iter;
         unsigned long long nup;
         if (launch_params(a, iter, nup)) {  // the instance is still running
-            if (threadIdx.x < 17) s_btab[threadIdx.x] = I->btab[threadIdx.x];
+            // -beta dE by dE + 8, then beta times the neighbour spin sum by code sum
+            if (threadIdx.x < kBetaTab)
+                s_btab[threadIdx.x] = I->btab[threadIdx.x < 17 ? threadIdx.x : 29 - threadIdx.x];
             // s_btab is read only after the block barrier inside the sweep's prologue
             if (LAT == kLatShared) {
                 win_sweep_block<kModeWeight, R, true, HS, true>(a, smem, cpb, item.blk, iter, nup, s_btab);

@@ -36,7 +36,7 @@
 //   k_sweep_win   the same window core with the Philox numbers drawn by the
 //                 chain's own lane, one window ahead;
 //   k_sweep_generic  the reference step by step on the packed layout, any L.
-#include "sweep_core.cuh"
+#include "window.cuh"
 
 #include <algorithm>
 #include <cstring>
@@ -54,10 +54,7 @@ __global__ void __launch_bounds__(256, 1) k_sweep_win(const SweepArgs a, uint32_
     uint32_t iter;
     unsigned long long nup;
     if (!launch_params(a, iter, nup)) return;
-    // with the lattice behind the row ring the scan fetches weights three
-    // attempts ahead (measured faster there, slower with the lattice in
-    // shared memory)
-    win_sweep_block<MODE, R, LAT_SMEM, true, false, RING, RING>(a, smem, cpb, blockIdx.x, iter, nup);
+    win_sweep_block<MODE, R, LAT_SMEM, true, false, RING>(a, smem, cpb, blockIdx.x, iter, nup);
 }
 
 // ---------------------------------------------------------------------------
@@ -260,9 +257,10 @@ __global__ void __launch_bounds__(256, 1) k_sweep_spec(const SweepArgs a, uint32
             return true;
         });
     } else {
-        const bool store = lane < cpb;
+        // lanes without a chain never accept (their E_Delta stays 3)
+        const bool store = cs.active;
         ChainState st;
-        st.E = cs.active ? a.edel[cs.chain] : (store ? 0 : 3);
+        st.E = cs.active ? a.edel[cs.chain] : 3;
         st.EJ = cs.active ? a.ej[cs.chain] : 0;
         st.M = (cs.active && MODE == kModeProduce) ? a.mag[cs.chain] : 0;
         const WT eps = (WT)a.log_eps;
@@ -326,8 +324,10 @@ __global__ void __launch_bounds__(256) k_sweep_generic(const SweepArgs a, uint32
     __syncthreads();
     ChainSetup<MODE, R> cs;
     cs.init(a, cpb, lane, blockIdx.x);
-    const bool store = lane < cpb;
-    int E = cs.active ? a.edel[cs.chain] : 0;
+    // lanes without a chain never accept, so that every weight index of theirs
+    // stays in [2, 4]
+    const bool store = cs.active;
+    int E = cs.active ? a.edel[cs.chain] : 3;
     int EJ = cs.active ? a.ej[cs.chain] : 0;
     int M = (cs.active && MODE == kModeProduce) ? a.mag[cs.chain] : 0;
     uint32_t c0 = 0;
@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(256) k_sweep_generic(const SweepArgs a, uint32
                 diff = __dsub_rn(__dadd_rn((double)(-dE * 2), (double)wS[E + dDel]), (double)wS[E]);
             bool acc = diff >= (WT)0;
             if (!acc) acc = (WT)logf(u01f(pick(r1, sub))) < diff;
-            if (acc) {
+            if (acc && cs.active) {
                 put(idx, ns);
                 EJ += dE;
                 E += dDel;
@@ -404,7 +404,7 @@ __global__ void k_logf_bracket(unsigned int *maxbits)
     unsigned int m = 0;
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < (1u << 23); k += gridDim.x * blockDim.x) {
         const float u = u01f(k << 9);
-        const float e = fabsf(__logf(u) - logf(u));
+        const float e = fabsf(fast_logf(u) - logf(u));
         m = max(m, __float_as_uint(e));
     }
 #pragma unroll
@@ -437,7 +437,7 @@ __global__ void k_table_bracket(const float *tab, unsigned int *maxbits)
     unsigned int m = 0;
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < (1u << 23); k += gridDim.x * blockDim.x) {
         const float u = u01f(k << 9);
-        const float e = fabsf(__logf(u) - tab[k]);
+        const float e = fabsf(fast_logf(u) - tab[k]);
         m = max(m, __float_as_uint(e));
     }
 #pragma unroll
@@ -522,6 +522,8 @@ SweepPlan plan_sweep(int mode, int rounds, uint32_t L, uint32_t nchains, size_t 
             cpb = c;
         }
     }
+    // the windowed kernel stages FP32 values in both modes
+    const size_t front = p.kernel == kKernelWindowed ? win_smem_base(mode, N, true) : base;
     p.cpb = cpb;
     p.blocks = (nchains + cpb - 1) / cpb;
     const uint32_t warps = (cpb + 31u) / 32u;
@@ -529,8 +531,8 @@ SweepPlan plan_sweep(int mode, int rounds, uint32_t L, uint32_t nchains, size_t 
     // a lattice in global memory: the windowed kernel keeps a four-row ring
     // per lane in shared memory when it fits
     p.row_ring = !p.lat_smem && p.kernel == kKernelWindowed && L % 4 == 0 && WPR <= 8 &&
-                 base + ring_bytes(L, cpb) <= optin;
-    p.smem = base + (p.kernel == kKernelSpecialized ? smem_ring_bytes(warps) : 0) +
+                 front + ring_bytes(L, cpb) <= optin;
+    p.smem = front + (p.kernel == kKernelSpecialized ? smem_ring_bytes(warps) : 0) +
              (p.lat_smem ? per_chain * cpb : 0) + (p.row_ring ? ring_bytes(L, cpb) : 0);
     return p;
 }

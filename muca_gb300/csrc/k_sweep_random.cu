@@ -78,11 +78,10 @@ __global__ void __launch_bounds__(256) k_sweep_random(const RandomArgs a, uint32
     k1.init(10u * W + 1000u * a.seed, 0xdecafbadu);
     k2.init(100u * W + 4000u * a.seed, 0x20202041u);
     k3.init(1000u * W + 10000u * a.seed, 0x11cafeadu);
-    // lanes of the last block past the chain count sweep their zero lattice
-    // (E_Delta 0) and never record; padding lanes (>= cpb) read lane 0's
-    // spins but never accept, so their E_Delta stays 1 and every weight
-    // index E + dDel stays in [0, 2]
-    int E = active ? a.edel[chain] : (store ? 0 : 1);
+    // lanes without a chain (padding lanes, which read lane 0's spins, and the
+    // last block's lanes past the chain count) never accept, so their E_Delta
+    // stays 1 and every weight index E + dDel stays in [0, 2]
+    int E = active ? a.edel[chain] : 1;
     int EJ = active ? a.ej[chain] : 0;
     const float fN = (float)N;
     uint32_t c0 = 0;
@@ -117,7 +116,7 @@ __global__ void __launch_bounds__(256) k_sweep_random(const RandomArgs a, uint32
             const uint32_t r = pick(r1, sub);
             const float2 tE = T[E];
             const float dl = dDel == 0 ? 0.0f : (dDel < 0 ? tE.x : tE.y);
-            const float g = __fsub_rn(__logf(u01f(r)), __fadd_rn(small_int_to_float(-2 * dE), dl));
+            const float g = __fsub_rn(fast_logf(u01f(r)), __fadd_rn(small_int_to_float(-2 * dE), dl));
             bool acc = g < 0.0f;
             if (fabsf(g) <= band) {
                 // in doubt: the reference's FP64 difference and exact log
@@ -128,7 +127,7 @@ __global__ void __launch_bounds__(256) k_sweep_random(const RandomArgs a, uint32
                     acc = (double)lg < diff;
                 }
             }
-            if (acc && store) {
+            if (acc && active) {
                 const uint32_t sh = 2u * (col & 15u);
                 *pw = (*pw & ~(3u << sh)) | ((uint32_t)(ns + 1) << sh);
                 EJ += dE;

@@ -212,7 +212,7 @@ __device__ __forceinline__ void decode_window(uint32_t *__restrict__ lat, uint32
         d.dM[t] = dv;
         if (BT) d.f2[t] = btab[d.dE[t] + 8];
         else    d.f2[t] = small_int_to_float(-2 * d.dE[t]);
-        d.lf[t] = __logf(u01f(r1[t]));
+        d.lf[t] = fast_logf(u01f(r1[t]));
         d.p[t] = r1[t];
     }
 }
@@ -770,147 +770,5 @@ __device__ __forceinline__ bool launch_params(const SweepArgs &a, uint32_t &iter
     }
     return true;
 }
-
-
-// The windowed sweep of chain block `blk` (cpb chains, lanes >= cpb are
-// padding): every lane draws its own Philox numbers one window ahead (n1/n3
-// hold the acceptance and direction words of the next two groups, counters
-// cc-1, cc).  Ends
-// with the block synchronised and, with HS, the shared histogram drained.
-// RING (with LAT_SMEM false): the lattice stays in global memory and each
-// lane keeps a four-row ring of its chain in shared memory (RowRing), at the
-// offset where the whole lattice would go.
-template <int MODE, int R, bool LAT_SMEM, bool HS = true, bool BT = false, bool RING = false, bool AHEAD2 = false>
-__device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned char *smem, uint32_t cpb, uint32_t blk,
-                                                uint32_t iter, unsigned long long nup,
-                                                const float *__restrict__ btab = nullptr)
-{
-    static_assert(!(RING && LAT_SMEM), "the ring serves lattices in global memory");
-    using WT = typename WeightType<MODE>::T;
-    const uint32_t lane = threadIdx.x;
-    WT *wS;
-    uint32_t *histS, *gl;
-    const size_t lat_off = smem_weights_bytes(MODE, a.N) + (HS ? smem_hist_bytes(MODE, a.N) : 0);
-    constexpr bool DT = MODE == kModeProduce;  // production scans on the FP32 difference table
-    float tol = 0.0f;
-    uint32_t *lat = prologue<MODE, LAT_SMEM, HS, DT>(a, smem, lat_off, cpb, lane, blk, wS, histS, gl, &tol);
-    RowRing<8> ring;
-    if (RING) {
-        ring.init(reinterpret_cast<uint32_t *>(smem + lat_off) + (lane < cpb ? lane : 0u), gl);
-        lat = ring.rs;
-    }
-    constexpr uint32_t rmask = RING ? 3u : ~0u;
-    __syncthreads();
-    const double *wG = reinterpret_cast<const double *>(a.w);
-    // the step-by-step path reads the weights it needs: FP64 ones from global memory in production
-    const WT *wP = DT ? reinterpret_cast<const WT *>(a.w) : wS;
-    ChainSetup<MODE, R> cs;
-    cs.init(a, cpb, lane, blk);
-    const bool store = lane < cpb;
-    ChainState st;
-    st.E = cs.active ? a.edel[cs.chain] : (store ? 0 : 3);
-    st.EJ = cs.active ? a.ej[cs.chain] : 0;
-    st.M = (cs.active && MODE == kModeProduce) ? a.mag[cs.chain] : 0;
-    const WT eps = (WT)a.log_eps;
-    const uint32_t L = a.L, WPR = a.WPR;
-    // draws of the next two groups (counters cc - 1, cc), the two streams apart
-    uint32_t n1[8], n3[8];
-    draw_pair<R>(1u, cs.seed, iter, cs.k1, cs.k3, n1, n3);
-    draw_pair<R>(2u, cs.seed, iter, cs.k1, cs.k3, n1 + 4, n3 + 4);
-    uint32_t cc = 2;
-    auto advance = [&](uint32_t groups) {
-        if (groups == 2) {
-            draw_pair<R>(cc + 1, cs.seed, iter, cs.k1, cs.k3, n1, n3);
-            draw_pair<R>(cc + 2, cs.seed, iter, cs.k1, cs.k3, n1 + 4, n3 + 4);
-            cc += 2;
-        } else {
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                n1[t] = n1[t + 4];
-                n3[t] = n3[t + 4];
-            }
-            draw_pair<R>(cc + 1, cs.seed, iter, cs.k1, cs.k3, n1 + 4, n3 + 4);
-            cc += 1;
-        }
-    };
-    // The reference's sweep order (for_each_window's): whole row-halves as a
-    // loop of full windows, W8 words of 8 same-parity sites and, with
-    // L % 16 == 8, one word of 4; a phase's last, partial row-half (only when
-    // therm or nup is not a multiple of L/2) step by step.
-    const uint32_t W8 = L >> 4, per_row = L >> 1;
-    const bool tail4 = (L & 15u) != 0;
-    // recorded attempts per lane since the shared u32 bins were last flushed:
-    // no bin can reach 2^32 while cpb * since stays below it
-    unsigned long long since = 0;
-    for (int phase = 0; phase < 2; ++phase) {
-        unsigned long long n = phase ? nup : a.therm;
-        const bool rec = phase == 1 && cs.active;
-        uint32_t row = 0, half = 0;
-        while (n >= per_row) {
-            if (RING) ring.row_start(row, L, cpb, WPR, store);
-            if (HS && MODE == kModeWeight && phase == 1) {
-                if ((since + per_row) * cpb > 0xFFFFFFFFull || (a.hooks & kHookFlushRows)) {  // uniform
-                    flush_hist<MODE>(histS, a.hist, a.N);
-                    since = 0;
-                }
-                since += per_row;
-            }
-            for (uint32_t q = 0; q < W8; ++q) {
-                uint32_t r1[8], r3[8];
-#pragma unroll
-                for (int t = 0; t < 8; ++t) {
-                    r1[t] = n1[t];
-                    r3[t] = n3[t];
-                }
-                advance(2);  // independent of the window below: overlaps its scan
-                window_core<MODE, 8, -1, HS, BT, AHEAD2>(lat, cpb, L, WPR, row, q, rec, store, false, wS, histS,
-                                                         a.hist, st, r1, r3, eps, btab, half, wG, tol, rmask);
-            }
-            if (tail4) {
-                uint32_t r1[4], r3[4];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    r1[t] = n1[t];
-                    r3[t] = n3[t];
-                }
-                advance(1);
-                window_core<MODE, 4, -1, HS, BT, AHEAD2>(lat, cpb, L, WPR, row, W8, rec, store, false, wS, histS,
-                                                         a.hist, st, r1, r3, eps, btab, half, wG, tol, rmask);
-            }
-            n -= per_row;
-            if (++row == L) {
-                row = 0;
-                half ^= 1u;
-            }
-        }
-        if (n) {
-            if (RING) ring.row_start(row, L, cpb, WPR, store);
-            for (uint32_t q = 0; n; ++q) {
-                const uint32_t cnt = (min(16u * q + 16u, L) - 16u * q) >> 1;
-                const uint32_t len = n < cnt ? (uint32_t)n : cnt;
-                uint32_t p[8];
-#pragma unroll
-                for (int t = 0; t < 8; ++t) p[t] = pack_draw(n1[t], n3[t]);
-                partial_core<MODE, HS, BT>(lat, cpb, L, WPR, row, q, half, len, rec, store, wP, histS, a.hist, st, p,
-                                           btab, rmask);
-                advance((len + 3u) >> 2);
-                n -= len;
-            }
-        }
-    }
-    if (LAT_SMEM && store) {
-        const uint32_t words = L * WPR;
-        for (uint32_t w = 0; w < words; ++w) gl[(size_t)w * cpb] = lat[(size_t)w * cpb];
-    }
-    if (RING) ring.finish(cpb, WPR, store);
-    if (cs.active) {
-        a.edel[cs.chain] = st.E;
-        a.ej[cs.chain] = st.EJ;
-        if (MODE == kModeProduce) a.mag[cs.chain] = st.M;
-    }
-    __syncthreads();
-    if (HS) drain_hist<MODE>(histS, a.hist, a.N);
-}
-
 
 }  // namespace muca

@@ -1,0 +1,88 @@
+"""The lean window of the sweep (window.cuh): the error bound of production's
+fast test (CPU), and chain counts that leave lanes without a chain, over
+several launches (GPU).
+
+The production window stages u[E] = fl32(w[E+1] - w[E]) and decides with
+g = fma(-dDel, u, h), h = fl32(l - f2), where the reference decides
+logf(u) < diff, diff = fl64(fl64(f2 + w[E+dDel]) - w[E])
+(produce2_multigpu.cu:474).  stage_differences takes
+
+    tol = 2 (2^-24 (2 m + 66) + 2^-53 (max|w| + 32 + 2 m))   (times 1.0001)
+
+with m = max|u| and claims |g - (l - diff)| <= tol / 2 for |l| < 17.
+"""
+import numpy as np
+import pytest
+
+F2 = np.arange(-16, 17, 2, dtype=np.float32)  # -2 dE for dE in [-8, 8]
+
+
+def _weights():
+    rng = np.random.default_rng(23)
+    N = 4096
+    walk = np.cumsum(rng.normal(0.0, 1.5, N + 1)) * 0.5
+    return {
+        "zero": np.zeros(N + 1),
+        "walk": walk,
+        "walk_offset_1e4": walk + 1.0e4,
+        "steep": np.cumsum(rng.normal(0.0, 40.0, N + 1)),
+        "near_f2": np.cumsum(rng.choice([-16.0, -8.0, 8.0, 16.0], N + 1) + rng.normal(0.0, 1e-6, N + 1)),
+        "large": rng.uniform(-1e5, 1e5, N + 1),
+    }
+
+
+@pytest.mark.parametrize("name", list(_weights().keys()))
+def test_fast_difference_within_half_tol(name):
+    w = _weights()[name]
+    u = np.append(np.diff(w).astype(np.float32), np.float32(0))
+    m = float(np.max(np.abs(u))) * 1.0001
+    tol = np.float32((2.0 * 2.0 ** -24 * (2.0 * m + 66.0) +
+                      2.0 * 2.0 ** -53 * (float(np.max(np.abs(w))) + 32.0 + 2.0 * m)) * 1.0001)
+    rng = np.random.default_rng(3)
+    E = np.arange(w.size)
+    worst = 0.0
+    for dd in (-1, 0, 1):
+        e = E[(E + dd >= 0) & (E + dd < w.size)]
+        ue = u[e - 1] if dd < 0 else u[e]
+        for f2 in F2:
+            diff = (np.float64(f2) + w[e + dd]) - w[e]
+            l = np.log(((2 * rng.integers(0, 1 << 23, e.size) + 1) * 2.0 ** -24)).astype(np.float32)
+            # half of them right at the threshold
+            l = np.where(rng.random(e.size) < 0.5, np.clip(diff, -16.7, -2.0 ** -24).astype(np.float32), l)
+            h = (l - f2).astype(np.float32)
+            g = (np.float64(-dd) * ue.astype(np.float64) + h.astype(np.float64)).astype(np.float32)  # one rounding
+            worst = max(worst, float(np.max(np.abs(g.astype(np.float64) - (l.astype(np.float64) - diff)))))
+    assert worst <= tol / 2, (name, worst, float(tol))
+
+
+# 1000 chains: 32 blocks of 32 lanes, 24 lanes of the last block without a
+# chain; 33 chains: a warp with one chain; 300: the last warps partly filled
+@pytest.mark.gpu
+@pytest.mark.parametrize("kernel", [0, 1, 2, 3])
+@pytest.mark.parametrize("L,nch", [(40, 1000), (8, 33), (16, 300)])
+@pytest.mark.parametrize("produce", [False, True])
+def test_lanes_without_a_chain(muca, orc, L, nch, produce, kernel):
+    """Several launches in a row: the lattices of lanes without a chain stay
+    as they were made, and every chain follows the oracle."""
+    N = L * L
+    rng = np.random.default_rng(L + nch)
+    lnw = np.cumsum(rng.normal(-0.6, 0.3, N + 1))
+    with muca.Engine(L, nchains=nch, kernel=kernel, mode=muca.MODE_PRODUCE if produce else muca.MODE_WEIGHT) as e:
+        e.set_weights(lnw)
+        e.init_chains(muca.INIT_GRADED, 0)
+        lat = e.get_lattice()
+        state = [np.ascontiguousarray(x, np.int32).copy() for x in e.chain_state()]
+        for it in range(3):
+            therm, nup = N // 2, N // 2 + 5
+            e.sweep(it, 100, 1000, therm, nup)
+            if produce:
+                lat, h = orc.produce_sweep(L, lat, *state, lnw, it, 100, therm, nup, nthreads=8)
+            else:
+                lat, h = orc.weight_sweep(L, lat, *state[:2], lnw.astype(np.float32), it, 100, therm, nup, nthreads=8)
+            np.testing.assert_array_equal(e.get_lattice(), lat)
+            ej, ed, mg = e.chain_state()
+            np.testing.assert_array_equal(ej, state[0])
+            np.testing.assert_array_equal(ed, state[1])
+            if produce:
+                np.testing.assert_array_equal(mg, state[2])
+            assert np.array_equal(e.histogram(), h)
