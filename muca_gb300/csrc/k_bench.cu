@@ -30,7 +30,7 @@
 // array by walls: the weights at E_Delta = 0..2 and N-2..N are -1e30, every
 // move onto them is rejected, and the loads reach at most three bins beyond
 // the current E_Delta.
-#include "sweep_core.cuh"
+#include "window.cuh"
 
 namespace muca {
 
@@ -73,14 +73,14 @@ __device__ __forceinline__ uint32_t floor_hash(uint32_t x)
 
 template <int PART>
 __global__ void __launch_bounds__(kFloorCpb, 1) k_sweep_floor(uint32_t windows, unsigned long long *cycles,
-                                                               uint32_t *sink, unsigned long long *hist_dummy)
+                                                               uint32_t *sink)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     float *wS = reinterpret_cast<float *>(smem);
-    uint32_t *histS = reinterpret_cast<uint32_t *>(smem + smem_weights_bytes(kModeWeight, kFloorN));
+    const uint32_t hist_off = (uint32_t)align16((size_t)(kFloorN + 1) * 4);
+    uint32_t *histS = reinterpret_cast<uint32_t *>(smem + hist_off);
     const uint32_t lane = threadIdx.x;
-    uint32_t *lat = reinterpret_cast<uint32_t *>(smem + smem_weights_bytes(kModeWeight, kFloorN) +
-                                                 smem_hist_bytes(kModeWeight, kFloorN)) + lane;
+    uint32_t *lat = reinterpret_cast<uint32_t *>(smem + win_smem_base(kModeWeight, kFloorN, true)) + lane;
     const bool walls = PART >= 2;
     for (uint32_t b = lane; b <= kFloorN; b += blockDim.x) {
         wS[b] = (walls && (b < 3 || b + 3 > kFloorN)) ? -1e30f : 0.0f;
@@ -99,39 +99,56 @@ __global__ void __launch_bounds__(kFloorCpb, 1) k_sweep_floor(uint32_t windows, 
         lat[(size_t)w * kFloorCpb] = word;
     }
     __syncthreads();
-    ChainState st;
-    st.E = walls ? (int)(kFloorN / 2) : E;
-    st.EJ = 0;
-    st.M = 0;
-    RoundKeys<7> k1, k3;
-    k1.init(2u * lane + 1u, 0xdecafbadu);
-    k3.init(2u * lane + 3u, 0xdecafbadu);
-    uint32_t n1[8], n3[8];
-    draw_pair<7>(1u, 100u, 0u, k1, k3, n1, n3);
-    draw_pair<7>(2u, 100u, 0u, k1, k3, n1 + 4, n3 + 4);
+    WState st;
+    st.e4 = 4u * (walls ? kFloorN / 2 : (uint32_t)E);
+    st.wE = *reinterpret_cast<const float *>(smem + st.e4);
+    st.ej2 = 0.0f;
+    Draws<7> dr;
+    dr.s1.init(2u * lane + 1u, 0xdecafbadu, 100u, 0u);
+    dr.s3.init(2u * lane + 3u, 0xdecafbadu, 100u, 0u);
+    dr.ln2 = kLn2;
+    Ahead ah;
+    draw8(dr, 1u, ah);
     uint32_t cc = 2, fold = 0;
-    WinDec<kModeWeight> d0, d1;
-    if (PART >= 2) {
-        decode_window<kModeWeight, 8>(lat, kFloorCpb, kFloorL, kFloorWPR, 3, 1, 0, n1, n3, nullptr, d0);
-        draw_pair<7>(3u, 100u, 0u, k1, k3, n1, n3);
-        draw_pair<7>(4u, 100u, 0u, k1, k3, n1 + 4, n3 + 4);
-        decode_window<kModeWeight, 8>(lat, kFloorCpb, kFloorL, kFloorWPR, 5, 2, 1, n1, n3, nullptr, d1);
+    auto decode_at = [&](uint32_t row, uint32_t q, Win<8> &w) {
+        const uint32_t *pc = lat + (row * kFloorWPR + q) * kFloorCpb;
+        decode<8, 0, false>(pc[0], pc[kFloorWPR * kFloorCpb], *(pc - kFloorWPR * kFloorCpb),
+                            q ? *(pc - kFloorCpb) : pc[(kFloorWPR - 1) * kFloorCpb], ah, nullptr, w);
+    };
+    Win<8> d0, d1;
+    if (PART == 2 || PART == 3) {
+        decode_at(3, 1, d0);
+        draw8(dr, 3u, ah);
+        decode_at(5, 2, d1);
     }
     // part 6: a permutation of the bins to chase through shared memory
     if (PART == 6)
         for (uint32_t b = lane; b <= kFloorN; b += blockDim.x) histS[b] = (b * 7u + 3u) % (kFloorN + 1u);
     __syncthreads();
-    float fx = 1.0f + u01f(n1[0]), fy = u01f(n1[1]);
-    int ix = (int)(n1[2] % (kFloorN + 1u));
+    float fx = 1.0f + u01f(floor_hash(lane)), fy = u01f(floor_hash(lane + 77u));
+    int ix = (int)(floor_hash(lane) % (kFloorN + 1u));
+    // replay draws never agree with a window's here: the windows are replayed
+    // rarely, and with any numbers
+    auto redraw = [&](uint32_t(&r1)[8]) {
+        dr.s1.block((unsigned long long)kPhiloxM0 * (cc - 1u), r1);
+        dr.s1.block((unsigned long long)kPhiloxM0 * cc, r1 + 4);
+    };
+    auto scan_store = [&](const Win<8> &w, uint32_t *p, uint32_t C) {
+        uint32_t Es[8];
+        const uint32_t accm = scan_weight<8, true>(w, smem, kFloorEps, st, Es, redraw);
+#pragma unroll
+        for (int t = 0; t < 8; ++t) atomicAdd(reinterpret_cast<uint32_t *>(smem + hist_off + Es[t]), 1u);
+        *p = C ^ ((w.ctr ^ w.vnib) & accm);
+    };
     const unsigned long long t0 = clock64();
     if (PART == 4) {
 #pragma unroll 1
         for (uint32_t k = 0; k < windows; ++k) {
-            draw_pair<7>(cc + 1, 100u, 0u, k1, k3, n1, n3);
-            draw_pair<7>(cc + 2, 100u, 0u, k1, k3, n1 + 4, n3 + 4);
+            draw8(dr, cc + 1, ah);
             cc += 2;
+            fold ^= ah.dn;
 #pragma unroll
-            for (int t = 0; t < 8; ++t) fold ^= n1[t] + n3[t];
+            for (int t = 0; t < 8; ++t) fold ^= __float_as_uint(ah.l[t]);
         }
     } else if (PART == 5) {
 #pragma unroll 1
@@ -148,61 +165,67 @@ __global__ void __launch_bounds__(kFloorCpb, 1) k_sweep_floor(uint32_t windows, 
         }
         fold = (uint32_t)ix;
     } else if (PART <= 1) {
-        uint32_t row = 0, q = 0, half = 0;
+        uint32_t row = 0, q = 0;
 #pragma unroll 1
         for (uint32_t k = 0; k < windows; ++k) {
-            uint32_t r1[8], r3[8];
-#pragma unroll
-            for (int t = 0; t < 8; ++t) {
-                r1[t] = n1[t];
-                r3[t] = n3[t];
-            }
-            draw_pair<7>(cc + 1, 100u, 0u, k1, k3, n1, n3);
-            draw_pair<7>(cc + 2, 100u, 0u, k1, k3, n1 + 4, n3 + 4);
+            uint32_t *pc = lat + (row * kFloorWPR + q) * kFloorCpb;
+            const uint32_t C = *pc, side = q ? *(pc - kFloorCpb) : pc[(kFloorWPR - 1) * kFloorCpb];
+            const uint32_t U = lat[((row + 1 == kFloorL ? 0 : row + 1) * kFloorWPR + q) * kFloorCpb];
+            const uint32_t D = lat[((row ? row - 1 : kFloorL - 1) * kFloorWPR + q) * kFloorCpb];
+            Win<8> w;
+            decode<8, 0, false>(C, U, D, side, ah, nullptr, w);
+            draw8(dr, cc + 1, ah);
             cc += 2;
             if (PART == 0) {
-                window_core<kModeWeight, 8, -1>(lat, kFloorCpb, kFloorL, kFloorWPR, row, q, true, true, false, wS,
-                                                histS, hist_dummy, st, r1, r3, kFloorEps, nullptr, half);
+                scan_store(w, pc, C);
             } else {
-                WinDec<kModeWeight> d;
-                decode_window<kModeWeight, 8>(lat, kFloorCpb, kFloorL, kFloorWPR, row, q, half, r1, r3, nullptr, d);
-                uint32_t f = d.C ^ d.vnib ^ (uint32_t)(size_t)d.pc;
+                uint32_t f = w.ctr ^ w.vnib ^ w.code[0];
 #pragma unroll
                 for (int t = 0; t < 8; ++t)
-                    f ^= ((uint32_t)d.dE[t] + ((uint32_t)d.dDel[t] << 8)) ^ __float_as_uint(d.f2[t]) ^
-                         __float_as_uint(d.lf[t]) ^ d.p[t];
+                    f ^= __float_as_uint(w.ns2[t]) ^ __float_as_uint(w.dv[t]) ^ __float_as_uint(w.l[t]);
                 fold += f;
             }
             // the full windows of the L = 72 rows: words 0..3 of each row
             if (++q == 4) {
                 q = 0;
-                if (++row == kFloorL) { row = 0; half ^= 1u; }
+                if (++row == kFloorL) row = 0;
             }
         }
     } else if (PART == 2) {
 #pragma unroll 1
         for (uint32_t k = 0; k < windows; k += 2) {
-            scan_window<kModeWeight, 8>(d0, true, true, false, wS, histS, hist_dummy, st, kFloorEps);
-            scan_window<kModeWeight, 8>(d1, true, true, false, wS, histS, hist_dummy, st, kFloorEps);
+            scan_store(d0, lat, 0u);
+            scan_store(d1, lat, 0u);
         }
     } else if (PART == 3) {
-        auto chain = [&](const WinDec<kModeWeight> &d) {
-            float wE = wS[st.E];
-            float A = wS[st.E + d.dDel[0]];
-            float c0 = wS[st.E + d.dDel[1]], c1 = wS[st.E + d.dDel[0] + d.dDel[1]];
+        auto chain = [&](const Win<8> &d) {
+            const uint32_t ddb[2] = {prmt_var(kTabDD4_0, kTabDD4_1, d.code[0]), prmt_var(kTabDD4_0, kTabDD4_1, d.code[1])};
+            int dd[8];
+            unrolled<8>([&](auto tc) {
+                constexpr int t = decltype(tc)::value;
+                dd[t] = sbyte<(t & 3)>(ddb[t >> 2]);
+            });
+            auto W = [&](uint32_t e) -> float { return *reinterpret_cast<const float *>(smem + e); };
+            uint32_t e1 = st.e4 + dd[0];
+            float A = W(e1), diff = __fsub_rn(__fadd_rn(d.dv[0], A), st.wE);
+            float c0 = W(st.e4 + dd[1]), c1 = W(e1 + dd[1]);
 #pragma unroll
             for (int t = 0; t < 8; ++t) {
-                const float diff = __fsub_rn(__fadd_rn(d.f2[t], A), wE);
-                const bool acc = d.lf[t] < diff;
-                if (acc) {
-                    st.E += d.dDel[t];
-                    wE = A;
+                float x0 = 0.0f, x1 = 0.0f;
+                if (t + 1 < 8) {
+                    x0 = __fsub_rn(__fadd_rn(d.dv[t + 1], c0), st.wE);
+                    x1 = __fsub_rn(__fadd_rn(d.dv[t + 1], c1), A);
                 }
+                const bool acc = d.l[t] < diff;
+                st.e4 = acc ? e1 : st.e4;
+                st.wE = acc ? A : st.wE;
                 if (t + 1 < 8) {
                     A = acc ? c1 : c0;
+                    diff = acc ? x1 : x0;
+                    e1 = st.e4 + dd[t + 1];
                     if (t + 2 < 8) {
-                        c0 = wS[st.E + d.dDel[t + 2]];
-                        c1 = wS[st.E + d.dDel[t + 1] + d.dDel[t + 2]];
+                        c0 = W(st.e4 + dd[t + 2]);
+                        c1 = W(e1 + dd[t + 2]);
                     }
                 }
             }
@@ -215,18 +238,17 @@ __global__ void __launch_bounds__(kFloorCpb, 1) k_sweep_floor(uint32_t windows, 
     }
     const unsigned long long t1 = clock64();
     if ((lane & 31u) == 0) cycles[lane >> 5] = t1 - t0;
-    sink[lane] = fold + (uint32_t)st.E + (uint32_t)st.EJ + lat[0] + (PART == 6 ? 0u : histS[lane]);
+    sink[lane] = fold + st.e4 + __float_as_uint(st.ej2) + lat[0] + (PART == 6 ? 0u : histS[lane]);
 }
 
 cudaError_t launch_sweep_floor(int part, uint32_t windows, unsigned long long *cycles, uint32_t *sink,
-                               unsigned long long *hist_dummy, cudaStream_t s)
+                               cudaStream_t s)
 {
-    const size_t smem = smem_weights_bytes(kModeWeight, kFloorN) + smem_hist_bytes(kModeWeight, kFloorN) +
-                        (size_t)kFloorL * kFloorWPR * kFloorCpb * 4;
+    const size_t smem = win_smem_base(kModeWeight, kFloorN, true) + (size_t)kFloorL * kFloorWPR * kFloorCpb * 4;
     auto go = [&](auto kern) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        kern<<<1, kFloorCpb, smem, s>>>(windows, cycles, sink, hist_dummy);
+        kern<<<1, kFloorCpb, smem, s>>>(windows, cycles, sink);
         return cudaGetLastError();
     };
     switch (part) {

@@ -991,20 +991,18 @@ muca_status muca_sweep_floor(int32_t device, uint32_t part, uint32_t windows, do
     int prev = 0;
     CUDA_TRY(nullptr, cudaGetDevice(&prev));
     CUDA_TRY(nullptr, cudaSetDevice(device));
-    unsigned long long *cyc = nullptr, *hd = nullptr;
+    unsigned long long *cyc = nullptr;
     uint32_t *sink = nullptr;
     cudaError_t err = cudaMalloc(&cyc, 4 * sizeof(unsigned long long));
-    if (err == cudaSuccess) err = cudaMalloc(&hd, sizeof(unsigned long long));
     if (err == cudaSuccess) err = cudaMalloc(&sink, 128 * sizeof(uint32_t));
     unsigned long long h[4] = {0, 0, 0, 0};
     // one launch to warm up, then the measured one
     for (int rep = 0; rep < 2 && err == cudaSuccess; ++rep) {
-        err = launch_sweep_floor((int)part, windows, cyc, sink, hd, 0);
+        err = launch_sweep_floor((int)part, windows, cyc, sink, 0);
         if (err == cudaSuccess) err = cudaDeviceSynchronize();
     }
     if (err == cudaSuccess) err = cudaMemcpy(h, cyc, sizeof(h), cudaMemcpyDeviceToHost);
     cudaFree(cyc);
-    cudaFree(hd);
     cudaFree(sink);
     cudaSetDevice(prev);
     if (err != cudaSuccess) return fail(nullptr, MUCA_ERR_CUDA, "sweep floor: %s", cudaGetErrorString(err));

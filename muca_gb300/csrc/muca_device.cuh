@@ -69,12 +69,14 @@ __device__ __forceinline__ float u01f(uint32_t r)
 // The fast logarithm of the acceptance tests.  The flush of subnormal inputs
 // (which saves the scaling of one) touches no u >= 2^-24.  Its difference to
 // logf over every u is measured (k_logf_bracket).
-__device__ __forceinline__ float fast_logf(float u)
+constexpr float kLn2 = 0.693147182464599609375f;
+__device__ __forceinline__ float lg2_ftz(float u)
 {
     float l;
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(u));
-    return __fmul_rn(l, 0.693147182464599609375f);
+    return l;
 }
+__device__ __forceinline__ float fast_logf(float u) { return __fmul_rn(lg2_ftz(u), kLn2); }
 
 // (float)k for a small integer k (|k| < 2^22) without an int-to-float
 // conversion: 1.5 * 2^23 + k is exact in FP32 (its ulp is 1), and so is the

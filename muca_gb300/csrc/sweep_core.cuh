@@ -603,30 +603,25 @@ __device__ __forceinline__ uint32_t *prologue(const SweepArgs &a, unsigned char 
 // stay in global memory.  A window of row r reads rows r - 1, r and r + 1
 // (periodic) and writes row r, so only those rows need to be near: slot
 // s = row & 3 of the ring holds row tag(s) (L is a multiple of 4, so the
-// slots follow the periodic rows).  At the start of every row the ring makes
-// rows r - 1 .. r + 1 resident (normally they already are) and starts
-// loading row r + 2 from global memory into registers, after writing the
-// slot's previous row (r - 2) back; those registers go into the slot at the
-// start of the next row, so the global latency hides behind a whole row of
-// windows.  A row that is not in its slot is not in the ring at all, so its
+// slots follow the periodic rows).  At the start of every row the ring writes
+// row r - 2 back and starts copying row r + 2 into its slot asynchronously
+// (cp.async: the copy in flight holds no register and none of the warp's
+// scoreboards, which the windows' loads need); it is waited for at the start
+// of the next row.  Rows r - 1 .. r + 1 are then resident.
+// A row that is not in its slot is not in the ring at all, so its
 // global copy is current: jumps (a new phase restarts the sweep at row 0)
-// fall back to loads at the row start.  Only the lane that owns the column
+// fall back to copies at the row start.  Only the lane that owns the column
 // (`store`) moves data; padding lanes read lane 0's ring and never write.
-// WMAX >= words per row (8 for L <= 128).
-template <int WMAX>
 struct RowRing {
     uint32_t *rs;  // the lane's ring column: word (slot, q) at rs[(slot * WPR + q) * cpb]
     uint32_t *gs;  // the lane's global column: word (row, q) at gs[(row * WPR + q) * cpb]
-    int t0, t1, t2, t3;  // row held by each slot, -1 for none
-    int prow;            // row whose words wait in pw, -1 for none
-    uint32_t pw[WMAX];
+    int t0, t1, t2, t3;  // row held (or being copied) by each slot, -1 for none
 
     __device__ __forceinline__ void init(uint32_t *ring_col, uint32_t *glob_col)
     {
         rs = ring_col;
         gs = glob_col;
         t0 = t1 = t2 = t3 = -1;
-        prow = -1;
     }
     __device__ __forceinline__ int tag(int s) const { return s == 0 ? t0 : s == 1 ? t1 : s == 2 ? t2 : t3; }
     __device__ __forceinline__ void set_tag(int s, int v)
@@ -636,54 +631,48 @@ struct RowRing {
         t2 = s == 2 ? v : t2;
         t3 = s == 3 ? v : t3;
     }
+    static __device__ __forceinline__ void wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+    // starts copying `row` into its slot, after writing back what is there
+    __device__ __forceinline__ void fetch(int row, uint32_t cpb, uint32_t WPR, bool store)
+    {
+        const int s = row & 3;
+        writeback(s, cpb, WPR, store);
+        if (store) {
+            const uint32_t *g = gs + (size_t)row * WPR * cpb;
+            uint32_t d = (uint32_t)__cvta_generic_to_shared(rs + (size_t)s * WPR * cpb);
+            for (uint32_t q = 0; q < WPR; ++q, g += cpb, d += 4u * cpb)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(g) : "memory");
+        }
+        set_tag(s, row);
+    }
     __device__ __forceinline__ void writeback(int s, uint32_t cpb, uint32_t WPR, bool store)
     {
         const int r = tag(s);
         if (r < 0) return;
-        if (store)
-            for (uint32_t q = 0; q < WPR; ++q) gs[((size_t)r * WPR + q) * cpb] = rs[((size_t)s * WPR + q) * cpb];
+        if (store) {
+            uint32_t *g = gs + (size_t)r * WPR * cpb;
+            const uint32_t *l = rs + (size_t)s * WPR * cpb;
+            for (uint32_t q = 0; q < WPR; ++q, g += cpb, l += cpb) *g = *l;
+        }
         set_tag(s, -1);
-    }
-    __device__ __forceinline__ void load(int row, uint32_t cpb, uint32_t WPR, bool store)
-    {
-        const int s = row & 3;
-        writeback(s, cpb, WPR, store);
-        if (store)
-            for (uint32_t q = 0; q < WPR; ++q) rs[((size_t)s * WPR + q) * cpb] = gs[((size_t)row * WPR + q) * cpb];
-        set_tag(s, row);
     }
     __device__ __forceinline__ void row_start(uint32_t r, uint32_t L, uint32_t cpb, uint32_t WPR, bool store)
     {
-        if (prow >= 0) {
-            const int s = prow & 3;
-            if (store) {
-#pragma unroll
-                for (int q = 0; q < WMAX; ++q)
-                    if ((uint32_t)q < WPR) rs[((size_t)s * WPR + q) * cpb] = pw[q];
-            }
-            set_tag(s, prow);
-            prow = -1;
-        }
+        wait();  // the row ordered at the last row start
         const int rm = r == 0 ? (int)L - 1 : (int)r - 1, rc = (int)r, rp = r + 1 == L ? 0 : (int)r + 1;
-        if (tag(rm & 3) != rm) load(rm, cpb, WPR, store);
-        if (tag(rc & 3) != rc) load(rc, cpb, WPR, store);
-        if (tag(rp & 3) != rp) load(rp, cpb, WPR, store);
-        const int P = rp + 1 == (int)L ? 0 : rp + 1;
-        const int s = P & 3;
-        if (tag(s) != P) {
-            writeback(s, cpb, WPR, store);
-            if (store) {
-#pragma unroll
-                for (int q = 0; q < WMAX; ++q)
-                    if ((uint32_t)q < WPR) pw[q] = gs[((size_t)P * WPR + q) * cpb];
-            }
-            prow = P;
+        if (tag(rm & 3) != rm || tag(rc & 3) != rc || tag(rp & 3) != rp) {
+            if (tag(rm & 3) != rm) fetch(rm, cpb, WPR, store);
+            if (tag(rc & 3) != rc) fetch(rc, cpb, WPR, store);
+            if (tag(rp & 3) != rp) fetch(rp, cpb, WPR, store);
+            wait();
         }
+        const int P = rp + 1 == (int)L ? 0 : rp + 1;
+        if (tag(P & 3) != P) fetch(P, cpb, WPR, store);
     }
     __device__ __forceinline__ void finish(uint32_t cpb, uint32_t WPR, bool store)
     {
+        wait();
         for (int s = 0; s < 4; ++s) writeback(s, cpb, WPR, store);
-        prow = -1;
     }
 };
 __host__ __device__ inline size_t ring_bytes(uint32_t L, uint32_t cpb)

@@ -24,6 +24,7 @@
 #pragma once
 #include "sweep_core.cuh"
 
+#include <cmath>
 #include <type_traits>
 
 namespace muca {
@@ -112,6 +113,12 @@ struct Stream {
 template <int R>
 struct Draws {
     Stream<R> s1, s3;  // acceptance, direction
+    // ln 2, the factor of the binary logarithm of u; -infinity in lanes
+    // without a chain: their logarithm is then +infinity (or, of 0, a NaN) and
+    // they never accept, with no test of their own on the chain of decisions
+    // (one cost 22 cycles per attempt)
+    float ln2;
+    __device__ __forceinline__ float log_u(uint32_t r) const { return __fmul_rn(lg2_ftz(u01s(r)), ln2); }
     __device__ __forceinline__ void group(uint32_t cc, uint32_t *r1, uint32_t *r3) const
     {
         const unsigned long long q = (unsigned long long)kPhiloxM0 * cc;
@@ -147,7 +154,7 @@ __device__ __forceinline__ void draw8(const Draws<R> &d, uint32_t c, Ahead &a)
     d.group(c + 1, r1 + 4, r3 + 4);
     a.dn = direction8(r3);
 #pragma unroll
-    for (int t = 0; t < 8; ++t) a.l[t] = fast_logf(u01s(r1[t]));
+    for (int t = 0; t < 8; ++t) a.l[t] = d.log_u(r1[t]);
 }
 // the second group moves up and group c follows it
 template <int R>
@@ -159,7 +166,7 @@ __device__ __forceinline__ void draw4(const Draws<R> &d, uint32_t c, Ahead &a)
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
         a.l[t] = a.l[t + 4];
-        a.l[t + 4] = fast_logf(u01s(r1[t]));
+        a.l[t + 4] = d.log_u(r1[t]);
     }
 }
 
@@ -178,8 +185,9 @@ constexpr uint32_t kTabDV_0 = 0x00000303u, kTabDV_1 = 0x00010104u;     // s_new 
 // u[E] = w[E+1] - w[E] for dDel = +1, u[E-1] for dDel = -1 (any for 0)
 constexpr uint32_t kTabUO_0 = 0x000000FCu, kTabUO_1 = 0x00FC0000u;
 constexpr uint32_t kTabDD_0 = 0x00010200u, kTabDD_1 = 0x00000201u;     // dDel + 1
-// (E_Delta, M) bin: b' - b = dDel E + k
-constexpr uint32_t kTabK_0 = 0x00FF0200u, kTabK_1 = 0x00FF0101u;
+// (E_Delta, M) bin: b' - b = dDel E + k, in bytes of u64 bins 2 dDel (4 E) + 8 k
+constexpr uint32_t kTabD2_0 = 0x000002FEu, kTabD2_1 = 0x00FE0200u;     // 2 dDel
+constexpr uint32_t kTabK8_0 = 0x00F81000u, kTabK8_1 = 0x00F80808u;     // 8 k
 
 // A window ready for its scan.  S slots; slot t's byte quantities are byte
 // t % 4 of word t / 4 of the tables' results.
@@ -250,6 +258,15 @@ struct WState {
     float wE, ej2;
 };
 
+// x += c if p: a predicated addition costs one issue slot where a select costs
+// two (it issues on the half-rate ALU pipe)
+__device__ __forceinline__ void add_if(bool p, uint32_t &x, uint32_t c)
+{
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p add.u32 %0, %0, %1;\n\t}"
+        : "+r"(x)
+        : "r"(c), "r"((uint32_t)p));
+}
+
 // The accept/reject scan of weight mode over E_Delta:
 //   accept  <=>  diff >= 0 || logf(u) < diff,
 //   diff = fl(fl(-beta dE + w[E + dDel]) - w[E])   (muca_delta_multigpu.cu:810-816),
@@ -259,11 +276,11 @@ struct WState {
 // The chain of one decision to the next is a select and a compare: both
 // values diff can take (the attempt before rejected or accepted) are formed
 // from weights loaded one attempt ahead.
-// `store` is false for padding lanes, which read another lane's spins and
-// never accept.  Es[] gets the bin offset after every attempt.
+// A lane without a chain has infinite logarithms and an infinite wE.
+// Es[] gets the bin offset after every attempt.
 template <int S, bool EJ, typename REDRAW>
-__device__ __forceinline__ uint32_t scan_weight(const Win<S> &w, const unsigned char *wS, bool store, float eps,
-                                                WState &st, uint32_t (&Es)[S], REDRAW &&redraw)
+__device__ __forceinline__ uint32_t scan_weight(const Win<S> &w, const unsigned char *wS, float eps, WState &st,
+                                                uint32_t (&Es)[S], REDRAW &&redraw)
 {
     const uint32_t ddb[2] = {prmt_var(kTabDD4_0, kTabDD4_1, w.code[0]),
                              S > 4 ? prmt_var(kTabDD4_0, kTabDD4_1, w.code[1]) : 0u};
@@ -291,13 +308,11 @@ __device__ __forceinline__ uint32_t scan_weight(const Win<S> &w, const unsigned 
             d0 = __fsub_rn(__fmaf_rn(w.dv[t + 1], w.ns2[t + 1], c0), st.wE);
             d1 = __fsub_rn(__fmaf_rn(w.dv[t + 1], w.ns2[t + 1], c1), A);
         }
-        const bool acc = store && (w.l[t] < diff);
+        const bool acc = w.l[t] < diff;
+        add_if(acc, accm, 0xFu << (4 * t));
         near |= fabsf(__fsub_rn(w.l[t], diff)) <= eps;
-        if (acc) {
-            accm |= 0xFu << (4 * t);
-            if (EJ) st.ej2 = __fmaf_rn(-w.dv[t], w.ns2[t], st.ej2);
-        }
-        st.e4 = acc ? e1 : st.e4;
+        if (EJ && acc) st.ej2 = __fmaf_rn(-w.dv[t], w.ns2[t], st.ej2);
+        add_if(acc, st.e4, (uint32_t)dd[t]);
         st.wE = acc ? A : st.wE;
         Es[t] = st.e4;
         if (t + 1 < S) {
@@ -321,7 +336,7 @@ __device__ __forceinline__ uint32_t scan_weight(const Win<S> &w, const unsigned 
             const float df = __fsub_rn(__fmaf_rn(w.dv[t], w.ns2[t], wn), st.wE);
             bool acc = df >= 0.0f;
             if (!acc) acc = logf(u01s(r1[t])) < df;
-            if (acc && store) {
+            if (acc) {
                 accm |= 0xFu << (4 * t);
                 if (EJ) st.ej2 = __fmaf_rn(-w.dv[t], w.ns2[t], st.ej2);
                 st.e4 += dd[t];
@@ -334,13 +349,34 @@ __device__ __forceinline__ uint32_t scan_weight(const Win<S> &w, const unsigned 
 }
 
 // A chain's running state in a production walk: the byte offset of its bin
-// in the staged weight differences, 2 E_J, M, and while recording the
-// (E_Delta, M) bin with the attempts spent there and not yet counted.
+// in the staged weight differences, 2 E_J, M, and while recording the byte
+// offset of its (E_Delta, M) bin and minus the attempts spent there and not
+// yet counted (relative to the end of the window being scanned).
 struct PState {
     uint32_t e4;
     float ej2, mag;
-    uint32_t bin, cnt;
+    uint32_t bin;
+    int since;
 };
+
+// An accepted attempt leaves the chain's bin of the 2D histogram: the attempts
+// since it came there go to the bin as one reduction, and the chain moves on
+// by `step` bytes.  `now` is the attempt's position against `since`'s origin.
+__device__ __forceinline__ void leave_bin(bool acc, unsigned long long *hist, uint32_t &bin, uint32_t step, int &since,
+                                          int now)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 a, v;\n\t.reg .b32 c;\n\t"
+        "setp.ne.u32 p, %5, 0;\n\t"
+        "cvt.u64.u32 a, %0;\n\tadd.u64 a, a, %2;\n\t"
+        "sub.s32 c, %4, %1;\n\tcvt.u64.u32 v, c;\n\t"
+        "@p red.global.add.u64 [a], v;\n\t"
+        "@p add.u32 %0, %0, %3;\n\t"
+        "@p mov.u32 %1, %4;\n\t}"
+        : "+r"(bin), "+r"(since)
+        : "l"(hist), "r"(step), "r"(now), "r"((uint32_t)acc)
+        : "memory");
+}
 
 // The scan of production.  The reference forms
 //   diff = ((double)(-2 dE) + w[E + dDel]) - w[E]   (produce2_multigpu.cu:474)
@@ -353,7 +389,7 @@ struct PState {
 // since logf(u) < 0.  Both values g can take are formed one attempt ahead.
 // REC: after every attempt the chain's (E_Delta, M) bin counts once; a run of
 // attempts in one bin goes to the u64 histogram as one reduction when the
-// chain leaves the bin (an accepted attempt always changes the bin).
+// chain leaves the bin (leave_bin; an accepted attempt always changes the bin).
 template <int S, bool REC, typename REDRAW>
 __device__ __forceinline__ uint32_t scan_produce(const Win<S> &w, const unsigned char *uS,
                                                  const double *__restrict__ wG, unsigned long long *histG,
@@ -363,18 +399,19 @@ __device__ __forceinline__ uint32_t scan_produce(const Win<S> &w, const unsigned
     const uint32_t ddb[2] = {prmt_var(kTabDD4_0, kTabDD4_1, lo), S > 4 ? prmt_var(kTabDD4_0, kTabDD4_1, hi) : 0u};
     const uint32_t uob[2] = {prmt_var(kTabUO_0, kTabUO_1, lo), S > 4 ? prmt_var(kTabUO_0, kTabUO_1, hi) : 0u};
     const uint32_t dfb[2] = {prmt_var(kTabDD_0, kTabDD_1, lo), S > 4 ? prmt_var(kTabDD_0, kTabDD_1, hi) : 0u};
-    const uint32_t kb[2] = {prmt_var(kTabK_0, kTabK_1, lo), S > 4 ? prmt_var(kTabK_0, kTabK_1, hi) : 0u};
-    int dd[S], uo[S], kk[S];
+    const uint32_t kb[2] = {prmt_var(kTabK8_0, kTabK8_1, lo), S > 4 ? prmt_var(kTabK8_0, kTabK8_1, hi) : 0u};
+    const uint32_t d2b[2] = {prmt_var(kTabD2_0, kTabD2_1, lo), S > 4 ? prmt_var(kTabD2_0, kTabD2_1, hi) : 0u};
+    int dd[S], uo[S];
     float nd[S], h[S];
     unrolled<S>([&](auto tc) {
         constexpr int t = decltype(tc)::value;
         dd[t] = sbyte<(t & 3)>(ddb[t >> 2]);
         uo[t] = sbyte<(t & 3)>(uob[t >> 2]);
-        if (REC) kk[t] = sbyte<(t & 3)>(kb[t >> 2]);
         nd[t] = __fsub_rn(8388609.0f, magic_byte<(t & 3)>(dfb[t >> 2]));  // -dDel
         h[t] = __fmaf_rn(-w.dv[t], w.ns2[t], w.l[t]);
     });
     auto U = [&](uint32_t e) -> float { return *reinterpret_cast<const float *>(uS + e); };
+    if (REC) st.since -= S;
     const PState s0 = st;
     uint32_t accm = 0;
     bool near = false;
@@ -394,16 +431,16 @@ __device__ __forceinline__ uint32_t scan_produce(const Win<S> &w, const unsigned
             g0 = __fmaf_rn(nd[t + 1], c0, h[t + 1]);
             g1 = __fmaf_rn(nd[t + 1], c1, h[t + 1]);
         }
-        const bool acc = store && (g < 0.0f);
+        const bool acc = g < 0.0f;
         near |= !(fabsf(g) > band);  // a NaN (differences beyond FP32) is in doubt too
         av[t] = acc;
         Eb[t] = st.e4;
+        add_if(acc, accm, 0xFu << (4 * t));
         if (acc) {
-            accm |= 0xFu << (4 * t);
             st.ej2 = __fmaf_rn(-w.dv[t], w.ns2[t], st.ej2);
             st.mag = __fadd_rn(st.mag, w.dv[t]);
         }
-        st.e4 = acc ? e1 : st.e4;
+        add_if(acc, st.e4, (uint32_t)dd[t]);
         if (t + 1 < S) {
             g = acc ? g1 : g0;
             e1 = st.e4 + dd[t + 1];
@@ -436,15 +473,12 @@ __device__ __forceinline__ uint32_t scan_produce(const Win<S> &w, const unsigned
         }
     }
     if (REC) {
-#pragma unroll
-        for (int t = 0; t < S; ++t) {
-            if (av[t] && active) {
-                if (st.cnt) atomicAdd(histG + st.bin, (unsigned long long)st.cnt);
-                st.bin += (dd[t] >> 2) * (int)(Eb[t] >> 2) + kk[t];
-                st.cnt = 0;
-            }
-            ++st.cnt;
-        }
+        unrolled<S>([&](auto tc) {
+            constexpr int t = decltype(tc)::value;
+            // bytes from this attempt's bin to the proposed one, 8 (dDel E + k)
+            const uint32_t step = (uint32_t)(sbyte<(t & 3)>(d2b[t >> 2]) * (int)Eb[t] + sbyte<(t & 3)>(kb[t >> 2]));
+            leave_bin(av[t], histG, st.bin, step, st.since, t - S);
+        });
     }
     return accm;
 }
@@ -531,6 +565,7 @@ __device__ __forceinline__ uint32_t *win_prologue(const SweepArgs &a, unsigned c
 // Lanes without a chain (padding lanes, and the last block's lanes past the
 // chain count) never accept and hold E_Delta = 3, so that every speculative
 // index stays inside the weights.
+constexpr int kIdleE = 3;
 template <int MODE, int R, bool LAT_SMEM, bool HS = true, bool BT = false, bool RING = false>
 __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned char *smem, uint32_t cpb, uint32_t blk,
                                                 uint32_t iter, unsigned long long nup,
@@ -544,7 +579,7 @@ __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned cha
     uint32_t *histS = reinterpret_cast<uint32_t *>(smem + hist_off), *gl;
     float tol;
     uint32_t *lat = win_prologue<MODE, LAT_SMEM, HS && !PROD>(a, smem, lat_off, cpb, lane, blk, histS, gl, tol);
-    RowRing<8> ring;
+    RowRing ring;
     const bool own = lane < cpb;  // owns its lattice column
     if (RING) {
         ring.init(reinterpret_cast<uint32_t *>(smem + lat_off) + (own ? lane : 0u), gl);
@@ -561,13 +596,21 @@ __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned cha
         const uint32_t seed = a.seed_base + a.seed_dev_mul * dev;
         dr.s1.init(a.k1_mul * W + a.k1_add, a.k1_hi, seed, iter);
         dr.s3.init(a.k3_mul * W + a.k3_add, a.k3_hi, seed, iter);
+        dr.ln2 = active ? kLn2 : -INFINITY;
     }
-    const int E0 = active ? a.edel[chain] : 3;
+    // lanes without a chain write their word and count their bin here, so that
+    // the windows need no test for them
+    __shared__ uint32_t s_scratch[2];
+    uint32_t *const scratch = &s_scratch[0];
+    unsigned char *const hist_lane =
+        active ? smem + hist_off : reinterpret_cast<unsigned char *>(&s_scratch[1]) - 4 * kIdleE;
+    const int E0 = active ? a.edel[chain] : kIdleE;
     const int EJ0 = active ? a.ej[chain] : 0;
     const int M0 = (active && PROD) ? a.mag[chain] : 0;
     WState ws{(uint32_t)E0 * 4u, 0.0f, (float)(2 * EJ0)};
-    PState ps{(uint32_t)E0 * 4u, (float)(2 * EJ0), (float)M0, 0u, 0u};
-    if (!PROD) ws.wE = reinterpret_cast<const float *>(smem)[E0];
+    PState ps{(uint32_t)E0 * 4u, (float)(2 * EJ0), (float)M0, 0u, 0};
+    // an infinite weight makes every difference of a lane without a chain -infinity
+    if (!PROD) ws.wE = active ? reinterpret_cast<const float *>(smem)[E0] : INFINITY;
     const float eps = (float)a.log_eps, band = tol + eps;
     const uint32_t L = a.L, WPR = a.WPR;
     const uint32_t W8 = L >> 4, per_row = L >> 1;
@@ -601,12 +644,11 @@ __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned cha
             accm = scan_produce<S, REC>(w, smem, wG, a.hist, active, active, band, ps, redraw);
         } else {
             uint32_t Es[S];
-            accm = scan_weight<S, !BT>(w, smem, active, eps, ws, Es, redraw);
-            if (REC && HS && active) {
+            accm = scan_weight<S, !BT>(w, smem, eps, ws, Es, redraw);
+            if (REC && HS) {
                 // one fire-and-forget shared atomic per attempt
 #pragma unroll
-                for (int t = 0; t < S; ++t)
-                    atomicAdd(reinterpret_cast<uint32_t *>(smem + hist_off + Es[t]), 1u);
+                for (int t = 0; t < S; ++t) atomicAdd(reinterpret_cast<uint32_t *>(hist_lane + Es[t]), 1u);
             } else if (REC && !HS && active) {
                 // entries merged into runs of equal bins: fewer global atomics
                 uint32_t cur = Es[0], cnt = 1;
@@ -620,7 +662,9 @@ __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned cha
                 atomicAdd(a.hist + (cur >> 2), (unsigned long long)cnt);
             }
         }
-        if (active) *p = C ^ (((w.ctr ^ w.vnib) & accm) << (HALF ? 2 : 0));
+        const uint32_t word = C ^ (((w.ctr ^ w.vnib) & accm) << (HALF ? 2 : 0));
+        if (LAT_SMEM || RING) *(active ? p : scratch) = word;
+        else if (active) *p = word;
     };
     auto row_half = [&](auto hc, auto rc, uint32_t row) {
         constexpr int HALF = decltype(hc)::value;
@@ -689,9 +733,9 @@ __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned cha
             st.E = (int)((PROD ? ps.e4 : ws.e4) >> 2);
             st.EJ = (int)(PROD ? ps.ej2 : ws.ej2) / 2;
             st.M = PROD ? (int)ps.mag : 0;
-            if (PROD && ps.cnt) {
-                if (active) atomicAdd(a.hist + ps.bin, (unsigned long long)ps.cnt);
-                ps.cnt = 0;
+            if (PROD && REC) {  // the step-by-step path counts for itself
+                if (active) atomicAdd(a.hist + (ps.bin >> 3), (unsigned long long)(uint32_t)-ps.since);
+                ps.since = 0;
             }
             for (uint32_t q = 0; n; ++q) {
                 const uint32_t cnt = (min(16u * q + 16u, L) - 16u * q) >> 1;
@@ -713,16 +757,16 @@ __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned cha
             ws.e4 = ps.e4 = (uint32_t)st.E * 4u;
             ws.ej2 = ps.ej2 = (float)(2 * st.EJ);
             ps.mag = (float)st.M;
-            if (!PROD) ws.wE = reinterpret_cast<const float *>(smem)[st.E];
+            if (!PROD && active) ws.wE = reinterpret_cast<const float *>(smem)[st.E];
         }
     };
     phase(std::false_type{}, a.therm);
     if (PROD) {
         const uint32_t E = ps.e4 >> 2;
-        ps.bin = (uint32_t)((int)ps.mag + (int)(E * E + 2u * E)) >> 1;
+        ps.bin = ((uint32_t)((int)ps.mag + (int)(E * E + 2u * E)) >> 1) * 8u;
     }
     phase(std::true_type{}, nup);
-    if (PROD && active && ps.cnt) atomicAdd(a.hist + ps.bin, (unsigned long long)ps.cnt);
+    if (PROD && active && ps.since) atomicAdd(a.hist + (ps.bin >> 3), (unsigned long long)(uint32_t)-ps.since);
     if (LAT_SMEM && own) {
         const uint32_t words = L * WPR;
         for (uint32_t w = 0; w < words; ++w) gl[(size_t)w * cpb] = lat[(size_t)w * cpb];
