@@ -93,7 +93,7 @@ typedef struct muca_params {
     uint32_t dev_offset; /* index of the first emulated device (a process that runs
                             reference devices k..k+ndev-1 sets k; seeds and init
                             counters follow the device index) */
-    uint32_t kernel;     /* sweep kernel: 0 auto (windowed when L % 8 == 0, else generic),
+    uint32_t kernel;     /* sweep kernel: 0 auto (windowed for even L >= 8, else generic),
                             1 generic (reference step by step), 2 windowed,
                             3 warp-specialised (2 and 3 need L % 8 == 0) */
     uint32_t algorithm;  /* muca_algorithm */

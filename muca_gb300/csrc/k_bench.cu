@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(kFloorCpb, 1) k_sweep_floor(uint32_t windows, 
     };
     auto scan_store = [&](const Win<8> &w, uint32_t *p, uint32_t C) {
         uint32_t Es[8];
-        const uint32_t accm = scan_weight<8, true>(w, smem, kFloorEps, st, Es, redraw);
+        const uint32_t accm = scan_weight<8, true, false>(8u, w, smem, kFloorEps, st, Es, redraw);
 #pragma unroll
         for (int t = 0; t < 8; ++t) atomicAdd(reinterpret_cast<uint32_t *>(smem + hist_off + Es[t]), 1u);
         *p = C ^ ((w.ctr ^ w.vnib) & accm);

@@ -45,19 +45,6 @@
 namespace muca {
 
 // ---------------------------------------------------------------------------
-// Windowed kernel: one block per chain block, blockDim = cpb rounded up to a warp.
-// RING: the lattice stays in global memory behind a four-row ring per lane.
-template <int MODE, int R, bool LAT_SMEM, bool RING = false>
-__global__ void __launch_bounds__(256, 1) k_sweep_win(const SweepArgs a, uint32_t cpb)
-{
-    extern __shared__ __align__(16) unsigned char smem[];
-    uint32_t iter;
-    unsigned long long nup;
-    if (!launch_params(a, iter, nup)) return;
-    win_sweep_block<MODE, R, LAT_SMEM, true, false, RING>(a, smem, cpb, blockIdx.x, iter, nup);
-}
-
-// ---------------------------------------------------------------------------
 // Warp-specialised kernel.  Warps [0, P) consume, warps [P, 2P) produce; the
 // pair (c, P+c) serves the 32 chain slots 32c..32c+31 of the block.
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -485,24 +472,47 @@ cudaError_t device_log_eps(int device, cudaStream_t s, double *eps)
 SweepPlan plan_sweep(int mode, int rounds, uint32_t L, uint32_t nchains, size_t smem_optin, int sms, int kernel)
 {
     SweepPlan p{};
-    // every mode and placement defaults to the windowed kernel: with its
-    // walk over whole row-halves it is also the faster one in production
-    // with the lattice in global memory (146 against 136 attempts/ns for the
-    // warp-specialised kernel at L=128, 142 against 138 at L=96, bit for bit
-    // the same)
+    // Every mode, size and placement defaults to the windowed kernel.  Odd
+    // sizes keep the generic one: there the sweep's even and odd sites are not
+    // the columns' parities.  Below L = 8 a row-half is less than a Philox
+    // group.
     p.mode = mode;
     p.rounds = rounds;
-    p.fast = (L % 8 == 0) && L >= 8;
-    p.kernel = !p.fast ? kKernelGeneric : (kernel < 0 ? kKernelWindowed : kernel);
+    const bool windows = L % 2 == 0 && L >= 8;
+    p.kernel = !windows ? kKernelGeneric : (kernel < 0 ? kKernelWindowed : kernel);
     const uint32_t N = L * L, WPR = (L + 15) / 16;
     const size_t per_chain = (size_t)L * WPR * 4;
-    // chains per SM if spread over all SMs, rounded up to a warp, at most 128
+    // chains per SM if spread over all SMs, rounded up to a warp
     const uint32_t per_sm = (nchains + (uint32_t)sms - 1) / (uint32_t)sms;
+    // keep 512 B of the opt-in limit for the kernels' static shared memory
+    const size_t optin = smem_optin > 512 ? smem_optin - 512 : 0;
+    if (p.kernel == kKernelWindowed && per_sm > 128 && L % 8 == 0) {
+        // More chains than one warp per SM sub-partition: one block of up to
+        // 512 of them per SM, four warps per sub-partition (128 registers
+        // each), in as few waves as that takes, evened out.  The lattices stay
+        // in shared memory when they fit there, else in global memory behind
+        // the row ring: the warps gained are worth more than the ring costs
+        // (L=72, 311296 chains: 9.92 ms with 128 chains per SM and their
+        // lattices in shared memory, 5.88 ms with 512 behind the ring).
+        const size_t front = win_smem_base(mode, N, true);
+        uint32_t most = 512;
+        while (most > 128 && front + ring_bytes(L, most) > optin) most -= 32;
+        const uint32_t waves = (per_sm + most - 1) / most;
+        const uint32_t cpb = ((per_sm + waves - 1) / waves + 31u) / 32u * 32u;
+        if (front + ring_bytes(L, cpb) <= optin) {
+            p.many = true;
+            p.cpb = cpb;
+            p.blocks = (nchains + cpb - 1) / cpb;
+            p.threads = cpb;
+            p.lat_smem = front + per_chain * cpb <= optin;
+            p.row_ring = !p.lat_smem;
+            p.smem = front + (p.lat_smem ? per_chain * cpb : ring_bytes(L, cpb));
+            return p;
+        }
+    }
     const uint32_t want = std::min<uint32_t>(128u, (per_sm + 31u) / 32u * 32u);
     const size_t base = smem_weights_bytes(mode, N) + smem_hist_bytes(mode, N);
     const size_t fixed = base + (p.kernel == kKernelSpecialized ? smem_ring_bytes((want + 31u) / 32u) : 0);
-    // keep 512 B of the opt-in limit for the kernels' static shared memory
-    const size_t optin = smem_optin > 512 ? smem_optin - 512 : 0;
     const size_t cap = optin > fixed ? (optin - fixed) / per_chain : 0;
     uint32_t cpb = want;
     // Lattice in shared memory when a block of at least one warp fits and that
@@ -530,8 +540,7 @@ SweepPlan plan_sweep(int mode, int rounds, uint32_t L, uint32_t nchains, size_t 
     p.threads = (p.kernel == kKernelSpecialized ? 2u : 1u) * warps * 32u;
     // a lattice in global memory: the windowed kernel keeps a four-row ring
     // per lane in shared memory when it fits
-    p.row_ring = !p.lat_smem && p.kernel == kKernelWindowed && L % 4 == 0 && WPR <= 8 &&
-                 front + ring_bytes(L, cpb) <= optin;
+    p.row_ring = !p.lat_smem && p.kernel == kKernelWindowed && L % 8 == 0 && front + ring_bytes(L, cpb) <= optin;
     p.smem = front + (p.kernel == kKernelSpecialized ? smem_ring_bytes(warps) : 0) +
              (p.lat_smem ? per_chain * cpb : 0) + (p.row_ring ? ring_bytes(L, cpb) : 0);
     return p;
@@ -541,9 +550,7 @@ template <int MODE, int R, bool LS>
 static cudaError_t launch_one(const SweepPlan &p, const SweepArgs &a, cudaStream_t s)
 {
     void (*kern)(const SweepArgs, uint32_t) =
-        p.kernel == kKernelSpecialized ? k_sweep_spec<MODE, R, LS>
-        : p.kernel == kKernelWindowed  ? (!LS && p.row_ring ? k_sweep_win<MODE, R, false, true> : k_sweep_win<MODE, R, LS>)
-                                       : k_sweep_generic<MODE, R, LS>;
+        p.kernel == kKernelSpecialized ? k_sweep_spec<MODE, R, LS> : k_sweep_generic<MODE, R, LS>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
     if (e != cudaSuccess) return e;
     kern<<<p.blocks, p.threads, p.smem, s>>>(a, p.cpb);
@@ -554,6 +561,8 @@ cudaError_t launch_sweep(const SweepPlan &p, const SweepArgs &a, cudaStream_t s)
 {
     // the generic kernel reads the sweep order and neighbours from tables
     if (p.kernel == kKernelGeneric && (a.index == nullptr || a.naver == nullptr)) return cudaErrorInvalidValue;
+    if (p.kernel == kKernelWindowed)
+        return p.mode == kModeWeight ? launch_sweep_win_weight(p, a, s) : launch_sweep_win_produce(p, a, s);
 #define MUCA_DISPATCH(M, R)                                                          \
     return p.lat_smem ? launch_one<M, R, true>(p, a, s) : launch_one<M, R, false>(p, a, s)
     if (p.mode == kModeWeight) {

@@ -58,7 +58,7 @@ struct SweepPlan {
     int mode;
     int rounds;
     int kernel;      // SweepKernel
-    bool fast;       // windowed kernels usable (L % 8 == 0)
+    bool many;       // windowed kernel with more than one warp of chains per SM sub-partition
     bool lat_smem;   // lattice resident in shared memory
     bool row_ring;   // lattice in global memory behind a four-row ring per lane (windowed kernel)
     uint32_t cpb;    // chains per block (lane stride of the packed lattice)
@@ -73,7 +73,7 @@ constexpr uint32_t kSlotWords = 30;
 
 // Chooses placement and block shape for (mode, L, nchains) on a device with
 // `smem_optin` bytes of opt-in shared memory per block and `sms` SMs.
-// kernel: -1 = choose (windowed when L % 8 == 0, else generic), else a SweepKernel.
+// kernel: -1 = choose (windowed when L is even and at least 8, else generic), else a SweepKernel.
 SweepPlan plan_sweep(int mode, int rounds, uint32_t L, uint32_t nchains, size_t smem_optin, int sms, int kernel = -1);
 // Worst case of |__logf(u) - logf(u)| over u = (2k+1) 2^-24, k < 2^23 (exhaustive, on the device).
 cudaError_t measure_logf_bracket(float *max_abs_err, cudaStream_t s);
@@ -82,6 +82,8 @@ cudaError_t measure_logf_bracket(float *max_abs_err, cudaStream_t s);
 // decision on the exact logf) if the measurement is implausible.
 cudaError_t device_log_eps(int device, cudaStream_t s, double *eps);
 cudaError_t launch_sweep(const SweepPlan &p, const SweepArgs &a, cudaStream_t s);
+cudaError_t launch_sweep_win_weight(const SweepPlan &p, const SweepArgs &a, cudaStream_t s);
+cudaError_t launch_sweep_win_produce(const SweepPlan &p, const SweepArgs &a, cudaStream_t s);
 
 // Random-site sweep of the reference's CPU weight program (k_sweep_random.cu,
 // muca_mag.cpp:312-393): chain c is WORKER worker0 + c, `seed` the jack

@@ -170,6 +170,38 @@ __device__ __forceinline__ void draw4(const Draws<R> &d, uint32_t c, Ahead &a)
     }
 }
 
+// The same for rows whose attempts do not come in whole groups: three groups
+// c - 2 .. c, of whose attempts the first `off` (0..3) are used up.
+struct AheadAny {
+    float l[12];
+    unsigned long long dn;
+    uint32_t off;
+};
+// drops the first group, draws group c
+template <int R>
+__device__ __forceinline__ void shift_in(const Draws<R> &d, uint32_t c, AheadAny &a)
+{
+    uint32_t r1[4], r3[4];
+    d.group(c, r1, r3);
+#pragma unroll
+    for (int t = 0; t < 8; ++t) a.l[t] = a.l[t + 4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) a.l[t + 8] = d.log_u(r1[t]);
+    a.dn = (a.dn >> 16) | ((unsigned long long)direction4(r3) << 32);
+}
+// the next eight attempts
+__device__ __forceinline__ Ahead next8(const AheadAny &a)
+{
+    Ahead x;
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+        const float x0 = (a.off & 1u) ? a.l[t + 1] : a.l[t], x2 = (a.off & 1u) ? a.l[t + 3] : a.l[t + 2];
+        x.l[t] = (a.off & 2u) ? x2 : x0;
+    }
+    x.dn = (uint32_t)(a.dn >> (4u * a.off)) & 0x11111111u;
+    return x;
+}
+
 // Tables over the 3-bit code (s + 1) | direction << 2, direction 0: s + 1,
 // 1: s - 1 (cyclic): codes 0, 1, 2 and 4, 5, 6 (3 and 7 do not occur).
 //   code   s -> s_new   dDel   s_new - s_old
@@ -273,14 +305,19 @@ __device__ __forceinline__ void add_if(bool p, uint32_t &x, uint32_t c)
 // which is logf(u) < diff, since logf(u) < 0 for every u <= 1 - 2^-24.  The
 // scan decides with fast_logf; where that lies within eps of diff in any lane
 // the window is replayed with logf.
-// The chain of one decision to the next is a select and a compare: both
-// values diff can take (the attempt before rejected or accepted) are formed
-// from weights loaded one attempt ahead.
-// A lane without a chain has infinite logarithms and an infinite wE.
+// At one warp per SM sub-partition the chain of one decision to the next is
+// kept to a select and a compare: both values diff can take (the attempt
+// before rejected or accepted) are formed from weights loaded one attempt
+// ahead.  With several warps (MANY) the load waits for the decision: the other
+// warps fill its latency, and an attempt takes eight instructions fewer (L=72,
+// 311296 chains: 6.20 ms with both values formed ahead, 5.88 ms without; one
+// warp: 0.62 and 0.68 ms).
+// len: the attempts that take place (a masked window's other logarithms are
+// infinite).  A lane without a chain has infinite logarithms and an infinite wE.
 // Es[] gets the bin offset after every attempt.
-template <int S, bool EJ, typename REDRAW>
-__device__ __forceinline__ uint32_t scan_weight(const Win<S> &w, const unsigned char *wS, float eps, WState &st,
-                                                uint32_t (&Es)[S], REDRAW &&redraw)
+template <int S, bool EJ, bool MANY, typename REDRAW>
+__device__ __forceinline__ uint32_t scan_weight(uint32_t len, const Win<S> &w, const unsigned char *wS, float eps,
+                                                WState &st, uint32_t (&Es)[S], REDRAW &&redraw)
 {
     const uint32_t ddb[2] = {prmt_var(kTabDD4_0, kTabDD4_1, w.code[0]),
                              S > 4 ? prmt_var(kTabDD4_0, kTabDD4_1, w.code[1]) : 0u};
@@ -293,35 +330,51 @@ __device__ __forceinline__ uint32_t scan_weight(const Win<S> &w, const unsigned 
     const WState s0 = st;
     uint32_t accm = 0;
     bool near = false;
-    uint32_t e1 = st.e4 + dd[0];  // the bin if this attempt is accepted
-    float A = W(e1);              // its weight
-    float diff = __fsub_rn(__fmaf_rn(w.dv[0], w.ns2[0], A), st.wE);
-    float c0 = 0.0f, c1 = 0.0f;
-    if (S > 1) {
-        c0 = W(st.e4 + dd[1]);
-        c1 = W(e1 + dd[1]);
-    }
+    if constexpr (MANY) {
 #pragma unroll
-    for (int t = 0; t < S; ++t) {
-        float d0 = 0.0f, d1 = 0.0f;
-        if (t + 1 < S) {  // the next attempt's diff if this one is rejected / accepted
-            d0 = __fsub_rn(__fmaf_rn(w.dv[t + 1], w.ns2[t + 1], c0), st.wE);
-            d1 = __fsub_rn(__fmaf_rn(w.dv[t + 1], w.ns2[t + 1], c1), A);
+        for (int t = 0; t < S; ++t) {
+            const uint32_t e1 = st.e4 + dd[t];
+            const float A = W(e1);
+            const float diff = __fsub_rn(__fmaf_rn(w.dv[t], w.ns2[t], A), st.wE);
+            const bool acc = w.l[t] < diff;
+            add_if(acc, accm, 0xFu << (4 * t));
+            near |= fabsf(__fsub_rn(w.l[t], diff)) <= eps;
+            if (EJ && acc) st.ej2 = __fmaf_rn(-w.dv[t], w.ns2[t], st.ej2);
+            add_if(acc, st.e4, (uint32_t)dd[t]);
+            st.wE = acc ? A : st.wE;
+            Es[t] = st.e4;
         }
-        const bool acc = w.l[t] < diff;
-        add_if(acc, accm, 0xFu << (4 * t));
-        near |= fabsf(__fsub_rn(w.l[t], diff)) <= eps;
-        if (EJ && acc) st.ej2 = __fmaf_rn(-w.dv[t], w.ns2[t], st.ej2);
-        add_if(acc, st.e4, (uint32_t)dd[t]);
-        st.wE = acc ? A : st.wE;
-        Es[t] = st.e4;
-        if (t + 1 < S) {
-            A = acc ? c1 : c0;
-            diff = acc ? d1 : d0;
-            e1 = st.e4 + dd[t + 1];
-            if (t + 2 < S) {
-                c0 = W(st.e4 + dd[t + 2]);
-                c1 = W(e1 + dd[t + 2]);
+    } else {
+        uint32_t e1 = st.e4 + dd[0];  // the bin if this attempt is accepted
+        float A = W(e1);              // its weight
+        float diff = __fsub_rn(__fmaf_rn(w.dv[0], w.ns2[0], A), st.wE);
+        float c0 = 0.0f, c1 = 0.0f;
+        if (S > 1) {
+            c0 = W(st.e4 + dd[1]);
+            c1 = W(e1 + dd[1]);
+        }
+#pragma unroll
+        for (int t = 0; t < S; ++t) {
+            float d0 = 0.0f, d1 = 0.0f;
+            if (t + 1 < S) {  // the next attempt's diff if this one is rejected / accepted
+                d0 = __fsub_rn(__fmaf_rn(w.dv[t + 1], w.ns2[t + 1], c0), st.wE);
+                d1 = __fsub_rn(__fmaf_rn(w.dv[t + 1], w.ns2[t + 1], c1), A);
+            }
+            const bool acc = w.l[t] < diff;
+            add_if(acc, accm, 0xFu << (4 * t));
+            near |= fabsf(__fsub_rn(w.l[t], diff)) <= eps;
+            if (EJ && acc) st.ej2 = __fmaf_rn(-w.dv[t], w.ns2[t], st.ej2);
+            add_if(acc, st.e4, (uint32_t)dd[t]);
+            st.wE = acc ? A : st.wE;
+            Es[t] = st.e4;
+            if (t + 1 < S) {
+                A = acc ? c1 : c0;
+                diff = acc ? d1 : d0;
+                e1 = st.e4 + dd[t + 1];
+                if (t + 2 < S) {
+                    c0 = W(st.e4 + dd[t + 2]);
+                    c1 = W(e1 + dd[t + 2]);
+                }
             }
         }
     }
@@ -336,6 +389,7 @@ __device__ __forceinline__ uint32_t scan_weight(const Win<S> &w, const unsigned 
             const float df = __fsub_rn(__fmaf_rn(w.dv[t], w.ns2[t], wn), st.wE);
             bool acc = df >= 0.0f;
             if (!acc) acc = logf(u01s(r1[t])) < df;
+            acc = acc && (uint32_t)t < len;
             if (acc) {
                 accm |= 0xFu << (4 * t);
                 if (EJ) st.ej2 = __fmaf_rn(-w.dv[t], w.ns2[t], st.ej2);
@@ -378,7 +432,8 @@ __device__ __forceinline__ void leave_bin(bool acc, unsigned long long *hist, ui
         : "memory");
 }
 
-// The scan of production.  The reference forms
+// The scan of production.  len: the attempts of the window that count (S, or
+// fewer in a masked window, whose other logarithms are infinite).  The reference forms
 //   diff = ((double)(-2 dE) + w[E + dDel]) - w[E]   (produce2_multigpu.cu:474)
 // with FP64 weights, and FP64 issues slowly on this GPU.  Here, on the FP32
 // differences u[E] = w[E+1] - w[E],
@@ -391,9 +446,9 @@ __device__ __forceinline__ void leave_bin(bool acc, unsigned long long *hist, ui
 // attempts in one bin goes to the u64 histogram as one reduction when the
 // chain leaves the bin (leave_bin; an accepted attempt always changes the bin).
 template <int S, bool REC, typename REDRAW>
-__device__ __forceinline__ uint32_t scan_produce(const Win<S> &w, const unsigned char *uS,
+__device__ __forceinline__ uint32_t scan_produce(uint32_t len, const Win<S> &w, const unsigned char *uS,
                                                  const double *__restrict__ wG, unsigned long long *histG,
-                                                 bool store, bool active, float band, PState &st, REDRAW &&redraw)
+                                                 bool store, float band, PState &st, REDRAW &&redraw)
 {
     const uint32_t lo = w.code[0], hi = w.code[1];
     const uint32_t ddb[2] = {prmt_var(kTabDD4_0, kTabDD4_1, lo), S > 4 ? prmt_var(kTabDD4_0, kTabDD4_1, hi) : 0u};
@@ -411,7 +466,7 @@ __device__ __forceinline__ uint32_t scan_produce(const Win<S> &w, const unsigned
         h[t] = __fmaf_rn(-w.dv[t], w.ns2[t], w.l[t]);
     });
     auto U = [&](uint32_t e) -> float { return *reinterpret_cast<const float *>(uS + e); };
-    if (REC) st.since -= S;
+    if (REC) st.since -= (int)len;
     const PState s0 = st;
     uint32_t accm = 0;
     bool near = false;
@@ -461,7 +516,7 @@ __device__ __forceinline__ uint32_t scan_produce(const Win<S> &w, const unsigned
             const double diff = __dsub_rn(__dadd_rn((double)__fmul_rn(w.dv[t], w.ns2[t]), wG[E + (dd[t] >> 2)]), wG[E]);
             bool acc = diff >= 0.0;
             if (!acc) acc = (double)logf(u01s(r1[t])) < diff;
-            acc = acc && store;
+            acc = acc && store && (uint32_t)t < len;
             av[t] = acc;
             Eb[t] = st.e4;
             if (acc) {
@@ -477,7 +532,7 @@ __device__ __forceinline__ uint32_t scan_produce(const Win<S> &w, const unsigned
             constexpr int t = decltype(tc)::value;
             // bytes from this attempt's bin to the proposed one, 8 (dDel E + k)
             const uint32_t step = (uint32_t)(sbyte<(t & 3)>(d2b[t >> 2]) * (int)Eb[t] + sbyte<(t & 3)>(kb[t >> 2]));
-            leave_bin(av[t], histG, st.bin, step, st.since, t - S);
+            leave_bin(av[t], histG, st.bin, step, st.since, t - (int)len);
         });
     }
     return accm;
@@ -566,12 +621,14 @@ __device__ __forceinline__ uint32_t *win_prologue(const SweepArgs &a, unsigned c
 // chain count) never accept and hold E_Delta = 3, so that every speculative
 // index stays inside the weights.
 constexpr int kIdleE = 3;
-template <int MODE, int R, bool LAT_SMEM, bool HS = true, bool BT = false, bool RING = false>
+template <int MODE, int R, bool LAT_SMEM, bool HS = true, bool BT = false, bool RING = false,
+          bool ALIGNED = true, bool MANY = false>
 __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned char *smem, uint32_t cpb, uint32_t blk,
                                                 uint32_t iter, unsigned long long nup,
                                                 const float *__restrict__ btab = nullptr)
 {
     static_assert(!(RING && LAT_SMEM), "the ring serves lattices in global memory");
+    static_assert(ALIGNED || !RING, "the ring serves L % 8 == 0");
     constexpr bool PROD = MODE == kModeProduce;
     const uint32_t lane = threadIdx.x;
     const size_t hist_off = align16((size_t)(a.N + 1) * 4);
@@ -613,47 +670,86 @@ __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned cha
     if (!PROD) ws.wE = active ? reinterpret_cast<const float *>(smem)[E0] : INFINITY;
     const float eps = (float)a.log_eps, band = tol + eps;
     const uint32_t L = a.L, WPR = a.WPR;
-    const uint32_t W8 = L >> 4, per_row = L >> 1;
-    const bool tail4 = (L & 15u) != 0;
-    Ahead ah;  // groups cc - 1 and cc
-    draw8(dr, 1u, ah);
-    uint32_t cc = 2;
+    const uint32_t W8 = L >> 4, per_row = L >> 1, tail = per_row & 7u;
+    const uint32_t last_sites = L - 16u * (WPR - 1u);  // sites of a row's last word
+    // the draws ahead: groups cc - 1 and cc (not ALIGNED: cc - 2 .. cc)
+    std::conditional_t<ALIGNED, Ahead, AheadAny> ah;
+    uint32_t cc;
+    if constexpr (ALIGNED) {
+        draw8(dr, 1u, ah);
+        cc = 2;
+    } else {
+        ah.dn = 0;
+        ah.off = 0;
+#pragma unroll
+        for (int t = 0; t < 12; ++t) ah.l[t] = 0.0f;
+        for (cc = 0; cc < 3;) shift_in(dr, ++cc, ah);
+    }
 
-    // one window: its word at p (C), its up / down / side words, slots from `ah`
-    auto window = [&](auto sc, auto hc, auto rc, uint32_t *p, uint32_t C, uint32_t Cm, uint32_t Uw, uint32_t Dw,
-                      uint32_t side) {
+    // One window: its word at p (C, with the site right of the row's last one
+    // merged in: Cm), its up / down / side words.  MASKED: only len of its
+    // attempts take place; the others' logarithms become infinite.
+    auto window = [&](auto sc, auto hc, auto rc, auto mc, uint32_t *p, uint32_t C, uint32_t Cm, uint32_t Uw,
+                      uint32_t Dw, uint32_t side, uint32_t len) {
         constexpr int S = decltype(sc)::value, HALF = decltype(hc)::value;
-        constexpr bool REC = decltype(rc)::value;
+        constexpr bool REC = decltype(rc)::value, MASKED = decltype(mc)::value;
         Win<S> w;
-        decode<S, HALF, BT>(Cm, Uw, Dw, side, ah, btab, w);
-        const uint32_t c0 = cc - 1u;
-        // the next window's draws, independent of the scan below
-        if (S == 8) {
-            draw8(dr, cc + 1u, ah);
-            cc += 2;
+        uint32_t c0, off = 0;
+        if constexpr (ALIGNED) {
+            decode<S, HALF, BT>(Cm, Uw, Dw, side, ah, btab, w);
+            c0 = cc - 1u;
+            // the next window's draws, independent of the scan below
+            if (S == 4 || (MASKED && len <= 4u)) {
+                draw4(dr, cc + 1u, ah);
+                cc += 1;
+            } else {
+                draw8(dr, cc + 1u, ah);
+                cc += 2;
+            }
         } else {
-            draw4(dr, cc + 1u, ah);
-            cc += 1;
+            const Ahead x = next8(ah);
+            decode<S, HALF, BT>(Cm, Uw, Dw, side, x, btab, w);
+            c0 = cc - 2u;
+            off = ah.off;
+            for (ah.off += len; ah.off >= 4u; ah.off -= 4u) shift_in(dr, ++cc, ah);
         }
+        if (MASKED)
+#pragma unroll
+            for (int t = 0; t < S; ++t)
+                if ((uint32_t)t >= len) w.l[t] = INFINITY;
         auto redraw = [&](uint32_t(&r1)[S]) {
-            dr.s1.block((unsigned long long)kPhiloxM0 * c0, r1);
-            if (S > 4) dr.s1.block((unsigned long long)kPhiloxM0 * (c0 + 1u), r1 + (S > 4 ? 4 : 0));
+            if (ALIGNED) {
+                dr.s1.block((unsigned long long)kPhiloxM0 * c0, r1);
+                if (S > 4) dr.s1.block((unsigned long long)kPhiloxM0 * (c0 + 1u), r1 + (S > 4 ? 4 : 0));
+            } else {
+                uint32_t r[12];
+#pragma unroll
+                for (int g = 0; g < 3; ++g) dr.s1.block((unsigned long long)kPhiloxM0 * (c0 + g), r + 4 * g);
+#pragma unroll
+                for (int t = 0; t < S; ++t) {
+                    const uint32_t x0 = (off & 1u) ? r[t + 1] : r[t], x2 = (off & 1u) ? r[t + 3] : r[t + 2];
+                    r1[t] = (off & 2u) ? x2 : x0;
+                }
+            }
         };
+        const uint32_t m = MASKED ? len : (uint32_t)S;
         uint32_t accm;
         if (PROD) {
-            accm = scan_produce<S, REC>(w, smem, wG, a.hist, active, active, band, ps, redraw);
+            accm = scan_produce<S, REC>(m, w, smem, wG, a.hist, active, band, ps, redraw);
         } else {
             uint32_t Es[S];
-            accm = scan_weight<S, !BT>(w, smem, eps, ws, Es, redraw);
+            accm = scan_weight<S, !BT, MANY>(m, w, smem, eps, ws, Es, redraw);
             if (REC && HS) {
                 // one fire-and-forget shared atomic per attempt
 #pragma unroll
-                for (int t = 0; t < S; ++t) atomicAdd(reinterpret_cast<uint32_t *>(hist_lane + Es[t]), 1u);
+                for (int t = 0; t < S; ++t)
+                    if (!MASKED || (uint32_t)t < len) atomicAdd(reinterpret_cast<uint32_t *>(hist_lane + Es[t]), 1u);
             } else if (REC && !HS && active) {
                 // entries merged into runs of equal bins: fewer global atomics
                 uint32_t cur = Es[0], cnt = 1;
 #pragma unroll
                 for (int t = 1; t < S; ++t) {
+                    if (MASKED && (uint32_t)t >= len) break;
                     const bool same = Es[t] == cur;
                     if (!same) atomicAdd(a.hist + (cur >> 2), (unsigned long long)cnt);
                     cnt = same ? cnt + 1u : 1u;
@@ -666,51 +762,57 @@ __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned cha
         if (LAT_SMEM || RING) *(active ? p : scratch) = word;
         else if (active) *p = word;
     };
-    auto row_half = [&](auto hc, auto rc, uint32_t row) {
+    using S8 = std::integral_constant<int, 8>;
+    using S4 = std::integral_constant<int, 4>;
+    using H0 = std::integral_constant<int, 0>;
+    using H1 = std::integral_constant<int, 1>;
+    // `left` attempts of row-half (row, HALF): PART false: all of them (full
+    // windows of 8, then the row's last word), else a phase's last ones.
+    auto row_half = [&](auto hc, auto rc, auto pc_, uint32_t row, uint32_t left) {
         constexpr int HALF = decltype(hc)::value;
-        using S8 = std::integral_constant<int, 8>;
-        using S4 = std::integral_constant<int, 4>;
+        constexpr bool PART = decltype(pc_)::value;
+        using Whole = std::false_type;
+        using Masked = std::true_type;
         const uint32_t rup = (row + 1 == L) ? 0u : row + 1, rdn = (row == 0) ? L - 1 : row - 1;
         uint32_t *pc = lat + (size_t)((row & rmask) * WPR) * cpb;
         const uint32_t *pu = lat + (size_t)((rup & rmask) * WPR) * cpb;
         const uint32_t *pd = lat + (size_t)((rdn & rmask) * WPR) * cpb;
-        if (HALF == 0) {
-            uint32_t side = pc[(size_t)(WPR - 1) * cpb] << (tail4 ? 16 : 0);
-            for (uint32_t q = 0; q < W8; ++q, pc += cpb, pu += cpb, pd += cpb) {
-                const uint32_t C = *pc;
-                window(S8{}, hc, rc, pc, C, C, *pu, *pd, side);
-                side = C;  // its odd sites do not change in this half
+        const uint32_t n8 = PART ? left >> 3 : W8, rest = PART ? left & 7u : tail;
+        uint32_t C = *pc;
+        const uint32_t first = C;  // (HALF 1) its even sites do not change in this half
+        // HALF 0: the word to the left, its last site at the top; its odd sites
+        // do not change in this half
+        uint32_t side = HALF == 0 ? pc[(size_t)(WPR - 1) * cpb] << (32u - 2u * last_sites) : 0u;
+        uint32_t q = 0;
+        for (; q < n8; ++q, pc += cpb, pu += cpb, pd += cpb) {
+            const uint32_t next = q + 1 < WPR ? pc[cpb] : first;
+            window(S8{}, hc, rc, Whole{}, pc, C, C, *pu, *pd, HALF == 0 ? side : next, 8u);
+            side = C;
+            C = next;
+        }
+        if (rest) {
+            uint32_t Cm = C;
+            if (HALF == 1) {
+                side = q + 1 < WPR ? pc[cpb] : first;
+                // the site right of the row's last one is its first
+                if (q + 1 == WPR && last_sites != 16u)
+                    Cm = (C & ((1u << (2u * last_sites)) - 1u)) | (first << (2u * last_sites));
             }
-            if (tail4) {
-                const uint32_t C = *pc;
-                window(S4{}, hc, rc, pc, C, C, *pu, *pd, side);
-            }
-        } else {
-            const uint32_t first = *pc;  // its even sites do not change in this half
-            uint32_t C = first;
-            for (uint32_t q = 0; q < W8; ++q, pc += cpb, pu += cpb, pd += cpb) {
-                const uint32_t next = q + 1 < WPR ? pc[cpb] : first;
-                window(S8{}, hc, rc, pc, C, C, *pu, *pd, next);
-                C = next;
-            }
-            // the site right of the word's last one is the row's first
-            if (tail4) window(S4{}, hc, rc, pc, C, (C & 0xFFFFu) | (first << 16), *pu, *pd, 0u);
+            if (ALIGNED && !PART) window(S4{}, hc, rc, Whole{}, pc, C, Cm, *pu, *pd, side, 4u);
+            else                  window(S8{}, hc, rc, Masked{}, pc, C, Cm, *pu, *pd, side, rest);
         }
     };
 
-    // The reference's sweep order (for_each_window's): whole row-halves as a
-    // loop of full windows, W8 words of 8 same-parity sites and, with
-    // L % 16 == 8, one word of 4; a phase's last, partial row-half (only when
-    // therm or nup is not a multiple of L/2) step by step.
-    using H0 = std::integral_constant<int, 0>;
-    using H1 = std::integral_constant<int, 1>;
-    // recorded attempts per lane since the shared u32 bins were last flushed:
+    // The reference's sweep order: the even sites row by row, then the odd
+    // ones (muca_delta_multigpu.cu:173).  A phase's last row-half is partial
+    // when therm or nup is not a multiple of L/2.
+    // Recorded attempts per lane since the shared u32 bins were last flushed:
     // no bin can reach 2^32 while cpb * since stays below it
     unsigned long long since = 0;
     auto phase = [&](auto rc, unsigned long long n) {
         constexpr bool REC = decltype(rc)::value;
         uint32_t row = 0, half = 0;
-        while (n >= per_row) {
+        auto row_begin = [&]() {
             if (RING) ring.row_start(row, L, cpb, WPR, own);
             if (HS && !PROD && REC) {
                 if ((since + per_row) * cpb > 0xFFFFFFFFull || (a.hooks & kHookFlushRows)) {  // uniform
@@ -719,8 +821,11 @@ __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned cha
                 }
                 since += per_row;
             }
-            if (half == 0) row_half(H0{}, rc, row);
-            else           row_half(H1{}, rc, row);
+        };
+        while (n >= per_row) {
+            row_begin();
+            if (half == 0) row_half(H0{}, rc, std::false_type{}, row, per_row);
+            else           row_half(H1{}, rc, std::false_type{}, row, per_row);
             n -= per_row;
             if (++row == L) {
                 row = 0;
@@ -728,36 +833,16 @@ __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned cha
             }
         }
         if (n) {
-            if (RING) ring.row_start(row, L, cpb, WPR, own);
-            ChainState st;
-            st.E = (int)((PROD ? ps.e4 : ws.e4) >> 2);
-            st.EJ = (int)(PROD ? ps.ej2 : ws.ej2) / 2;
-            st.M = PROD ? (int)ps.mag : 0;
-            if (PROD && REC) {  // the step-by-step path counts for itself
-                if (active) atomicAdd(a.hist + (ps.bin >> 3), (unsigned long long)(uint32_t)-ps.since);
-                ps.since = 0;
+            row_begin();
+            if (half == 0) row_half(H0{}, rc, std::true_type{}, row, (uint32_t)n);
+            else           row_half(H1{}, rc, std::true_type{}, row, (uint32_t)n);
+        }
+        // a phase's draws start at a new group
+        if constexpr (!ALIGNED) {
+            if (ah.off) {
+                shift_in(dr, ++cc, ah);
+                ah.off = 0;
             }
-            for (uint32_t q = 0; n; ++q) {
-                const uint32_t cnt = (min(16u * q + 16u, L) - 16u * q) >> 1;
-                const uint32_t len = n < cnt ? (uint32_t)n : cnt, groups = (len + 3u) >> 2;
-                uint32_t r1[8], r3[8], p[8];
-                dr.group(cc - 1u, r1, r3);
-                dr.group(cc, r1 + 4, r3 + 4);
-#pragma unroll
-                for (int t = 0; t < 8; ++t) p[t] = pack_draw(r1[t], r3[t]);
-                using WT = typename WeightType<MODE>::T;
-                partial_core<MODE, HS && !PROD, BT>(lat, cpb, L, WPR, row, q, half, len, REC && active, active,
-                                                    PROD ? reinterpret_cast<const WT *>(a.w)
-                                                         : reinterpret_cast<const WT *>(smem),
-                                                    histS, a.hist, st, p, btab, rmask);
-                cc += groups;
-                n -= len;
-            }
-            draw8(dr, cc - 1u, ah);
-            ws.e4 = ps.e4 = (uint32_t)st.E * 4u;
-            ws.ej2 = ps.ej2 = (float)(2 * st.EJ);
-            ps.mag = (float)st.M;
-            if (!PROD && active) ws.wE = reinterpret_cast<const float *>(smem)[st.E];
         }
     };
     phase(std::false_type{}, a.therm);

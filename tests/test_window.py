@@ -1,6 +1,7 @@
 """The lean window of the sweep (window.cuh): the error bound of production's
-fast test (CPU), and chain counts that leave lanes without a chain, over
-several launches (GPU).
+fast test (CPU); chain counts that leave lanes without a chain, over several
+launches, sizes that are not a multiple of 8, and more chains than one warp
+per SM sub-partition, against the oracle (GPU).
 
 The production window stages u[E] = fl32(w[E+1] - w[E]) and decides with
 g = fma(-dDel, u, h), h = fl32(l - f2), where the reference decides
@@ -86,3 +87,79 @@ def test_lanes_without_a_chain(muca, orc, L, nch, produce, kernel):
             if produce:
                 np.testing.assert_array_equal(mg, state[2])
             assert np.array_equal(e.histogram(), h)
+
+
+# sizes that are not a multiple of 8: every remainder of L mod 16, row-halves
+# that leave the Philox groups at every offset, one word per row and several
+@pytest.mark.gpu
+@pytest.mark.parametrize("L", [10, 12, 14, 18, 20, 22, 26, 28, 30, 34, 36, 50, 100, 126])
+@pytest.mark.parametrize("produce,rounds", [(False, 7), (True, 7), (False, 10)])
+def test_even_sizes(muca, orc, L, produce, rounds):
+    N, nch = L * L, 40
+    rng = np.random.default_rng(L)
+    lnw = np.cumsum(rng.normal(0.0, 1.2, N + 1)) * 0.5
+    with muca.Engine(L, nchains=nch, rounds=rounds, mode=muca.MODE_PRODUCE if produce else muca.MODE_WEIGHT) as e:
+        assert e.info.kernel == muca.KERNEL_WINDOWED
+        e.set_weights(lnw)
+        e.init_chains(muca.INIT_GRADED, 0)
+        lat = e.get_lattice()
+        state = [np.ascontiguousarray(x, np.int32).copy() for x in e.chain_state()]
+        for it, (therm, nup) in enumerate([(N, N), (L // 2 + 3, 2 * L + 1), (0, 7), (5, 0)]):
+            e.sweep(it, 100, 1000, therm, nup)
+            if produce:
+                lat, h = orc.produce_sweep(L, lat, *state, lnw, it, 100, therm, nup, rounds=rounds, nthreads=8)
+            else:
+                lat, h = orc.weight_sweep(L, lat, *state[:2], lnw.astype(np.float32), it, 100, therm, nup,
+                                          rounds=rounds, nthreads=8)
+            np.testing.assert_array_equal(e.get_lattice(), lat)
+            ej, ed, mg = e.chain_state()
+            np.testing.assert_array_equal(ej, state[0])
+            np.testing.assert_array_equal(ed, state[1])
+            if produce:
+                np.testing.assert_array_equal(mg, state[2])
+            assert np.array_equal(e.histogram(), h)
+        e.set_log_bracket(1e30)  # every window on the exact path
+        e.sweep(9, 100, 1000, L, L + 1)
+        if produce:
+            lat, h = orc.produce_sweep(L, lat, *state, lnw, 9, 100, L, L + 1, rounds=rounds, nthreads=8)
+        else:
+            lat, h = orc.weight_sweep(L, lat, *state[:2], lnw.astype(np.float32), 9, 100, L, L + 1, rounds=rounds,
+                                      nthreads=8)
+        np.testing.assert_array_equal(e.get_lattice(), lat)
+        assert np.array_equal(e.histogram(), h)
+
+
+# more chains than one warp per SM sub-partition: blocks of up to 512 chains,
+# lattices in shared memory (L = 16, 40) and behind the row ring (64, 128)
+@pytest.mark.gpu
+@pytest.mark.parametrize("L,nch,smem", [(16, 20011, 1), (40, 60000, 1), (64, 80000, 0), (128, 30000, 0)])
+@pytest.mark.parametrize("produce", [False, True])
+def test_many_chains(muca, orc, L, nch, smem, produce):
+    N = L * L
+    rng = np.random.default_rng(L)
+    lnw = np.cumsum(rng.normal(-0.6, 0.3, N + 1))
+    therm, nup = 3 * L + 1, 5 * L + 2
+    with muca.Engine(L, nchains=nch, mode=muca.MODE_PRODUCE if produce else muca.MODE_WEIGHT) as e:
+        assert e.info.chains_per_block > 128 and e.info.lattice_in_smem == smem
+        cpb = e.info.chains_per_block
+        e.set_weights(lnw)
+        e.init_chains(muca.INIT_GRADED, 0)
+        lat0 = e.get_lattice()
+        s0 = e.chain_state()
+        e.sweep(2, 100, 1000, therm, nup)
+        lat1 = e.get_lattice()
+        s1 = e.chain_state()
+        h = e.histogram()
+    assert int(h.sum()) == nch * nup
+    mid = (nch // cpb // 2) * cpb
+    for lo, hi in ((0, 40), (mid - 20, mid + 20), (nch - 40, nch)):
+        a = lat0[lo:hi].copy()
+        st = [np.ascontiguousarray(x[lo:hi], np.int32).copy() for x in s0]
+        if produce:
+            orc.produce_sweep(L, a, *st, lnw, 2, 100, therm, nup, chain0=lo, nthreads=8)
+            np.testing.assert_array_equal(s1[2][lo:hi], st[2])
+        else:
+            orc.weight_sweep(L, a, *st[:2], lnw.astype(np.float32), 2, 100, therm, nup, chain0=lo, nthreads=8)
+        np.testing.assert_array_equal(lat1[lo:hi], a.reshape(hi - lo, N))
+        np.testing.assert_array_equal(s1[0][lo:hi], st[0])
+        np.testing.assert_array_equal(s1[1][lo:hi], st[1])
