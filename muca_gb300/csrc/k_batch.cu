@@ -112,22 +112,32 @@ static BatchKernel batch_kernel(int rounds, uint32_t lat, bool hist_smem)
     return rounds == 10 ? batch_kernel_r<10>(lat, hist_smem) : batch_kernel_r<7>(lat, hist_smem);
 }
 
-cudaError_t batch_sweep_occupancy(uint32_t cpb, int rounds, uint32_t lat, bool hist_smem, size_t smem, int *blocks)
+// Every launch raises the kernel's limit to all that a block may have: a limit
+// set to one batch's own size would be the wrong one for another batch of the
+// process that shares the kernel.
+static cudaError_t raise_smem_limit(BatchKernel k, size_t smem_limit)
+{
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_limit);
+}
+
+cudaError_t batch_sweep_occupancy(uint32_t cpb, int rounds, uint32_t lat, bool hist_smem, size_t smem,
+                                  size_t smem_limit, int *blocks)
 {
     if (lat > kLatWhereFits) return cudaErrorInvalidValue;
     const BatchKernel k = batch_kernel(rounds, lat, hist_smem);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = raise_smem_limit(k, smem_limit);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k, (int)((cpb + 31u) / 32u * 32u), smem);
 }
 
 cudaError_t launch_batch_sweep(const BatchInst *insts, const BatchItem *items, uint32_t n_items, uint32_t *next_item,
                                uint32_t cpb, int rounds, uint32_t lat, bool hist_smem, uint32_t grid, size_t smem,
-                               cudaStream_t s)
+                               size_t smem_limit, cudaStream_t s)
 {
-    // the shared-memory attribute was set by batch_sweep_occupancy for this shape
     if (cpb == 0 || cpb > 256 || lat > kLatWhereFits) return cudaErrorInvalidValue;
     const BatchKernel k = batch_kernel(rounds, lat, hist_smem);
+    const cudaError_t e = raise_smem_limit(k, smem_limit);
+    if (e != cudaSuccess) return e;
     k<<<grid, (cpb + 31u) / 32u * 32u, smem, s>>>(insts, items, n_items, next_item, cpb, (uint32_t)smem);
     return cudaGetLastError();
 }

@@ -486,6 +486,7 @@ SweepPlan plan_sweep(int mode, int rounds, uint32_t L, uint32_t nchains, size_t 
     const uint32_t per_sm = (nchains + (uint32_t)sms - 1) / (uint32_t)sms;
     // keep 512 B of the opt-in limit for the kernels' static shared memory
     const size_t optin = smem_optin > 512 ? smem_optin - 512 : 0;
+    p.smem_limit = optin;
     if (p.kernel == kKernelWindowed && per_sm > 128 && L % 8 == 0) {
         // More chains than one warp per SM sub-partition: one block of up to
         // 512 of them per SM, four warps per sub-partition (128 registers
@@ -551,7 +552,8 @@ static cudaError_t launch_one(const SweepPlan &p, const SweepArgs &a, cudaStream
 {
     void (*kern)(const SweepArgs, uint32_t) =
         p.kernel == kKernelSpecialized ? k_sweep_spec<MODE, R, LS> : k_sweep_generic<MODE, R, LS>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)p.smem_limit);
     if (e != cudaSuccess) return e;
     kern<<<p.blocks, p.threads, p.smem, s>>>(a, p.cpb);
     return cudaGetLastError();

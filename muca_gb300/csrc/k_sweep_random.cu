@@ -155,10 +155,11 @@ __global__ void __launch_bounds__(256) k_sweep_random(const RandomArgs a, uint32
 }
 
 template <int R, bool LS>
-static cudaError_t launch_random_one(const RandomArgs &a, uint32_t cpb, uint32_t blocks, size_t smem, cudaStream_t s)
+static cudaError_t launch_random_one(const RandomArgs &a, uint32_t cpb, uint32_t blocks, size_t smem, size_t smem_limit,
+                                     cudaStream_t s)
 {
     const cudaError_t e = cudaFuncSetAttribute(k_sweep_random<R, LS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem);
+                                               (int)smem_limit);
     if (e != cudaSuccess) return e;
     k_sweep_random<R, LS><<<blocks, (cpb + 31u) / 32u * 32u, smem, s>>>(a, cpb);
     return cudaGetLastError();
@@ -203,10 +204,11 @@ cudaError_t launch_sweep_random(const RandomArgs &a, uint32_t cpb, uint32_t bloc
     // (512 B of the opt-in limit stay free for the kernel's static shared memory)
     const bool ls = random_sweep_smem(a.L, cpb, true) + 512 <= smem_optin;
     const size_t smem = random_sweep_smem(a.L, cpb, ls);
-    if (smem > smem_optin) return cudaErrorInvalidValue;
+    if (smem + 512 > smem_optin) return cudaErrorInvalidValue;
+    const size_t limit = smem_optin - 512;
     if (rounds == 10)
-        return ls ? launch_random_one<10, true>(a, cpb, blocks, smem, s) : launch_random_one<10, false>(a, cpb, blocks, smem, s);
-    return ls ? launch_random_one<7, true>(a, cpb, blocks, smem, s) : launch_random_one<7, false>(a, cpb, blocks, smem, s);
+        return ls ? launch_random_one<10, true>(a, cpb, blocks, smem, limit, s) : launch_random_one<10, false>(a, cpb, blocks, smem, limit, s);
+    return ls ? launch_random_one<7, true>(a, cpb, blocks, smem, limit, s) : launch_random_one<7, false>(a, cpb, blocks, smem, limit, s);
 }
 
 }  // namespace muca

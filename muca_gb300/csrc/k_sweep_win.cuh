@@ -31,7 +31,7 @@ cudaError_t launch_sweep_win(const SweepPlan &p, const SweepArgs &a, cudaStream_
     } else {
         kern = p.lat_smem ? k_sweep_win<MODE, R, true, false, false, false> : k_sweep_win<MODE, R, false, false, false, false>;
     }
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem_limit);
     if (e != cudaSuccess) return e;
     kern<<<p.blocks, p.threads, p.smem, s>>>(a, p.cpb);
     return cudaGetLastError();

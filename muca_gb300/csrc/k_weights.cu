@@ -548,9 +548,9 @@ static size_t update_smem(uint32_t N, int rule) { return rule == 2 ? (size_t)N *
 
 static cudaError_t prep_update(uint32_t N, int rule)
 {
-    const size_t dyn = update_smem(N, rule);
-    if (dyn > 48 * 1024)
-        return cudaFuncSetAttribute(k_weight_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+    if (update_smem(N, rule) > 48 * 1024)
+        return cudaFuncSetAttribute(k_weight_update, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)update_smem(16384, 2));
     return cudaSuccess;
 }
 
@@ -576,9 +576,11 @@ cudaError_t launch_run_update(const unsigned long long *hist, double *lnw, float
 
 cudaError_t prepare_batch_update(uint32_t max_N, int any_recursion)
 {
-    const size_t dyn = any_recursion ? update_smem(max_N, 2) : 0;
-    if (dyn > 48 * 1024)
-        return cudaFuncSetAttribute(k_batch_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+    // the limit of the largest size, whatever this batch's: another batch of the
+    // process shares the kernel
+    if (any_recursion && update_smem(max_N, 2) > 48 * 1024)
+        return cudaFuncSetAttribute(k_batch_update, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)update_smem(16384, 2));
     return cudaSuccess;
 }
 

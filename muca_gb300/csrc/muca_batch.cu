@@ -232,7 +232,8 @@ muca_status apply_shape(muca_batch *b, const muca_batch_shape &s, uint32_t rule)
     if (muca_status st = set_layout(b, s.chains_per_block, rule)) return st;
     const size_t smem = shape_smem(b, s.chains_per_block, s.lattice_in_smem, s.hist_in_smem);
     int per_sm = 0;
-    BCUDA(b, batch_sweep_occupancy(s.chains_per_block, b->rounds, s.lattice_in_smem, s.hist_in_smem, smem, &per_sm));
+    BCUDA(b, batch_sweep_occupancy(s.chains_per_block, b->rounds, s.lattice_in_smem, s.hist_in_smem, smem, smem_budget(b),
+                                   &per_sm));
     if (per_sm < 1) return bfail(b, MUCA_ERR_BAD_ARG, "shape does not fit on an SM");
     b->shape = s;
     b->shape.blocks_per_sm = (uint32_t)per_sm;
@@ -329,7 +330,7 @@ muca_status sweep_once(muca_batch *b)
     BCUDA(b, launch_batch_prep(b->d_inst, b->n, b->d_counters, b->d_counters + 1, b->stream));
     BCUDA(b, launch_batch_sweep(b->d_inst, b->d_items, b->n_items, b->d_counters, b->shape.chains_per_block,
                                 b->rounds, b->shape.lattice_in_smem, b->shape.hist_in_smem, b->grid, b->smem,
-                                b->stream));
+                                smem_budget(b), b->stream));
     return MUCA_OK;
 }
 
@@ -618,7 +619,7 @@ muca_status muca_batch_run(muca_batch *b, const muca_batch_run_opts *o, muca_bat
             if (e == cudaSuccess)
                 e = launch_batch_sweep(b->d_inst, b->d_items, b->n_items, b->d_counters, b->shape.chains_per_block,
                                        b->rounds, b->shape.lattice_in_smem, b->shape.hist_in_smem, b->grid, b->smem,
-                                       b->stream);
+                                       smem_budget(b), b->stream);
             if (e == cudaSuccess) e = launch_batch_update(b->d_inst, b->n, b->max_N, rec, b->d_counters + 1, b->stream);
         }
         cudaGraph_t g = nullptr;

@@ -65,6 +65,8 @@ struct SweepPlan {
     uint32_t threads;  // threads per block
     uint32_t blocks;
     size_t smem;     // dynamic shared memory bytes
+    size_t smem_limit;  // the limit the launch raises its kernel to: the same for every plan of a device,
+                        // so that no other context or thread can lower it between the two calls
 };
 // Warp-specialised sweep: ring slots per warp pair (the producer runs at most
 // this many decoded windows ahead), and u32 words per slot and lane.
@@ -224,14 +226,15 @@ enum BatchLattice : uint32_t { kLatGlobal = 0, kLatShared = 1, kLatWhereFits = 2
 // `smem` bytes.
 cudaError_t launch_batch_sweep(const BatchInst *insts, const BatchItem *items, uint32_t n_items, uint32_t *next_item,
                                uint32_t cpb, int rounds, uint32_t lat, bool hist_smem, uint32_t grid, size_t smem,
-                               cudaStream_t s);
+                               size_t smem_limit, cudaStream_t s);
 // Dynamic shared memory of one batch sweep block for an instance of size L,
 // with its lattice, or without it (then optionally with its four-row ring).
 size_t batch_sweep_smem(uint32_t L, uint32_t cpb, bool lat_smem, bool hist_smem, bool row_ring = false);
 // Blocks of the batch sweep that fit on one SM with `smem` bytes each; also
 // sets the kernel's shared-memory limit to `smem` (call before any capture).
 // The launch with that shape needs no further attribute call.
-cudaError_t batch_sweep_occupancy(uint32_t cpb, int rounds, uint32_t lat, bool hist_smem, size_t smem, int *blocks);
+cudaError_t batch_sweep_occupancy(uint32_t cpb, int rounds, uint32_t lat, bool hist_smem, size_t smem,
+                                  size_t smem_limit, int *blocks);
 // Sets the update kernel's shared-memory limit (call before any capture).
 cudaError_t prepare_batch_update(uint32_t max_N, int any_recursion);
 // The update step of every instance; *running += instances not stopped.

@@ -180,3 +180,19 @@ def test_batch_autotuner_table(muca):
     assert info.grid % 152 == 0 or info.grid > 0
     assert info.n_items == sum((nc + info.shape.chains_per_block - 1) // info.shape.chains_per_block
                                for _, nc, _, _ in INSTANCES)
+
+
+@pytest.mark.gpu
+def test_two_batches_share_a_kernel(muca):
+    """A batch's launches do not depend on the sizes of another batch made
+    after it (the two share a kernel and its shared-memory limit)."""
+    big, small = [(96, 64, 2.0, 0), (72, 64, 2.0, 1)], [(16, 64, 2.0, 0)]
+    opts = dict(starting_M=64, max_iter=4, graph_iters=2)
+    with muca.Batch(big, shape=(64, 0, 1)) as b:
+        b.run(**opts)
+        alone = [b.get_weights(i) for i in range(2)]
+    with muca.Batch(big, shape=(64, 0, 1)) as b, muca.Batch(small, shape=(64, 0, 1)) as c:
+        c.run(**opts)
+        b.run(**opts)
+        for i in range(2):
+            np.testing.assert_array_equal(b.get_weights(i), alone[i])
