@@ -270,10 +270,10 @@ cudaError_t launch_observables_static(int device, const unsigned long long *hist
 size_t mlp_param_count();
 cudaError_t mlp_prepare();  // shared-memory limits (call before any capture)
 // scratch floats of a minibatch of B points: Xb [B][4] at 0, Tb [B] at 4B,
-// Y [B] at 5B, then (aligned) Z, dZ and partials
+// Y [B] at 5B, then (aligned) activations, deltas and partials
 size_t mlp_scratch_floats(uint32_t B);
-// Y[0..B) = net(Xb) (Z: pre-activations [3][B][128] or NULL)
-cudaError_t launch_mlp_forward(const float *P, const float *Xb, uint32_t B, float *Z, float *Y, cudaStream_t s);
+// Y[0..B) = net(Xb)
+cudaError_t launch_mlp_forward(const float *P, const float *Xb, uint32_t B, float *Y, cudaStream_t s);
 // Gradient of the mean squared error on a minibatch (drawn from (X, T, n)
 // when gather, else already in scratch) into G; with m and v also one Adam
 // step; the loss goes to losses[*step - *base] (or losses[0] without step).

@@ -23,7 +23,7 @@ struct muca_mlp {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     float *d_P = nullptr, *d_G = nullptr, *d_m = nullptr, *d_v = nullptr;
-    uint32_t *d_step = nullptr;  // [0] step count, [1] step count at the start of train()
+    uint32_t *d_step = nullptr;  // [0] step count, [1] step count at the start of train(), [2] of the step in hand
     float *d_X = nullptr, *d_T = nullptr;
     uint32_t n_data = 0;
     float *d_scratch = nullptr;
@@ -135,7 +135,7 @@ muca_status reset_optimizer(muca_mlp *m)
     const size_t np = mlp_param_count();
     MCUDA(m, cudaMemsetAsync(m->d_m, 0, np * sizeof(float), m->stream));
     MCUDA(m, cudaMemsetAsync(m->d_v, 0, np * sizeof(float), m->stream));
-    MCUDA(m, cudaMemsetAsync(m->d_step, 0, 2 * sizeof(uint32_t), m->stream));
+    MCUDA(m, cudaMemsetAsync(m->d_step, 0, 3 * sizeof(uint32_t), m->stream));
     return MUCA_OK;
 }
 
@@ -176,7 +176,7 @@ muca_status muca_mlp_create(int32_t device, uint64_t seed, void *stream, muca_ml
     MTRY(cudaMalloc(&m->d_G, np * sizeof(float)));
     MTRY(cudaMalloc(&m->d_m, np * sizeof(float)));
     MTRY(cudaMalloc(&m->d_v, np * sizeof(float)));
-    MTRY(cudaMalloc(&m->d_step, 2 * sizeof(uint32_t)));
+    MTRY(cudaMalloc(&m->d_step, 3 * sizeof(uint32_t)));
     MTRY(mlp_prepare());
     const std::vector<float> p = init_params(seed);
     MTRY(cudaMemcpyAsync(m->d_P, p.data(), np * sizeof(float), cudaMemcpyHostToDevice, m->stream));
@@ -320,7 +320,7 @@ muca_status muca_mlp_predict(muca_mlp *m, const float *x, uint32_t n, float *y)
     if (muca_status st = ensure_scratch(m, n)) return st;
     float *Xb = m->d_scratch, *Y = Xb + (size_t)n * 4 + n;
     MCUDA(m, cudaMemcpyAsync(Xb, x, (size_t)n * 4 * sizeof(float), cudaMemcpyHostToDevice, m->stream));
-    MCUDA(m, launch_mlp_forward(m->d_P, Xb, n, nullptr, Y, m->stream));
+    MCUDA(m, launch_mlp_forward(m->d_P, Xb, n, Y, m->stream));
     MCUDA(m, cudaMemcpyAsync(y, Y, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
     MCUDA(m, cudaStreamSynchronize(m->stream));
     return MUCA_OK;
