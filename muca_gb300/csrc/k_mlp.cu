@@ -222,6 +222,19 @@ __device__ __forceinline__ void columns_product(const float *__restrict__ W, con
             for (int q = 0; q < 4; ++q) acc[a][q] = fmaf(wv[a], dv[q], acc[a][q]);
     }
 }
+// Starts copying W [kHid][kHid] to sW [kHid][kPitch] as one cp.async group.
+__device__ __forceinline__ void stage_async(const float *__restrict__ W, float *sW)
+{
+    for (int t = threadIdx.x; t < kHid * kHid / 4; t += kThreads) {
+        const int o = (4 * t) / kHid, j = 4 * t - o * kHid;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                         (uint32_t)__cvta_generic_to_shared(sW + o * kPitch + j)),
+                     "l"(W + 4 * t)
+                     : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
 // Forward and backward pass of the minibatch, one tile of 32 points per block.
 // Point k is row k of (X, T), or with a step number row
 // minibatch_index(k) of n.  Leaves the inputs in Xb [B][kIn], the activations
@@ -262,11 +275,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_points(const float *__restr
         reinterpret_cast<float4 *>(sx)[tid] = x;
         st[tid] = t;
     }
-    for (int t = tid; t < kHid * kHid / 4; t += kThreads) {
-        const int o = (4 * t) / kHid, j = 4 * t - o * kHid;
-        *reinterpret_cast<float4 *>(sW2 + o * kPitch + j) = reinterpret_cast<const float4 *>(P + kOffW2)[t];
-        *reinterpret_cast<float4 *>(sW3 + o * kPitch + j) = reinterpret_cast<const float4 *>(P + kOffW3)[t];
-    }
+    // both matrices on their way (one group each), waited for where they are used
+    stage_async(P + kOffW2, sW2);
+    stage_async(P + kOffW3, sW3);
     __syncthreads();
     // layer l's activations h of this thread's units and points, to global memory
     auto keep = [&](int l, const float (&h)[4][4]) {
@@ -292,6 +303,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_points(const float *__restr
         *reinterpret_cast<float4 *>(d1 + o * kPtPitch + b0) = make_float4(d[a][0], d[a][1], d[a][2], d[a][3]);
     }
     keep(1, h);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncthreads();
     // layer 2
 #pragma unroll
@@ -310,6 +322,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_points(const float *__restr
         *reinterpret_cast<float4 *>(d2 + o * kPtPitch + b0) = make_float4(d[a][0], d[a][1], d[a][2], d[a][3]);
     }
     keep(2, h);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     // layer 3, over layer 1's activations; its derivatives stay in registers
 #pragma unroll
@@ -395,11 +408,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_points(const float *__restr
     }
 }
 
-// Weight gradients of slice blockIdx.y of the minibatch, summed over its
-// points in order, into part + blockIdx.y * kPartPitch.  Blocks 0..7: a 64 x
+// Weight gradients of slice blockIdx.x of the minibatch, summed over its
+// points in order, into part + blockIdx.x * kPartPitch.  blockIdx.y 0..7: a 64 x
 // 64 tile of layer 2 (0..3) or 3 (4..7), 4 x 4 outputs per thread, chunks of
 // 32 points in shared memory, the next chunk's loads in flight meanwhile;
-// block 8: layers 1 and 4.  128 + 16 blocks fill the GPU once.
+// 8 and 9: 64 units of layer 1, one input per thread, by the same chunks;
+// 10: layer 4.  The 128 blocks of the large layers come first, one per SM; the
+// small ones fill the rest.
 constexpr int kWTile = 64, kWChunk = 32;
 __global__ void __launch_bounds__(256) k_mlp_wgrad(const float *__restrict__ Xb, const float *__restrict__ H,
                                                    const float *__restrict__ D, const float *__restrict__ Dy,
@@ -408,31 +423,22 @@ __global__ void __launch_bounds__(256) k_mlp_wgrad(const float *__restrict__ Xb,
     __shared__ __align__(16) float sD[2][kWChunk][kWTile], sH[2][kWChunk][kWTile];
     const int tid = threadIdx.x;
     const uint32_t slice = (B + kWSplit - 1) / kWSplit;
-    const uint32_t c0 = min(B, blockIdx.y * slice), c1 = min(B, c0 + slice);
-    float *g = part + (size_t)blockIdx.y * kPartPitch;
-    if (blockIdx.x == 8) {
-        // layer 1: outputs (o, i), i < 4 the inputs and i = 4 the bias; then
-        // layer 4: its weights and, output 128, its bias
-        for (int t = tid; t < kHid * (kIn + 1); t += 256) {
-            const int i = t / kHid, o = t - i * kHid;
-            float acc = 0.0f;
-#pragma unroll 8
-            for (uint32_t p = c0; p < c1; ++p)
-                acc = fmaf(D[(size_t)p * kHid + o], i < kIn ? Xb[(size_t)p * kIn + i] : 1.0f, acc);
-            if (i < kIn) g[kOffW1 + o * kIn + i] = acc;
-            else g[kOffB1 + o] = acc;
-        }
+    const uint32_t c0 = min(B, blockIdx.x * slice), c1 = min(B, c0 + slice);
+    float *g = part + (size_t)blockIdx.x * kPartPitch;
+    if (blockIdx.y == 10) {  // output 128 is the bias, which follows the weights
         if (tid <= kHid) {
             float acc = 0.0f;
-#pragma unroll 8
+#pragma unroll 32
             for (uint32_t p = c0; p < c1; ++p)
                 acc = fmaf(Dy[p], tid < kHid ? H[((size_t)2 * B + p) * kHid + tid] : 1.0f, acc);
-            g[kOffW4 + tid] = acc;  // the bias follows the weights
+            g[kOffW4 + tid] = acc;
         }
         return;
     }
-    const int l = blockIdx.x >> 2, o0 = (blockIdx.x >> 1 & 1) * kWTile, i0 = (blockIdx.x & 1) * kWTile;
-    const float *Dl = D + (size_t)(l + 1) * B * kHid + o0, *Hl = H + (size_t)l * B * kHid + i0;
+    const bool first = blockIdx.y >= 8;  // layer 1
+    const int l = blockIdx.y >> 2, o0 = first ? (blockIdx.y & 1) * kWTile : (blockIdx.y >> 1 & 1) * kWTile;
+    const int i0 = first ? 0 : (blockIdx.y & 1) * kWTile;
+    const float *Dl = D + (first ? 0 : (size_t)(l + 1) * B * kHid) + o0, *Hl = first ? Xb : H + (size_t)l * B * kHid + i0;
     const int ti = tid & 15, to = tid >> 4;
     // thread's share of a chunk: rows r and r + 16, 4 columns
     const int r = tid >> 4, c = 4 * (tid & 15);
@@ -444,7 +450,8 @@ __global__ void __launch_bounds__(256) k_mlp_wgrad(const float *__restrict__ Xb,
             nd[k] = nh[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             if (q < c1) {
                 nd[k] = *reinterpret_cast<const float4 *>(Dl + (size_t)q * kHid + c);
-                nh[k] = *reinterpret_cast<const float4 *>(Hl + (size_t)q * kHid + c);
+                if (!first) nh[k] = *reinterpret_cast<const float4 *>(Hl + (size_t)q * kHid + c);
+                else if (c == 0) nh[k] = *reinterpret_cast<const float4 *>(Hl + (size_t)q * kIn);
             }
         }
     };
@@ -463,18 +470,29 @@ __global__ void __launch_bounds__(256) k_mlp_wgrad(const float *__restrict__ Xb,
         }
         __syncthreads();  // two buffers: the chunk before last has been read by every thread
         fetch(p + kWChunk);
+        if (first) {
 #pragma unroll 8
-        for (int k = 0; k < kWChunk; ++k) {
-            const float4 x = *reinterpret_cast<const float4 *>(&sD[buf][k][4 * to]);
-            const float4 y = *reinterpret_cast<const float4 *>(&sH[buf][k][4 * ti]);
-            const float xv[4] = {x.x, x.y, x.z, x.w}, yv[4] = {y.x, y.y, y.z, y.w};
+            for (int k = 0; k < kWChunk; ++k) acc[0][0] = fmaf(sD[buf][k][tid & 63], sH[buf][k][tid >> 6], acc[0][0]);
+        } else {
+#pragma unroll 8
+            for (int k = 0; k < kWChunk; ++k) {
+                const float4 x = *reinterpret_cast<const float4 *>(&sD[buf][k][4 * to]);
+                const float4 y = *reinterpret_cast<const float4 *>(&sH[buf][k][4 * ti]);
+                const float xv[4] = {x.x, x.y, x.z, x.w}, yv[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
+                for (int a = 0; a < 4; ++a)
 #pragma unroll
-                for (int b = 0; b < 4; ++b) acc[a][b] = fmaf(xv[a], yv[b], acc[a][b]);
+                    for (int b = 0; b < 4; ++b) acc[a][b] = fmaf(xv[a], yv[b], acc[a][b]);
+            }
         }
         if (i0 == 0 && tid < kWTile)
+#pragma unroll
             for (int k = 0; k < kWChunk; ++k) bias += sD[buf][k][tid];
+    }
+    if (first) {
+        g[kOffW1 + (o0 + (tid & 63)) * kIn + (tid >> 6)] = acc[0][0];
+        if (tid < kWTile) g[kOffB1 + o0 + tid] = bias;
+        return;
     }
     float *gW = g + (l == 0 ? kOffW2 : kOffW3), *gb = g + (l == 0 ? kOffB2 : kOffB3);
 #pragma unroll
@@ -588,7 +606,7 @@ cudaError_t launch_mlp_step(float *P, float *G, float *m, float *v, const float 
     uint32_t *st = gather ? step : nullptr;
     k_mlp_points<<<nt, kThreads, points_smem(), s>>>(P, gather ? X : sc.Xb, gather ? T : sc.Tb, n, B, st, seed, sc.Xb,
                                                      sc.H, sc.D, sc.Dy, sc.lpart);
-    k_mlp_wgrad<<<dim3(9, kWSplit), 256, 0, s>>>(sc.Xb, sc.H, sc.D, sc.Dy, B, sc.part);
+    k_mlp_wgrad<<<dim3(kWSplit, 11), 256, 0, s>>>(sc.Xb, sc.H, sc.D, sc.Dy, B, sc.part);
     k_mlp_update<<<(kParams + 255) / 256, 256, 0, s>>>(sc.part, sc.lpart, nt, B, P, G, m, v, st, base, lr, losses,
                                                        losses_cap);
     return cudaGetLastError();
