@@ -34,6 +34,7 @@ struct muca_ctx {
     float *d_w32 = nullptr;
     unsigned long long *d_hist = nullptr;
     uint32_t *d_index = nullptr, *d_naver = nullptr;
+    // the statistics and, behind them, the error word: one copy brings both
     HistStatsDev *d_stats = nullptr, *h_stats = nullptr;
     UpdScratch *d_upd = nullptr;  // the multi-block weight update
     RunCtl *d_ctl = nullptr, *h_ctl = nullptr;
@@ -89,10 +90,10 @@ void free_all(muca_ctx *c)
 {
     void *dp[] = {c->d_lat, c->d_ej, c->d_edel, c->d_mag, c->d_lnw, c->d_lnw_obs, c->d_pacc, c->d_w32, c->d_hist,
                   c->d_index, c->d_naver, c->d_stats, c->d_ctl, c->d_recs, c->d_obs_part, c->d_obs_out,
-                  c->d_jk, c->d_tmp, c->d_bad, c->d_err, c->d_logf_tab, c->d_upd, c->rec.ds, c->rec.valid};
+                  c->d_jk, c->d_tmp, c->d_bad, c->d_logf_tab, c->d_upd, c->rec.ds, c->rec.valid};
     for (void *p : dp)
         if (p) cudaFree(p);
-    void *hp[] = {c->h_stats, c->h_ctl, c->h_obs_out, c->h_bad, c->h_err};
+    void *hp[] = {c->h_stats, c->h_ctl, c->h_obs_out, c->h_bad};
     for (void *p : hp)
         if (p) cudaFreeHost(p);
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
@@ -129,9 +130,12 @@ muca_status recompute_energies(muca_ctx *c)
     return MUCA_OK;
 }
 
+// Synchronises and reports a wait that gave up; h_stats has the statistics
+// of the last update afterwards.
 muca_status check_err(muca_ctx *c)
 {
-    CUDA_TRY(c, cudaMemcpyAsync(c->h_err, c->d_err, sizeof(unsigned int), cudaMemcpyDeviceToHost, c->stream));
+    CUDA_TRY(c, cudaMemcpyAsync(c->h_stats, c->d_stats, sizeof(HistStatsDev) + sizeof(unsigned int),
+                                cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     if (*c->h_err) {
         const unsigned int e = *c->h_err;
@@ -311,7 +315,8 @@ muca_status muca_create(const muca_params *p, muca_ctx **out)
     CREATE_TRY(cudaMemsetAsync(c->d_lnw_obs, 0, ((size_t)N + 1) * 8, c->stream));
     CREATE_TRY(dmalloc(c, &c->d_w32, (size_t)N + 1));
     CREATE_TRY(dmalloc(c, &c->d_hist, c->hist_len));
-    CREATE_TRY(dmalloc(c, &c->d_stats, 1));
+    CREATE_TRY(dmalloc(c, &c->d_stats, 2));
+    c->d_err = reinterpret_cast<unsigned int *>(c->d_stats + 1);
     CREATE_TRY(dmalloc(c, &c->d_upd, 1));
     CREATE_TRY(cudaMemsetAsync(c->d_upd, 0, sizeof(UpdScratch), c->stream));
     if (c->mode == MUCA_MODE_WEIGHT) {
@@ -320,10 +325,9 @@ muca_status muca_create(const muca_params *p, muca_ctx **out)
     }
     CREATE_TRY(dmalloc(c, &c->d_ctl, 1));
     CREATE_TRY(dmalloc(c, &c->d_bad, 1));
-    CREATE_TRY(dmalloc(c, &c->d_err, 1));
-    CREATE_TRY(cudaMallocHost((void **)&c->h_err, sizeof(unsigned int)));
-    CREATE_TRY(cudaMemsetAsync(c->d_err, 0, sizeof(unsigned int), c->stream));
-    CREATE_TRY(cudaMallocHost((void **)&c->h_stats, sizeof(HistStatsDev)));
+    CREATE_TRY(cudaMemsetAsync(c->d_stats, 0, 2 * sizeof(HistStatsDev), c->stream));
+    CREATE_TRY(cudaMallocHost((void **)&c->h_stats, 2 * sizeof(HistStatsDev)));
+    c->h_err = reinterpret_cast<unsigned int *>(c->h_stats + 1);
     CREATE_TRY(cudaMallocHost((void **)&c->h_ctl, sizeof(RunCtl)));
     CREATE_TRY(cudaMallocHost((void **)&c->h_bad, sizeof(unsigned long long)));
     CREATE_TRY(cudaMallocHost((void **)&c->h_obs_out, 4 * sizeof(double)));
@@ -521,8 +525,7 @@ muca_status muca_set_weights(muca_ctx *c, const double *lnw, size_t n)
         if (!std::isfinite(lnw[i])) return fail(c, MUCA_ERR_BAD_ARG, "weight %zu is not finite", i);
     CUDA_TRY(c, cudaSetDevice(c->device));
     CUDA_TRY(c, cudaMemcpyAsync(c->d_lnw, lnw, n * 8, cudaMemcpyHostToDevice, c->stream));
-    CUDA_TRY(c, cudaMemcpyAsync(c->d_lnw_obs, c->d_lnw, n * 8, cudaMemcpyDeviceToDevice, c->stream));
-    CUDA_TRY(c, launch_weights_to_f32(c->d_lnw, c->d_w32, (uint32_t)n, c->stream));
+    CUDA_TRY(c, launch_weights_in(c->d_lnw, c->d_w32, c->d_lnw_obs, (uint32_t)n, nullptr, 0, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     return MUCA_OK;
 }
@@ -612,7 +615,6 @@ static muca_status update_impl(muca_ctx *c, int rule, muca_hist_stats *st)
     CUDA_TRY(c, launch_weight_update(c->d_hist, c->N, c->d_lnw, c->d_w32, c->d_pacc, rule, c->d_stats, c->stream, c->d_upd,
                                      &c->rec));
     if (!st) return MUCA_OK;  // enqueue only
-    CUDA_TRY(c, cudaMemcpyAsync(c->h_stats, c->d_stats, sizeof(HistStatsDev), cudaMemcpyDeviceToHost, c->stream));
     if (muca_status e = check_err(c)) return e;
     stats_out(*c->h_stats, st);
     return MUCA_OK;
@@ -645,13 +647,11 @@ muca_status muca_iterate_host(muca_ctx *c, const double *lnw_in, uint32_t iter, 
     if (lnw_in) {
         // read by the stream before this call returns (it synchronises below)
         CUDA_TRY(c, cudaMemcpyAsync(c->d_lnw, lnw_in, n * 8, cudaMemcpyHostToDevice, c->stream));
-        CUDA_TRY(c, cudaMemcpyAsync(c->d_lnw_obs, c->d_lnw, n * 8, cudaMemcpyDeviceToDevice, c->stream));
-        CUDA_TRY(c, launch_weights_to_f32(c->d_lnw, c->d_w32, (uint32_t)n, c->stream));
+        CUDA_TRY(c, launch_weights_in(c->d_lnw, c->d_w32, c->d_lnw_obs, (uint32_t)n, c->d_hist, (uint32_t)n, c->stream));
     }
-    if (muca_status e = do_sweep(c, iter, seed_base, seed_dev_mul, therm, nup, true)) return e;
+    if (muca_status e = do_sweep(c, iter, seed_base, seed_dev_mul, therm, nup, !lnw_in)) return e;
     CUDA_TRY(c, launch_weight_update(c->d_hist, c->N, c->d_lnw, c->d_w32, c->d_pacc, (int)rule, c->d_stats, c->stream,
                                      c->d_upd, &c->rec));
-    if (st) CUDA_TRY(c, cudaMemcpyAsync(c->h_stats, c->d_stats, sizeof(HistStatsDev), cudaMemcpyDeviceToHost, c->stream));
     if (lnw_out) CUDA_TRY(c, cudaMemcpyAsync(lnw_out, c->d_lnw, n * 8, cudaMemcpyDeviceToHost, c->stream));
     if (hist_out) CUDA_TRY(c, cudaMemcpyAsync(hist_out, c->d_hist, n * 8, cudaMemcpyDeviceToHost, c->stream));
     if (muca_status e = check_err(c)) return e;  // the one synchronisation
@@ -717,6 +717,8 @@ static muca_status run_impl(muca_ctx *c, const muca_run_opts *o, muca_run_result
     h.rec_cap = (uint32_t)need;
     h.rec_ring = cb ? 1u : 0u;
     CUDA_TRY(c, cudaMemcpyAsync(c->d_ctl, &h, sizeof h, cudaMemcpyHostToDevice, c->stream));
+    // each iteration's update clears the histogram for the next one
+    CUDA_TRY(c, cudaMemsetAsync(c->d_hist, 0, c->hist_len * 8, c->stream));
     // therm_coeff * N (:315-316); the CPU program's random-site runs thermalise 0 (muca_mag.cpp:140)
     const uint64_t therm = o->therm ? o->therm : (c->algo == MUCA_ALGO_RANDOM_SITE ? 0 : c->N);
     SweepArgs a = sweep_args(c, 0, 100u, 1000u, therm, 0);  // seed SEED+1000*l (:393)
@@ -734,16 +736,14 @@ static muca_status run_impl(muca_ctx *c, const muca_run_opts *o, muca_run_result
     muca_status rs = MUCA_OK;
     const bool graph_mode = o->graph_iters > 0 && !cb;
     if (graph_mode) {
-        // K iterations (clear, sweep, update) captured once and replayed; the
+        // K iterations (sweep, update) captured once and replayed; the
         // device stops them itself, so one host round trip serves K iterations
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
         cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed);
         const bool capturing = e == cudaSuccess;
         for (uint32_t j = 0; j < o->graph_iters && e == cudaSuccess; ++j) {
-            e = launch_run_clear(c->d_hist, (uint32_t)c->hist_len, c->d_ctl, c->stream);
-            if (e == cudaSuccess)
-                e = c->algo == MUCA_ALGO_RANDOM_SITE
+            e = c->algo == MUCA_ALGO_RANDOM_SITE
                         ? launch_sweep_random(ra, c->plan.cpb, c->plan.blocks, (int)c->rounds, c->smem_optin, c->stream)
                         : launch_sweep(c->plan, a, c->stream);
             if (e == cudaSuccess) e = launch_run_update(c->d_hist, c->d_lnw, c->d_w32, c->d_pacc, c->d_ctl, c->stream,
@@ -776,8 +776,7 @@ static muca_status run_impl(muca_ctx *c, const muca_run_opts *o, muca_run_result
     while (!graph_mode) {
         // one iteration per host round trip, like the reference loop; the
         // device decides the schedule and convergence
-        cudaError_t e = launch_run_clear(c->d_hist, (uint32_t)c->hist_len, c->d_ctl, c->stream);
-        if (e == cudaSuccess) e = cudaEventRecord(e0, c->stream);
+        cudaError_t e = cudaEventRecord(e0, c->stream);
         if (e == cudaSuccess)
             e = c->algo == MUCA_ALGO_RANDOM_SITE
                     ? launch_sweep_random(ra, c->plan.cpb, c->plan.blocks, (int)c->rounds, c->smem_optin, c->stream)

@@ -559,7 +559,8 @@ muca_status muca_batch_set_weights(muca_batch *b, uint32_t i, const double *lnw,
         if (!std::isfinite(lnw[k])) return bfail(b, MUCA_ERR_BAD_ARG, "weight %zu is not finite", k);
     BCUDA(b, cudaSetDevice(b->device));
     BCUDA(b, cudaMemcpyAsync(b->d_lnw + b->off_w[i], lnw, n * 8, cudaMemcpyHostToDevice, b->stream));
-    BCUDA(b, launch_weights_to_f32(b->d_lnw + b->off_w[i], b->d_w32 + b->off_w[i], (uint32_t)n, b->stream));
+    BCUDA(b, launch_weights_in(b->d_lnw + b->off_w[i], b->d_w32 + b->off_w[i], nullptr, (uint32_t)n, nullptr, 0,
+                               b->stream));
     BCUDA(b, cudaMemsetAsync(b->d_pacc + b->off_w[i], 0, n * 8, b->stream));
     BCUDA(b, cudaStreamSynchronize(b->stream));
     return MUCA_OK;

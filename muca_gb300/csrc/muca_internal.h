@@ -157,7 +157,7 @@ struct UpdPart {
 struct UpdScratch {
     UpdPart part[kUpdBlocks];
     unsigned int done;
-    int upd;
+    int upd, clear;
     double tmp;
     int start, end;  // the histogram's range (bins with H > 1), for the recursion
 };
@@ -172,7 +172,7 @@ struct RecScratch {
 // (zero-initialised once) rules -1, 0 and 1 spread their FP64 work over
 // kUpdBlocks blocks, and so does rule 2 when `rs` is given too (its prefix
 // then runs as one block's segmented scan); otherwise one block does all.
-cudaError_t launch_weight_update(const unsigned long long *hist, uint32_t N, double *lnw, float *w32,
+cudaError_t launch_weight_update(unsigned long long *hist, uint32_t N, double *lnw, float *w32,
                                  double *p_acc, int rule, HistStatsDev *stats, cudaStream_t s,
                                  UpdScratch *sc = nullptr, const RecScratch *rs = nullptr);
 
@@ -243,12 +243,13 @@ cudaError_t launch_batch_update(const BatchInst *insts, uint32_t n_inst, uint32_
 
 // One iteration's tail: statistics, width/convergence bookkeeping, weight
 // update, schedule of the next NUPDATES; a no-op once st.stop is set.
-cudaError_t launch_run_update(const unsigned long long *hist, double *lnw, float *w32, double *p_acc,
+cudaError_t launch_run_update(unsigned long long *hist, double *lnw, float *w32, double *p_acc,
                               RunCtl *ctl, cudaStream_t s, uint32_t N, int rule, UpdScratch *sc = nullptr,
                               const RecScratch *rs = nullptr);
-// Clears the weight histogram unless the run has stopped.
-cudaError_t launch_run_clear(unsigned long long *hist, uint32_t n, const RunCtl *ctl, cudaStream_t s);
-cudaError_t launch_weights_to_f32(const double *lnw, float *w32, uint32_t n, cudaStream_t s);
+// After FP64 weights have arrived in lnw[0..n): the FP32 shadow, the copy obs
+// (unless NULL), and the histogram's first n_hist bins cleared.
+cudaError_t launch_weights_in(const double *lnw, float *w32, double *obs, uint32_t n, unsigned long long *hist,
+                              uint32_t n_hist, cudaStream_t s);
 
 // Production reweighting (k_observables.cu).
 cudaError_t launch_weight_shift(double *lnw, uint32_t N, double beta, double delta, cudaStream_t s);

@@ -163,3 +163,30 @@ def test_many_chains(muca, orc, L, nch, smem, produce):
         np.testing.assert_array_equal(lat1[lo:hi], a.reshape(hi - lo, N))
         np.testing.assert_array_equal(s1[0][lo:hi], st[0])
         np.testing.assert_array_equal(s1[1][lo:hi], st[1])
+
+
+# the update of one cluster (L <= 90) and of three launches (above), one and
+# two bins per thread, and bins at the edges of the cluster's strides
+@pytest.mark.gpu
+@pytest.mark.parametrize("L", [2, 8, 16, 30, 64, 66, 90, 92, 128])
+@pytest.mark.parametrize("rule", [0, 1])
+def test_update_over_a_cluster(muca, orc, L, rule):
+    N = L * L
+    rng = np.random.default_rng(L + rule)
+    h = rng.integers(0, 4, N + 1).astype(np.uint64) * rng.integers(0, 5000, N + 1).astype(np.uint64)
+    lnw = rng.normal(0.0, 50.0, N + 1)
+    with muca.Engine(L, nchains=32) as e:
+        e.set_weights(lnw)
+        e.set_histogram(h)
+        s = e.update_weights(rule)
+        w = e.get_weights()
+        assert np.array_equal(e.histogram(), h)
+    with np.errstate(divide="ignore"):
+        ln = np.log(h.astype(np.float64))
+    upd = h > (1 if rule == 0 else 0)
+    x = np.where(upd, lnw - ln, lnw)
+    x = x - x[0] if rule == 0 else np.where(h > 0, x - x[0], x)
+    np.testing.assert_allclose(w, x, rtol=1e-13, atol=1e-10)
+    assert (s.start, s.end) == orc.hist_range(h)
+    assert s.events == int(h.sum()) and s.visited == int((h > 0).sum()) and s.min_count == int(h.min())
+    np.testing.assert_allclose(s.d_kl, orc.kull_leibler(h), rtol=1e-11)
