@@ -29,6 +29,36 @@ __device__ __forceinline__ uint4 init_block(const InitArgs &ia, uint32_t W, uint
     return philox<R>(c[0], c[1], c[2], c[3], k);
 }
 
+// Word w of a chain's packed lattice.
+template <int R>
+__device__ __forceinline__ uint32_t init_word(const InitArgs &ia, uint32_t L, uint32_t WPR, uint32_t w, uint32_t chain,
+                                              uint32_t nchains, uint32_t chains_per_dev, uint32_t jack)
+{
+    if (chain >= nchains) return kZeroWord;
+    const uint32_t dev = chain / chains_per_dev, W = chain - dev * chains_per_dev;
+    const uint32_t row = w / WPR, q = w - row * WPR;
+    const uint32_t c_lo = 16u * q, c_hi = min(16u * q + 16u, L);
+    uint32_t word = 0;
+    uint32_t g_cur = 0xFFFFFFFFu;
+    uint4 r = make_uint4(0, 0, 0, 0);
+    for (uint32_t col = c_lo; col < c_hi; ++col) {
+        int s;
+        if (ia.ordered) {
+            s = 1;
+        } else {
+            const uint32_t site = row * L + col, g = site >> 2;
+            if (g != g_cur) {
+                r = init_block<R>(ia, W, dev, chain, jack, g);
+                g_cur = g;
+            }
+            const uint32_t rw = pick(r, (int)(site & 3u));
+            s = ia.graded ? graded_spin(rw, W, chains_per_dev) : init_spin(rw);
+        }
+        word |= (uint32_t)(s + 1) << (2u * (col - c_lo));
+    }
+    return word;
+}
+
 template <int R>
 __global__ void k_init(uint32_t *lat, uint32_t L, uint32_t WPR, uint32_t cpb, uint32_t nchains,
                        uint32_t chains_per_dev, uint32_t jack, InitArgs ia)
@@ -50,32 +80,24 @@ __global__ void k_init(uint32_t *lat, uint32_t L, uint32_t WPR, uint32_t cpb, ui
             blk = (uint32_t)(bw / words);
             w = (uint32_t)(bw - (size_t)blk * words);
         }
-        const uint32_t chain = blk * cpb + lane;
-        uint32_t word = kZeroWord;
-        if (chain < nchains) {
-            const uint32_t dev = chain / chains_per_dev, W = chain - dev * chains_per_dev;
-            const uint32_t row = w / WPR, q = w - row * WPR;
-            const uint32_t c_lo = 16u * q, c_hi = min(16u * q + 16u, L);
-            word = 0;
-            uint32_t g_cur = 0xFFFFFFFFu;
-            uint4 r = make_uint4(0, 0, 0, 0);
-            for (uint32_t col = c_lo; col < c_hi; ++col) {
-                int s;
-                if (ia.ordered) {
-                    s = 1;
-                } else {
-                    const uint32_t site = row * L + col, g = site >> 2;
-                    if (g != g_cur) {
-                        r = init_block<R>(ia, W, dev, chain, jack, g);
-                        g_cur = g;
-                    }
-                    const uint32_t rw = pick(r, (int)(site & 3u));
-                    s = ia.graded ? graded_spin(rw, W, chains_per_dev) : init_spin(rw);
-                }
-                word |= (uint32_t)(s + 1) << (2u * (col - c_lo));
-            }
-        }
-        lat[t] = word;
+        lat[t] = init_word<R>(ia, L, WPR, w, blk * cpb + lane, nchains, chains_per_dev, jack);
+    }
+}
+
+// The lattices of a batch's instances: blockIdx.x = work item, the words of
+// its chain block spread over blockIdx.y; emulated device index = the
+// instance's seed.
+__global__ void k_batch_init(const BatchInst *__restrict__ insts, const BatchItem *__restrict__ items, uint32_t cpb,
+                             InitArgs ia)
+{
+    const BatchItem it = items[blockIdx.x];
+    const BatchInst &I = insts[it.inst];
+    const uint32_t L = I.a.L, WPR = I.a.WPR, words = L * WPR, nch = I.a.nchains;
+    ia.ctr0[0] += ia.ctr0_dev_mul[0] * I.seed;
+    uint32_t *lat = I.a.lat + (size_t)it.blk * words * cpb;
+    for (uint32_t t = blockIdx.y * blockDim.x + threadIdx.x; t < words * cpb; t += gridDim.y * blockDim.x) {
+        const uint32_t w = t / cpb, lane = t - w * cpb;
+        lat[t] = init_word<7>(ia, L, WPR, w, it.blk * cpb + lane, nch, nch, 0);
     }
 }
 
@@ -123,30 +145,75 @@ __global__ void k_unpack(const uint32_t *lat, int8_t *dst, uint32_t L, uint32_t 
 // E_J = -sum over bonds (right and up neighbour of every site), which equals
 // total_energy of muca_delta_multigpu.cu:563-571 (the sum over all four
 // neighbours, halved), E_Delta = sum s^2, M = sum s.
-__global__ void k_energies(const uint32_t *lat, int32_t *ej, int32_t *edel, int32_t *mag, uint32_t L, uint32_t WPR,
-                           uint32_t cpb, uint32_t nchains)
+// A block of 32 x kEnergyRows threads takes 32 chains, thread (x, y) rows y,
+// y + kEnergyRows, ... of chain x, whole words at a time: a code is nonzero
+// where its low bit is clear, its high bit the sign, so a word's 16 bonds are
+// two population counts.  (Site by site, one thread per chain, L = 128 took
+// 300 us however few the chains.)
+constexpr uint32_t kEnergyRows = 8;
+__device__ __forceinline__ void chain_energies(const uint32_t *base, uint32_t L, uint32_t WPR, uint32_t cpb, bool on,
+                                               int32_t *ej, int32_t *edel, int32_t *mag)
 {
-    const uint32_t chain = blockIdx.x * blockDim.x + threadIdx.x;
-    if (chain >= nchains) return;
-    const uint32_t words = L * WPR;
-    const uint32_t *base = lat + (size_t)(chain / cpb) * words * cpb + (chain % cpb);
-    auto get = [&](uint32_t r, uint32_t c) -> int {
-        return (int)spin_code(base[(size_t)(r * WPR + (c >> 4)) * cpb], c) - 1;
-    };
+    __shared__ int sh[3][kEnergyRows][32];
+    const uint32_t x = threadIdx.x & 31u, y = threadIdx.x >> 5;
+    const uint32_t last = L - 16u * (WPR - 1u);  // sites of a row's last word
     int bonds = 0, d = 0, m = 0;
-    for (uint32_t r = 0; r < L; ++r) {
-        const uint32_t ru = (r + 1 == L) ? 0 : r + 1;
-        for (uint32_t c = 0; c < L; ++c) {
-            const int s = get(r, c);
-            const uint32_t cr = (c + 1 == L) ? 0 : c + 1;
-            bonds += s * (get(r, cr) + get(ru, c));
-            d += s * s;
-            m += s;
+    auto pairs = [](uint32_t nz, uint32_t a, uint32_t b) -> int {
+        const uint32_t both = nz & ~b;
+        return __popc(both) - 2 * __popc(both & ((a ^ b) >> 1));
+    };
+    for (uint32_t r = y; on && r < L; r += kEnergyRows) {
+        const uint32_t *row = base + (size_t)(r * WPR) * cpb;
+        const uint32_t *up = base + (size_t)((r + 1 == L ? 0u : r + 1u) * WPR) * cpb;
+        const uint32_t first = row[0];
+        uint32_t C = first;
+        for (uint32_t q = 0; q < WPR; ++q) {
+            const bool end = q + 1 == WPR;
+            const uint32_t next = end ? first : row[(size_t)(q + 1) * cpb], U = up[(size_t)q * cpb];
+            const uint32_t valid = end && last < 16u ? (1u << (2u * last)) - 1u : ~0u;
+            const uint32_t nz = ~C & valid & 0x55555555u;
+            const uint32_t right = end ? ((C & valid) >> 2) | (first << (2u * last - 2u)) : (C >> 2) | (next << 30);
+            bonds += pairs(nz, C, right) + pairs(nz, C, U);
+            const int n = __popc(nz);
+            d += n;
+            m += 2 * __popc(nz & (C >> 1)) - n;
+            C = next;
         }
     }
-    ej[chain] = -bonds;
-    edel[chain] = d;
-    if (mag) mag[chain] = m;
+    sh[0][y][x] = bonds;
+    sh[1][y][x] = d;
+    sh[2][y][x] = m;
+    __syncthreads();
+    if (y < 3 && on) {
+        int v = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < kEnergyRows; ++k) v += sh[y][k][x];
+        if (y == 0) *ej = -v;
+        else if (y == 1) *edel = v;
+        else if (mag) *mag = v;
+    }
+}
+__global__ void __launch_bounds__(32 * kEnergyRows) k_energies(const uint32_t *lat, int32_t *ej, int32_t *edel,
+                                                               int32_t *mag, uint32_t L, uint32_t WPR, uint32_t cpb,
+                                                               uint32_t nchains)
+{
+    const uint32_t chain = blockIdx.x * 32u + (threadIdx.x & 31u);
+    const bool on = chain < nchains;
+    const uint32_t c = on ? chain : 0u;
+    chain_energies(lat + (size_t)(c / cpb) * L * WPR * cpb + c % cpb, L, WPR, cpb, on, ej + c, edel + c,
+                   mag ? mag + c : nullptr);
+}
+// blockIdx.x = work item of a batch, blockIdx.y = 32 of its chains
+__global__ void __launch_bounds__(32 * kEnergyRows) k_batch_energies(const BatchInst *__restrict__ insts,
+                                                                     const BatchItem *__restrict__ items, uint32_t cpb)
+{
+    const BatchItem it = items[blockIdx.x];
+    const SweepArgs &a = insts[it.inst].a;
+    const uint32_t lane = blockIdx.y * 32u + (threadIdx.x & 31u), chain = it.blk * cpb + lane;
+    const bool on = lane < cpb && chain < a.nchains;
+    const uint32_t c = on ? chain : 0u;
+    chain_energies(a.lat + (size_t)it.blk * a.L * a.WPR * cpb + (on ? lane : 0u), a.L, a.WPR, cpb, on, a.ej + c,
+                   a.edel + c, a.mag + c);
 }
 
 __global__ void k_validate(const int8_t *src, size_t n, unsigned long long *bad)
@@ -195,7 +262,15 @@ cudaError_t launch_unpack(const uint32_t *lat, int8_t *dst, uint32_t L, uint32_t
 cudaError_t launch_energies(const uint32_t *lat, int32_t *ej, int32_t *edel, int32_t *mag, uint32_t L, uint32_t WPR,
                             uint32_t cpb, uint32_t nchains, cudaStream_t s)
 {
-    k_energies<<<(nchains + 127) / 128, 128, 0, s>>>(lat, ej, edel, mag, L, WPR, cpb, nchains);
+    k_energies<<<(nchains + 31) / 32, 32 * kEnergyRows, 0, s>>>(lat, ej, edel, mag, L, WPR, cpb, nchains);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_batch_init(const BatchInst *insts, const BatchItem *items, uint32_t n_items, uint32_t cpb,
+                              const InitArgs &ia, cudaStream_t s)
+{
+    k_batch_init<<<dim3(n_items, 16), 256, 0, s>>>(insts, items, cpb, ia);
+    k_batch_energies<<<dim3(n_items, (cpb + 31) / 32), 32 * kEnergyRows, 0, s>>>(insts, items, cpb);
     return cudaGetLastError();
 }
 

@@ -537,29 +537,34 @@ __device__ __forceinline__ unsigned long long cluster_load(const void *p, uint32
     return v;
 }
 
-__global__ void __launch_bounds__(kClusterThreads) k_upd_cluster(unsigned long long *__restrict__ hist, uint32_t N,
-                                                                 double *__restrict__ lnw, float *__restrict__ w32,
-                                                                 int rule, HistStatsDev *__restrict__ stats,
-                                                                 RunCtl *__restrict__ ctl)
+// The update by this block's cluster (kClusterBlocks successive blocks), PER
+// bins per thread at most.  CLEAR: in a device-driven run, zero the histogram
+// for the next iteration unless this was the last.  Returns whether this
+// thread (one of the cluster) has seen the run go on.
+template <int PER, bool CLEAR>
+__device__ __forceinline__ bool cluster_update(unsigned long long *__restrict__ hist, uint32_t N,
+                                               double *__restrict__ lnw, float *__restrict__ w32, int rule,
+                                               HistStatsDev *__restrict__ stats, RunCtl *__restrict__ ctl)
 {
+    const uint32_t rank = blockIdx.x % kClusterBlocks;
     __shared__ HistSum shs[32];
     __shared__ double shd[32];
     __shared__ unsigned long long s_part[4], s_kl, s_do;
     __shared__ RunCtl s_ctl;
     // (read by every block before the first barrier, written after the second)
-    if (ctl && ctl->st.stop) return;
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, i0 = blockIdx.x * kClusterThreads + tid;
+    if (ctl && ctl->st.stop) return false;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, i0 = rank * kClusterThreads + tid;
     constexpr uint32_t st = kClusterBlocks * kClusterThreads;
     // the run state, near for the one thread that keeps the books
-    if (ctl && blockIdx.x == 0 && tid < sizeof(RunCtl) / 4)
+    if (ctl && rank == 0 && tid < sizeof(RunCtl) / 4)
         reinterpret_cast<uint32_t *>(&s_ctl)[tid] = reinterpret_cast<const uint32_t *>(ctl)[tid];
     const unsigned long long h0 = hist[0], thr = rule == 0 ? 1ull : 0ull;
     const double lnw0 = lnw[0];
-    unsigned long long h[kClusterPer];
-    double x[kClusterPer];
+    unsigned long long h[PER];
+    double x[PER];
     HistSum v{(int)N + 1, -1, 0ull, 0ull, ~0ull};
 #pragma unroll
-    for (int k = 0; k < kClusterPer; ++k) {
+    for (int k = 0; k < PER; ++k) {
         const uint32_t i = i0 + k * st;
         h[k] = 0ull;
         x[k] = 0.0;
@@ -590,7 +595,7 @@ __global__ void __launch_bounds__(kClusterThreads) k_upd_cluster(unsigned long l
     const double num_event = (double)v.ev, Q = __ddiv_rn(1.0, (double)v.vis);
     double kl = 0.0;
 #pragma unroll
-    for (int k = 0; k < kClusterPer; ++k) {
+    for (int k = 0; k < PER; ++k) {
         if (h[k] > 0) {
             const double P = __ddiv_rn((double)h[k], num_event);
             kl = __dadd_rn(kl, __dmul_rn(P, log(__ddiv_rn(P, Q))));
@@ -599,7 +604,7 @@ __global__ void __launch_bounds__(kClusterThreads) k_upd_cluster(unsigned long l
     kl = block_reduce(kl, AddD(), shd);
     if (tid == 0) s_kl = (unsigned long long)__double_as_longlong(kl);
     cluster_sync();
-    if (blockIdx.x == 0 && tid < 32) {
+    if (rank == 0 && tid < 32) {
         // the blocks' sums joined as a tree
         double klt = lane < kClusterBlocks ? __longlong_as_double((long long)cluster_load(&s_kl, lane)) : 0.0;
 #pragma unroll
@@ -617,7 +622,7 @@ __global__ void __launch_bounds__(kClusterThreads) k_upd_cluster(unsigned long l
     if (rule >= 0) {
         const double tmp = h0 > thr ? __dsub_rn(lnw0, log((double)h0)) : lnw0;
 #pragma unroll
-        for (int k = 0; k < kClusterPer; ++k) {
+        for (int k = 0; k < PER; ++k) {
             if (h[k] > thr) x[k] = __dsub_rn(x[k], log((double)h[k]));
             if (rule == 0 || h[k] > 0) x[k] = __dsub_rn(x[k], tmp);
         }
@@ -625,34 +630,64 @@ __global__ void __launch_bounds__(kClusterThreads) k_upd_cluster(unsigned long l
     cluster_sync();
     const uint32_t todo = (uint32_t)cluster_load(&s_do, 0);
 #pragma unroll
-    for (int k = 0; k < kClusterPer; ++k) {
+    for (int k = 0; k < PER; ++k) {
         const uint32_t i = i0 + k * st;
         if (i <= N) {
             if (todo & 1u) {
                 lnw[i] = x[k];
                 w32[i] = (float)x[k];
             }
-            if (todo & 2u) hist[i] = 0ull;
+            if (CLEAR && (todo & 2u)) hist[i] = 0ull;
         }
     }
     cluster_sync();  // no block leaves while another may read its shared memory
+    return rank == 0 && tid == 0 && (todo & 2u);
 }
+__global__ void __launch_bounds__(kClusterThreads) k_upd_cluster(unsigned long long *__restrict__ hist, uint32_t N,
+                                                                 double *__restrict__ lnw, float *__restrict__ w32,
+                                                                 int rule, HistStatsDev *__restrict__ stats,
+                                                                 RunCtl *__restrict__ ctl)
+{
+    cluster_update<kClusterPer, true>(hist, N, lnw, w32, rule, stats, ctl);
+}
+
+// One iteration's tail for every instance of a batch without the recursion
+// (a cluster per instance, up to 16385 bins), and the count of the instances
+// still running.  The FP64 work spreads over the whole chip; a block per
+// instance left the largest one's 16385 bins to one SM (378 us at L = 128).
+constexpr int kBatchPer = 5;
+static_assert(kClusterBlocks * kClusterThreads * kBatchPer >= 16385, "bins of the largest instance");
+__global__ void __launch_bounds__(kClusterThreads) k_batch_update(const BatchInst *__restrict__ insts,
+                                                                  uint32_t *__restrict__ running)
+{
+    const BatchInst &I = insts[blockIdx.x / kClusterBlocks];
+    if (cluster_update<kBatchPer, false>(I.a.hist, I.a.N, I.lnw, I.w32, (int)I.rule, nullptr, I.ctl))
+        atomicAdd(running, 1u);
+}
+
+static cudaLaunchConfig_t cluster_config(cudaLaunchAttribute *at, uint32_t updates, cudaStream_t s)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(kClusterBlocks * updates);
+    cfg.blockDim = dim3(kClusterThreads);
+    cfg.stream = s;
+    *at = cudaLaunchAttribute{};
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = kClusterBlocks;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
 
 static cudaError_t launch_update_cluster(unsigned long long *hist, uint32_t N, double *lnw, float *w32, int rule,
                                          HistStatsDev *stats, RunCtl *ctl, cudaStream_t s)
 {
     const cudaError_t e = cudaFuncSetAttribute(k_upd_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(kClusterBlocks);
-    cfg.blockDim = dim3(kClusterThreads);
-    cfg.stream = s;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = kClusterBlocks;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg = cluster_config(&at, 1, s);
     return cudaLaunchKernelEx(&cfg, k_upd_cluster, hist, N, lnw, w32, rule, stats, ctl);
 }
 
@@ -704,10 +739,9 @@ static cudaError_t launch_update_multi(unsigned long long *hist, uint32_t N, dou
     return cudaGetLastError();
 }
 
-// One iteration's tail for every instance of a batch (block i = instance i),
-// then the count of instances that are still running.
-__global__ void __launch_bounds__(kUpdThreads) k_batch_update(const BatchInst *__restrict__ insts,
-                                                               uint32_t *__restrict__ running)
+// The tail of a batch's iteration with the recursion: block i = instance i.
+__global__ void __launch_bounds__(kUpdThreads) k_batch_update_rec(const BatchInst *__restrict__ insts,
+                                                                   uint32_t *__restrict__ running)
 {
     extern __shared__ __align__(16) unsigned char dyn[];
     const BatchInst &I = insts[blockIdx.x];
@@ -764,21 +798,26 @@ cudaError_t launch_run_update(unsigned long long *hist, double *lnw, float *w32,
     return cudaGetLastError();
 }
 
-cudaError_t prepare_batch_update(uint32_t max_N, int any_recursion)
+cudaError_t prepare_batch_update(uint32_t max_N)
 {
+    const cudaError_t e = cudaFuncSetAttribute(k_batch_update, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     // the limit of the largest size, whatever this batch's: another batch of the
     // process shares the kernel
-    if (any_recursion && update_smem(max_N, 2) > 48 * 1024)
-        return cudaFuncSetAttribute(k_batch_update, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (e == cudaSuccess && update_smem(max_N, 2) > 48 * 1024)
+        return cudaFuncSetAttribute(k_batch_update_rec, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)update_smem(16384, 2));
-    return cudaSuccess;
+    return e;
 }
 
-cudaError_t launch_batch_update(const BatchInst *insts, uint32_t n_inst, uint32_t max_N, int any_recursion,
+cudaError_t launch_batch_update(const BatchInst *insts, uint32_t n_inst, uint32_t max_N, int recursion,
                                 uint32_t *running, cudaStream_t s)
 {
-    const size_t dyn = any_recursion ? update_smem(max_N, 2) : 0;
-    k_batch_update<<<n_inst, kUpdThreads, dyn, s>>>(insts, running);
+    if (!recursion) {
+        cudaLaunchAttribute at;
+        const cudaLaunchConfig_t cfg = cluster_config(&at, n_inst, s);
+        return cudaLaunchKernelEx(&cfg, k_batch_update, insts, running);
+    }
+    k_batch_update_rec<<<n_inst, kUpdThreads, update_smem(max_N, 2), s>>>(insts, running);
     return cudaGetLastError();
 }
 

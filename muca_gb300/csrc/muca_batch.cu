@@ -198,6 +198,7 @@ muca_status set_layout(muca_batch *b, uint32_t cpb, uint32_t rule)
         t.w32 = b->d_w32 + b->off_w[i];
         for (int d = -8; d <= 8; ++d) t.btab[d + 8] = (float)(-b->inst[i].beta * (double)d);
         t.rule = rule;
+        t.seed = b->inst[i].seed;
     }
     BCUDA(b, cudaMemcpyAsync(b->d_inst, ti.data(), ti.size() * sizeof(BatchInst), cudaMemcpyHostToDevice, b->stream));
     BCUDA(b, cudaStreamSynchronize(b->stream));  // `items`/`ti` are pageable locals
@@ -252,21 +253,13 @@ muca_status apply_shape(muca_batch *b, const muca_batch_shape &s, uint32_t rule)
 // Philox words through graded_spin (MUCA_INIT_GRADED).
 muca_status init_chains(muca_batch *b, bool graded = false)
 {
-    for (uint32_t i = 0; i < b->n; ++i) {
-        const muca_instance &m = b->inst[i];
-        InitArgs ia{};
-        ia.rounds = 7;
-        ia.key0_mul = 10; ia.key0_jack_mul = 2; ia.key1 = 0xdecafbadu;
-        ia.ctr0[0] = 2u * m.seed; ia.ctr0[1] = 100; ia.ctr0[2] = 0xBADCAB1Eu; ia.ctr0[3] = 0xBADC0DEDu;
-        ia.ctr0_dev_mul[0] = 2; ia.ctr_word = 0;
-        ia.chain_offset = m.seed * m.nchains;
-        ia.graded = graded ? 1u : 0u;
-        const uint32_t cpb = b->shape.chains_per_block;
-        uint32_t *lat = b->d_lat + b->off_lat[i];
-        BCUDA(b, launch_init(lat, m.L, wpr_of(m.L), cpb, m.nchains, m.nchains, 0, ia, b->stream));
-        BCUDA(b, launch_energies(lat, b->d_ej + b->off_chain[i], b->d_edel + b->off_chain[i],
-                                 b->d_mag + b->off_chain[i], m.L, wpr_of(m.L), cpb, m.nchains, b->stream));
-    }
+    InitArgs ia{};
+    ia.rounds = 7;
+    ia.key0_mul = 10; ia.key0_jack_mul = 2; ia.key1 = 0xdecafbadu;
+    ia.ctr0[1] = 100; ia.ctr0[2] = 0xBADCAB1Eu; ia.ctr0[3] = 0xBADC0DEDu;
+    ia.ctr0_dev_mul[0] = 2; ia.ctr_word = 0;
+    ia.graded = graded ? 1u : 0u;
+    BCUDA(b, launch_batch_init(b->d_inst, b->d_items, b->n_items, b->shape.chains_per_block, ia, b->stream));
     return MUCA_OK;
 }
 
@@ -479,7 +472,7 @@ muca_status muca_batch_create(const muca_batch_params *p, const muca_instance *i
     BTRY(cudaMemsetAsync(b->d_recs, 0, n * sizeof(IterRecordDev), b->stream));
     BTRY(cudaMemsetAsync(b->d_err, 0, sizeof(unsigned int), b->stream));
     BTRY(device_log_eps(b->device, b->stream, &b->log_eps));
-    BTRY(prepare_batch_update(b->max_N, 1));
+    BTRY(prepare_batch_update(b->max_N));
     muca_status st;
     if (p->shape_chains_per_block) {
         muca_batch_shape s{};

@@ -207,12 +207,16 @@ struct BatchInst {
     double *lnw, *p_acc;
     float *w32;
     float btab[17];
-    uint32_t rule;
+    uint32_t rule, seed;
 };
 // A unit of sweep work: chain block `blk` of instance `inst`.
 struct BatchItem {
     uint32_t inst, blk;
 };
+// Initial lattices of every instance (ia: those of emulated device 0; the
+// instance's seed is its device index) and their energies.
+cudaError_t launch_batch_init(const BatchInst *insts, const BatchItem *items, uint32_t n_items, uint32_t cpb,
+                              const InitArgs &ia, cudaStream_t s);
 // Clears the histograms of the running instances and resets the work counter.
 cudaError_t launch_batch_prep(const BatchInst *insts, uint32_t n_inst, uint32_t *next_item, uint32_t *running,
                               cudaStream_t s);
@@ -235,10 +239,10 @@ size_t batch_sweep_smem(uint32_t L, uint32_t cpb, bool lat_smem, bool hist_smem,
 // The launch with that shape needs no further attribute call.
 cudaError_t batch_sweep_occupancy(uint32_t cpb, int rounds, uint32_t lat, bool hist_smem, size_t smem,
                                   size_t smem_limit, int *blocks);
-// Sets the update kernel's shared-memory limit (call before any capture).
-cudaError_t prepare_batch_update(uint32_t max_N, int any_recursion);
+// Sets the update kernels' shared-memory and cluster limits (call before any capture).
+cudaError_t prepare_batch_update(uint32_t max_N);
 // The update step of every instance; *running += instances not stopped.
-cudaError_t launch_batch_update(const BatchInst *insts, uint32_t n_inst, uint32_t max_N, int any_recursion,
+cudaError_t launch_batch_update(const BatchInst *insts, uint32_t n_inst, uint32_t max_N, int recursion,
                                 uint32_t *running, cudaStream_t s);
 
 // One iteration's tail: statistics, width/convergence bookkeeping, weight

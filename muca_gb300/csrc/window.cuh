@@ -713,10 +713,15 @@ __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned cha
             off = ah.off;
             for (ah.off += len; ah.off >= 4u; ah.off -= 4u) shift_in(dr, ++cc, ah);
         }
-        if (MASKED)
+        if (MASKED) {
+            // slots past the last attempt: never accepted, and no move to look ahead for
 #pragma unroll
             for (int t = 0; t < S; ++t)
                 if ((uint32_t)t >= len) w.l[t] = INFINITY;
+            const uint32_t keep = (1u << (4u * len)) - 1u;  // len < 8
+            w.code[0] = (w.code[0] & keep) | (0x22222222u & ~keep);
+            w.code[1] = w.code[0] >> 16;
+        }
         auto redraw = [&](uint32_t(&r1)[S]) {
             if (ALIGNED) {
                 dr.s1.block((unsigned long long)kPhiloxM0 * c0, r1);
