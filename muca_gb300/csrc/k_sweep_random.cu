@@ -15,35 +15,60 @@
 //         host libm's logf (the CPU program) when a table of its values is
 //         given, else CUDA's logf (mcs2).
 // The lattice uses the packed layout of the other sweeps (2-bit codes, rows
-// of 16-site words, [block][word][lane]); the FP32 difference table of the
-// FP64 weights (stage_diff_table) and a u32 histogram are staged in shared
-// memory, the lattice too when it fits.
+// of 16-site words, [block][word][lane]); the FP32 differences of the FP64
+// weights (stage_differences) and a u32 histogram are staged in shared memory,
+// the lattice too when it fits.
 //
-// FP64 issues slowly on this GPU, and the exact log is a table lookup in
-// global memory (host libm values) or a full logf: both used to sit on every
-// attempt's dependency chain.  The test is decided in FP32 instead, as the
-// production scan does it: log(u) < 0 for every u <= 1 - 2^-24, so the
-// reference's test is  log(u) < diff;  with fast = -2 dE + T[E].(dDel)
-// within tol of the FP64 diff and __logf(u) within `log_eps` of the exact
-// log (measured over every u: against CUDA's logf, or against the host
-// table), g = __logf(u) - fast has the sign of log(u) - diff whenever
-// |g| > tol + log_eps.  Otherwise that lane forms the reference's FP64 diff
-// from the global weights and the exact log, so every decision is the
-// reference's.
-#include "sweep_core.cuh"
+// The test is decided in FP32, as the production window does it, and where
+// that is in doubt by the reference's FP64 difference and the exact log (host
+// libm value or logf): see scan_produce for the bound.
+//
+// What bounds it: at one warp per SM sub-partition the instructions of the
+// warp, and beneath them the chain from one attempt's store to the next one's
+// loads and decision.  So what does not depend on the spins (the draws, the
+// sites, the addresses of their neighbours) is formed one group of four
+// attempts ahead, in the same stretch of code as the scan of the group before,
+// and the scan has no branch: an attempt in doubt is noticed at the end of its
+// group, whose stores are then taken back and repeated.
+//   * a site is split into row and column with FP32 (exact: idx < 2^14); a
+//     number in the mantissa of 2^23 goes into the address products as it is,
+//     the constant they carry is in the address base;
+//   * a word is rotated until its site is at the bottom, and code and
+//     direction are the selector of a byte table whose entries 3 and 7 complete
+//     the float 2^23 + entry;
+//   * lattice columns in shared memory lie a multiple of 32 lanes apart where
+//     that fits, so that lanes at different sites meet no bank conflict.
+// L = 72, 16384 chains, 85 M attempts: @@ us, 1815 us with draws, site and
+// test of every attempt on one dependency chain.
+#include "window.cuh"
 
 #include <algorithm>
 
 namespace muca {
 
-// shared memory: the difference table (float2 per bin) | u32 histogram | lattice
+// shared memory: 16 B (read for E = 0, never used) | differences | u32 histogram | lattice
 __host__ __device__ inline size_t random_smem_base(uint32_t N)
 {
-    return align16((size_t)(N + 1) * 8) + align16((size_t)(N + 1) * 4);
+    return 16 + 2 * align16((size_t)(N + 1) * 4);
 }
 
+// The drawn side of an attempt: the acceptance logarithm, the byte offsets of
+// the site's word and its neighbours', twice their sites (rotations count
+// modulo 32), and the selector of the byte tables less the site's code.
+struct RandomAttempt {
+    float l;
+    uint32_t aC, aU, aD, aL, aR, sC, sL, sR, dsel;
+};
+// Byte tables by code | direction << 2 (window.cuh), entry 3 = 0; entry 7 =
+// 0x4B where the value is to be the float 2^23 + entry, else 0.
+constexpr uint32_t kRndDV_0 = 0x00000303u, kRndDV_1 = 0x4B010104u;  // s_new - s_old + 2
+constexpr uint32_t kRndND_0 = 0x00010002u, kRndND_1 = 0x4B020001u;  // 1 - dDel
+constexpr uint32_t kRndD4_0 = 0x00040800u, kRndD4_1 = 0x00000804u;  // 4 dDel + 4
+constexpr uint32_t kRndVX_0 = 0x00020301u, kRndVX_1 = 0x00030102u;  // old code ^ new code
+constexpr uint32_t kRndSel = 0x7330u;
+
 template <int R, bool LAT_SMEM>
-__global__ void __launch_bounds__(256) k_sweep_random(const RandomArgs a, uint32_t cpb)
+__global__ void __launch_bounds__(256) k_sweep_random(const RandomArgs a, uint32_t cpb, uint32_t pitch)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     uint32_t iter = a.iter;
@@ -54,114 +79,210 @@ __global__ void __launch_bounds__(256) k_sweep_random(const RandomArgs a, uint32
         nup = a.dyn[1];
     }
     const uint32_t N = a.N, L = a.L, WPR = a.WPR, nt = blockDim.x, tid = threadIdx.x, lane = threadIdx.x;
-    float2 *T = reinterpret_cast<float2 *>(smem);
-    uint32_t *histS = reinterpret_cast<uint32_t *>(smem + align16((size_t)(N + 1) * 8));
-    uint32_t *latS = reinterpret_cast<uint32_t *>(smem + random_smem_base(N));
+    float *u = reinterpret_cast<float *>(smem + 16);
+    uint32_t *histS = reinterpret_cast<uint32_t *>(smem + 16 + align16((size_t)(N + 1) * 4));
+    const uint32_t lat_off = (uint32_t)random_smem_base(N);
     const double *__restrict__ w64 = a.w;
-    const float band = stage_diff_table(w64, N, T) + (float)a.log_eps;
-    for (uint32_t i = tid; i <= N; i += nt) histS[i] = 0u;
     const uint32_t words = L * WPR;
-    const bool store = lane < cpb;
-    const uint32_t l = store ? lane : 0u;
-    uint32_t *gl = a.lat + (size_t)blockIdx.x * words * cpb + l;
-    uint32_t *lat = gl;
+    const bool store = lane < cpb;  // owns its lattice column
+    uint32_t *gl = a.lat + (size_t)blockIdx.x * words * cpb + (store ? lane : 0u);
+    // the lane's column: its own; without one a padding column, or else lane 0's, which it only reads
+    const uint32_t column = LAT_SMEM ? (lane < pitch ? lane : 0u) : (store ? lane : 0u);
     if (LAT_SMEM) {
-        if (store)
-            for (uint32_t w = 0; w < words; ++w) latS[(size_t)w * cpb + lane] = gl[(size_t)w * cpb];
-        lat = latS + l;
+        uint32_t *latS = reinterpret_cast<uint32_t *>(smem + lat_off) + column;
+        if (store) {
+            uint32_t d = (uint32_t)__cvta_generic_to_shared(latS);
+            for (uint32_t w = 0; w < words; ++w, d += 4u * pitch)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(gl + (size_t)w * cpb) : "memory");
+        } else if (lane < pitch) {
+            for (uint32_t w = 0; w < words; ++w) latS[(size_t)w * pitch] = kZeroWord;
+        }
     }
+    const float band = stage_differences(w64, N, u) + (float)a.log_eps;
+    if (tid == 0) u[-1] = 0.0f;
+    for (uint32_t i = tid; i <= N; i += nt) histS[i] = 0u;
+    if (LAT_SMEM) asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     const uint32_t chain = blockIdx.x * cpb + lane;
     const bool active = store && chain < a.nchains;
     const uint32_t W = a.worker0 + chain;
-    RoundKeys<R> k1, k2, k3;
-    k1.init(10u * W + 1000u * a.seed, 0xdecafbadu);
-    k2.init(100u * W + 4000u * a.seed, 0x20202041u);
-    k3.init(1000u * W + 10000u * a.seed, 0x11cafeadu);
-    // lanes without a chain (padding lanes, which read lane 0's spins, and the
-    // last block's lanes past the chain count) never accept, so their E_Delta
-    // stays 1 and every weight index E + dDel stays in [0, 2]
-    int E = active ? a.edel[chain] : 1;
-    int EJ = active ? a.ej[chain] : 0;
-    const float fN = (float)N;
-    uint32_t c0 = 0;
-    uint4 r1 = make_uint4(0, 0, 0, 0), r2 = r1, r3 = r1;
-    auto code_at = [&](uint32_t row, uint32_t col) -> uint32_t {
-        return spin_code(lat[(size_t)(row * WPR + (col >> 4)) * cpb], col);
+    Stream<R> s1, s2, s3;
+    s1.init(10u * W + 1000u * a.seed, 0xdecafbadu, 0xbadbad11u, 2u * iter);
+    s2.init(100u * W + 4000u * a.seed, 0x20202041u, 0xbadbad11u, 2u * iter);
+    s3.init(1000u * W + 10000u * a.seed, 0x11cafeadu, 0xbadbad11u, 2u * iter);
+    // lanes without a chain: an infinite logarithm (or a NaN), so they never
+    // accept, E_Delta stays 1, and they count in the bin after the last, which
+    // the rounded-up size of the histogram has (N + 1 is no multiple of 4)
+    const float ln2 = active ? kLn2 : -INFINITY;
+    uint32_t e4 = active ? 4u * (uint32_t)a.edel[chain] : 4u;
+    float ej2 = active ? (float)(2 * a.ej[chain]) : 0.0f;
+    unsigned char *hist_lane = reinterpret_cast<unsigned char *>(histS) + (active ? 0u : 4u * N);
+
+    unsigned char *const base = LAT_SMEM ? smem : reinterpret_cast<unsigned char *>(a.lat + (size_t)blockIdx.x * words * cpb);
+    const uint32_t p4 = 4u * (LAT_SMEM ? pitch : cpb), rs = WPR * p4;  // bytes from a word (row) to the next
+    // word q of row r lies at bits(2^23 + r) rs + (bits(2^23 + col) >> 4) p4 + k0
+    const uint32_t k0 = (LAT_SMEM ? lat_off : 0u) + 4u * column - 0x4B000000u * rs - 0x04B00000u * p4;
+    const float fN = (float)N, fL = (float)L, inv = __frcp_rn(fL), half_inv = 0.5f * inv, magic = 8388608.0f;
+    const float row_last = magic + (fL - 1.0f);
+    const uint32_t col_last = 0x4B000000u + L - 1u, wrap = (L - 1u) * rs;
+
+    auto word = [&](uint32_t off) -> uint32_t & { return *reinterpret_cast<uint32_t *>(base + off); };
+    auto prep = [&](uint32_t c, RandomAttempt (&at)[4]) {
+        uint32_t r1[4], r2[4], r3[4];
+        const unsigned long long q = (unsigned long long)kPhiloxM0 * c;
+        s1.block(q, r1);
+        s2.block(q, r2);
+        s3.block(q, r3);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            RandomAttempt &x = at[t];
+            x.l = __fmul_rn(lg2_ftz(u01s(r1[t])), ln2);
+            // 2^23 + idx, idx = (unsigned)(u N); row = floor((idx + 1/2) / L)
+            const float ib = __fadd_rz(__fmul_rn(u01s(r2[t]), fN), magic);
+            const float rowb = __fadd_rz(__fmaf_rn(__fsub_rn(ib, magic), inv, half_inv), magic);
+            const float colb = __fmaf_rn(__fsub_rn(rowb, magic), -fL, ib);
+            const uint32_t col = __float_as_uint(colb), row = __float_as_uint(rowb) * rs + k0;
+            const uint32_t cl = colb == magic ? col_last : col - 1u, cr = col == col_last ? 0x4B000000u : col + 1u;
+            x.aC = (col >> 4) * p4 + row;
+            x.aU = x.aC + (rowb == row_last ? 0u - wrap : rs);
+            x.aD = x.aC + (rowb == magic ? wrap : 0u - rs);
+            x.aL = (cl >> 4) * p4 + row;
+            x.aR = (cr >> 4) * p4 + row;
+            x.sC = 2u * col;
+            x.sL = 2u * cl;
+            x.sR = 2u * cr;
+            x.dsel = ((r3[t] >> 29) & 4u) | kRndSel;  // u01fixedpt<float>(r3) < 0.5 <=> top bit clear: s + 1
+        }
     };
-    for (int phase = 0; phase < 2; ++phase) {
-        const unsigned long long n = phase ? nup : a.therm;
-        for (unsigned long long i = 0; i < n; ++i) {
-            const int sub = (int)(i & 3ull);
-            if (sub == 0) {
-                ++c0;
-                r1 = philox<R>(c0, 0xbadbad11u, 2u * iter, kCtrTag, k1);
-                r2 = philox<R>(c0, 0xbadbad11u, 2u * iter, kCtrTag, k2);
-                r3 = philox<R>(c0, 0xbadbad11u, 2u * iter, kCtrTag, k3);
+    // code of the site that the rotation brings to the bottom
+    auto code = [](uint32_t w, uint32_t s2x) -> uint32_t { return __funnelshift_r(w, w, s2x) & 3u; };
+    struct Move {
+        uint32_t word, sel;
+        float dv, ns2;
+    };
+    auto decode = [&](const RandomAttempt &x) -> Move {
+        Move m;
+        m.word = word(x.aC);
+        m.sel = code(m.word, x.sC) | x.dsel;
+        const uint32_t nb = code(word(x.aU), x.sC) + code(word(x.aD), x.sC) + code(word(x.aL), x.sL) +
+                            code(word(x.aR), x.sR);
+        m.ns2 = __fmaf_rn(__uint_as_float(0x4B000000u + nb), 2.0f, -16777224.0f);
+        m.dv = __fsub_rn(__uint_as_float(prmt_var(kRndDV_0, kRndDV_1, m.sel)), 8388610.0f);
+        return m;
+    };
+    auto moved = [&](const RandomAttempt &x, const Move &m) -> uint32_t {
+        return __funnelshift_l(0u, prmt_var(kRndVX_0, kRndVX_1, m.sel), x.sC);
+    };
+    const unsigned char *uS = smem + 16;
+    auto U = [&](uint32_t e) -> float { return *reinterpret_cast<const float *>(uS + e); };
+
+    uint32_t c0 = 1;
+    RandomAttempt nx[4];
+    prep(c0, nx);
+    uint32_t unflushed = 0;
+    auto run = [&](unsigned long long n, auto rec) {
+        constexpr bool REC = decltype(rec)::value;
+        while (n > 0) {
+            const uint32_t len = n < 4ull ? (uint32_t)n : 4u;
+            n -= len;
+            RandomAttempt at[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) at[t] = nx[t];
+            if (len < 4u) {
+#pragma unroll
+                for (int t = 1; t < 4; ++t)
+                    if ((uint32_t)t >= len) at[t].l = INFINITY;  // never accepted
             }
-            const uint32_t idx = __float2uint_rz(__fmul_rn(u01f(pick(r2, sub)), fN));
-            // idx / L as a high product with ceil(2^32 / L): exact for idx < 2^16
-            // and L <= 128 (the rounding error idx / 2^32 < 1/L)
-            const uint32_t row = __umulhi(idx, a.inv_L), col = idx - row * L;
-            uint32_t *pw = lat + (size_t)(row * WPR + (col >> 4)) * cpb;
-            const int os = (int)spin_code(*pw, col) - 1;
-            int ns = os + ((pick(r3, sub) >> 31) ? -1 : 1);  // u01fixedpt<float>(r3) < 0.5 <=> top bit clear
-            ns = ns - 3 * (ns == 2) + 3 * (ns == -2);
-            const uint32_t cl = col ? col - 1 : L - 1, cr = (col + 1 == L) ? 0u : col + 1;
-            const uint32_t ru = (row + 1 == L) ? 0u : row + 1, rd = row ? row - 1 : L - 1;
-            const int nb = (int)(code_at(row, cl) + code_at(row, cr) + code_at(ru, col) + code_at(rd, col)) - 4;
-            const int tmp = ns * (os == 0) + os;  // the trial value the reference stores before forming dE
-            const int dE = ((os == 0) + os * (ns - os)) * (-tmp) * nb;
-            const int dDel = ns * ns - os * os;
-            const uint32_t r = pick(r1, sub);
-            const float2 tE = T[E];
-            const float dl = dDel == 0 ? 0.0f : (dDel < 0 ? tE.x : tE.y);
-            const float g = __fsub_rn(fast_logf(u01f(r)), __fadd_rn(small_int_to_float(-2 * dE), dl));
-            bool acc = g < 0.0f;
-            if (fabsf(g) <= band) {
-                // in doubt: the reference's FP64 difference and exact log
-                const double diff = __dsub_rn(__dadd_rn((double)(-dE * 2), w64[E + dDel]), w64[E]);
-                acc = diff >= 0.0;
-                if (!acc) {
-                    const float lg = a.logf_tab ? __ldg(a.logf_tab + (r >> 9)) : logf(u01f(r));
-                    acc = (double)lg < diff;
+            prep(c0 + 1u, nx);
+            const uint32_t e4_0 = e4;
+            const float ej2_0 = ej2;
+            uint32_t old[4], Es[4];
+            bool near = false;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const RandomAttempt &x = at[t];
+                const float um = U(e4 - 4u), up = U(e4);
+                const Move m = decode(x);
+                const float nd = __fsub_rn(__uint_as_float(prmt_var(kRndND_0, kRndND_1, m.sel)), 8388609.0f);
+                // logf(u) - f2 - (w[E + dDel] - w[E]), f2 = -2 dE = dv ns2
+                const float g = __fmaf_rn(nd, nd > 0.0f ? um : up, __fmaf_rn(-m.dv, m.ns2, x.l));
+                const bool acc = g < 0.0f;
+                near |= !(fabsf(g) > band);  // a NaN (differences beyond FP32) is in doubt too
+                old[t] = m.word;
+                const uint32_t next = e4 + prmt_var(kRndD4_0, kRndD4_1, m.sel) - 4u;
+                const uint32_t changed = m.word ^ (acc ? moved(x, m) : 0u);
+                if (store) word(x.aC) = changed;
+                if (acc) ej2 = __fmaf_rn(-m.dv, m.ns2, ej2);
+                e4 = acc ? next : e4;
+                Es[t] = e4;
+            }
+            if (near) {
+                // in doubt: the group again, with the reference's FP64
+                // difference and exact log
+                uint32_t r1[4];
+                s1.block((unsigned long long)kPhiloxM0 * c0, r1);
+                e4 = e4_0;
+                ej2 = ej2_0;
+                if (store) {
+#pragma unroll
+                    for (int t = 3; t >= 0; --t) word(at[t].aC) = old[t];
+                }
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    const Move m = decode(at[t]);
+                    const int E = (int)(e4 >> 2), d4 = (int)prmt_var(kRndD4_0, kRndD4_1, m.sel) - 4;
+                    if (active && (uint32_t)t < len) {
+                        const double diff = __dsub_rn(__dadd_rn((double)__fmul_rn(m.dv, m.ns2), w64[E + d4 / 4]), w64[E]);
+                        bool acc = diff >= 0.0;
+                        if (!acc) {
+                            const float lg = a.logf_tab ? __ldg(a.logf_tab + (r1[t] >> 9)) : logf(u01s(r1[t]));
+                            acc = (double)lg < diff;
+                        }
+                        if (acc) {
+                            word(at[t].aC) = m.word ^ moved(at[t], m);
+                            ej2 = __fmaf_rn(-m.dv, m.ns2, ej2);
+                            e4 += (uint32_t)d4;
+                        }
+                    }
+                    Es[t] = e4;
                 }
             }
-            if (acc && active) {
-                const uint32_t sh = 2u * (col & 15u);
-                *pw = (*pw & ~(3u << sh)) | ((uint32_t)(ns + 1) << sh);
-                EJ += dE;
-                E += dDel;
-            }
-            if (phase == 1 && active) {
-                // a u32 shared bin is drained into the u64 device bin at 2^31
-                const uint32_t old = atomicAdd(&histS[E], 1u);
-                if (old >= 0x80000000u) atomicAdd(&a.hist[E], (unsigned long long)atomicExch(&histS[E], 0u));
+            ++c0;
+            if (REC) {
+#pragma unroll
+                for (int t = 0; t < 4; ++t)
+                    if (t == 0 || (uint32_t)t < len) atomicAdd(reinterpret_cast<uint32_t *>(hist_lane + Es[t]), 1u);
+                // no more than 256 lanes x 4 x 2^20 = 2^30 entries between two flushes
+                if (++unflushed == (1u << 20)) {
+                    flush_hist<kModeWeight>(histS, a.hist, N);
+                    unflushed = 0;
+                }
             }
         }
-    }
+    };
+    run(a.therm, std::false_type{});
+    run(nup, std::true_type{});
     if (LAT_SMEM && store) {
-        for (uint32_t w = 0; w < words; ++w) gl[(size_t)w * cpb] = lat[(size_t)w * cpb];
+        const uint32_t *lat = reinterpret_cast<const uint32_t *>(smem + lat_off) + column;
+#pragma unroll 8
+        for (uint32_t w = 0; w < words; ++w) gl[(size_t)w * cpb] = lat[(size_t)w * pitch];
     }
     if (active) {
-        a.edel[chain] = E;
-        a.ej[chain] = EJ;
+        a.edel[chain] = (int32_t)(e4 >> 2);
+        a.ej[chain] = (int32_t)ej2 / 2;
     }
     __syncthreads();
-    for (uint32_t b = tid; b <= N; b += nt) {
-        const uint32_t v = histS[b];
-        if (v) atomicAdd(&a.hist[b], (unsigned long long)v);
-    }
+    drain_hist<kModeWeight>(histS, a.hist, N);
 }
 
 template <int R, bool LS>
-static cudaError_t launch_random_one(const RandomArgs &a, uint32_t cpb, uint32_t blocks, size_t smem, size_t smem_limit,
-                                     cudaStream_t s)
+static cudaError_t launch_random_one(const RandomArgs &a, uint32_t cpb, uint32_t pitch, uint32_t blocks, size_t smem,
+                                     size_t smem_limit, cudaStream_t s)
 {
     const cudaError_t e = cudaFuncSetAttribute(k_sweep_random<R, LS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)smem_limit);
     if (e != cudaSuccess) return e;
-    k_sweep_random<R, LS><<<blocks, (cpb + 31u) / 32u * 32u, smem, s>>>(a, cpb);
+    k_sweep_random<R, LS><<<blocks, (cpb + 31u) / 32u * 32u, smem, s>>>(a, cpb, pitch);
     return cudaGetLastError();
 }
 
@@ -191,10 +312,10 @@ SweepPlan plan_random(uint32_t L, uint32_t nchains, size_t smem_optin, int sms)
     return p;
 }
 
-size_t random_sweep_smem(uint32_t L, uint32_t cpb, bool lat_smem)
+size_t random_sweep_smem(uint32_t L, uint32_t pitch, bool lat_smem)
 {
     const uint32_t WPR = (L + 15) / 16;
-    return random_smem_base(L * L) + (lat_smem ? (size_t)L * WPR * 4 * cpb : 0);
+    return random_smem_base(L * L) + (lat_smem ? (size_t)L * WPR * 4 * pitch : 0);
 }
 
 cudaError_t launch_sweep_random(const RandomArgs &a, uint32_t cpb, uint32_t blocks, int rounds, size_t smem_optin,
@@ -202,13 +323,15 @@ cudaError_t launch_sweep_random(const RandomArgs &a, uint32_t cpb, uint32_t bloc
 {
     if (cpb == 0 || cpb > 256 || a.L < 3) return cudaErrorInvalidValue;
     // (512 B of the opt-in limit stay free for the kernel's static shared memory)
-    const bool ls = random_sweep_smem(a.L, cpb, true) + 512 <= smem_optin;
-    const size_t smem = random_sweep_smem(a.L, cpb, ls);
+    auto fits = [&](uint32_t pitch) { return random_sweep_smem(a.L, pitch, true) + 512 <= smem_optin; };
+    const uint32_t whole = (cpb + 31u) / 32u * 32u, pitch = fits(whole) ? whole : cpb;
+    const bool ls = fits(pitch);
+    const size_t smem = random_sweep_smem(a.L, pitch, ls);
     if (smem + 512 > smem_optin) return cudaErrorInvalidValue;
     const size_t limit = smem_optin - 512;
     if (rounds == 10)
-        return ls ? launch_random_one<10, true>(a, cpb, blocks, smem, limit, s) : launch_random_one<10, false>(a, cpb, blocks, smem, limit, s);
-    return ls ? launch_random_one<7, true>(a, cpb, blocks, smem, limit, s) : launch_random_one<7, false>(a, cpb, blocks, smem, limit, s);
+        return ls ? launch_random_one<10, true>(a, cpb, pitch, blocks, smem, limit, s) : launch_random_one<10, false>(a, cpb, pitch, blocks, smem, limit, s);
+    return ls ? launch_random_one<7, true>(a, cpb, pitch, blocks, smem, limit, s) : launch_random_one<7, false>(a, cpb, pitch, blocks, smem, limit, s);
 }
 
 }  // namespace muca

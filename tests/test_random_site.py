@@ -117,3 +117,44 @@ def test_row_from_high_product_is_exact():
         inv = ((1 << 32) + L - 1) // L
         idx = np.arange(N, dtype=np.uint64)
         assert np.array_equal((idx * np.uint64(inv)) >> np.uint64(32), idx // np.uint64(L)), L
+
+
+def test_site_split_in_fp32_is_exact():
+    """The kernel's split of idx = row L + col: row = floor((idx + 1/2) / L)
+    as one FP32 fused multiply-add, rounded down."""
+    f = np.float32
+    for L in range(3, 129):
+        idx = np.arange(L * L)
+        inv = f(1) / f(L)
+        x = (idx * np.float64(inv) + np.float64(f(0.5) * inv)).astype(f)
+        assert np.array_equal(np.floor(x).astype(np.int64), idx // L), L
+
+
+# lattices in shared memory with padded and unpadded columns (130 chains per
+# SM at L = 72) and in global memory (140; L = 128 with padding lanes), row
+# remainders of 1, 2 and 16 sites, lanes without a chain, groups of 1..3
+# attempts at the end of either phase, several launches
+@pytest.mark.gpu
+@pytest.mark.parametrize("L,nch,therm,nup", [
+    (3, 5, 3, 21), (8, 300, 2, 7), (15, 33, 5, 41), (16, 40, 0, 6), (17, 4000, 1, 9), (33, 100, 7, 30),
+    (72, 19760, 2, 5), (72, 21280, 3, 6), (128, 4560, 4, 7), (128, 300, 0, 1), (32, 40000, 1, 3)])
+def test_random_site_layouts(muca, orc, L, nch, therm, nup):
+    N = L * L
+    lnw = np.cumsum(np.random.default_rng(L + nch).normal(-0.2, 0.6, N + 1))
+    orc.use_device_logf(False)
+    with muca.Engine(L, nchains=nch, algorithm=muca.ALGO_RANDOM_SITE, host_logf=1) as e:
+        e.set_weights(lnw)
+        e.init_chains(muca.INIT_MUCA_MAG, 2)
+        lat = e.get_lattice().copy()
+        ej, ed, _ = (np.asarray(x).astype(np.int32).copy() for x in e.chain_state())
+        for it in (0, 5):
+            e.sweep(it, 2, 0, therm, nup)
+        got, (ej1, ed1, _), h = e.get_lattice(), e.chain_state(), e.histogram()
+    oh = np.zeros(N + 1, np.uint64)
+    for it in (0, 5):
+        lat, ej, ed, hi = _oracle_chains(orc, L, nch, 2, lnw, it, 2, therm, nup, lat, ej, ed)
+        oh = hi if it else oh
+    np.testing.assert_array_equal(got, lat)
+    np.testing.assert_array_equal(ej1, ej)
+    np.testing.assert_array_equal(ed1, ed)
+    np.testing.assert_array_equal(h, oh)
