@@ -25,11 +25,10 @@
 //
 // What bounds it: at one warp per SM sub-partition the instructions of the
 // warp, and beneath them the chain from one attempt's store to the next one's
-// loads and decision.  So what does not depend on the spins (the draws, the
-// sites, the addresses of their neighbours) is formed one group of four
-// attempts ahead, in the same stretch of code as the scan of the group before,
-// and the scan has no branch: an attempt in doubt is noticed at the end of its
-// group, whose stores are then taken back and repeated.
+// loads and decision.  So the draws come one group of four attempts ahead of the
+// scan, in one stretch of code with it and with the sites' and neighbours'
+// addresses, and the scan has no branch: an attempt in doubt is noticed at the
+// end of its group, whose stores are then taken back and repeated.
 //   * a site is split into row and column with FP32 (exact: idx < 2^14); a
 //     number in the mantissa of 2^23 goes into the address products as it is,
 //     the constant they carry is in the address base;
@@ -38,8 +37,12 @@
 //     the float 2^23 + entry;
 //   * lattice columns in shared memory lie a multiple of 32 lanes apart where
 //     that fits, so that lanes at different sites meet no bank conflict.
-// L = 72, 16384 chains, 85 M attempts: @@ us, 1815 us with draws, site and
-// test of every attempt on one dependency chain.
+// L = 72, 16384 chains, 85 M attempts: 0.56 ms (205 cycles an attempt and
+// warp); 0.68 with the addresses too kept from one group to the next (a move for
+// each), selects instead of predicated additions and stores, and a group's
+// length tested in its loop; 0.79 with tables of a row's and a column's
+// addresses in shared memory; 1.79 with draws, site and test of every attempt on
+// one dependency chain.
 #include "window.cuh"
 
 #include <algorithm>
@@ -52,9 +55,14 @@ __host__ __device__ inline size_t random_smem_base(uint32_t N)
     return 16 + 2 * align16((size_t)(N + 1) * 4);
 }
 
-// The drawn side of an attempt: the acceptance logarithm, the byte offsets of
-// the site's word and its neighbours', twice their sites (rotations count
-// modulo 32), and the selector of the byte tables less the site's code.
+// What a group's draws leave for its scan: the acceptance logarithm, 2^23 + site
+// and the selector of the byte tables less the site's code ...
+struct RandomDraw {
+    float l, ib;
+    uint32_t dsel;
+};
+// ... and with the byte offsets of the site's word and its neighbours', and twice
+// their columns (rotations count modulo 32).
 struct RandomAttempt {
     float l;
     uint32_t aC, aU, aD, aL, aR, sC, sL, sR, dsel;
@@ -81,6 +89,7 @@ __global__ void __launch_bounds__(256) k_sweep_random(const RandomArgs a, uint32
     const uint32_t N = a.N, L = a.L, WPR = a.WPR, nt = blockDim.x, tid = threadIdx.x, lane = threadIdx.x;
     float *u = reinterpret_cast<float *>(smem + 16);
     uint32_t *histS = reinterpret_cast<uint32_t *>(smem + 16 + align16((size_t)(N + 1) * 4));
+    const uint32_t hist_off = 16u + (uint32_t)align16((size_t)(N + 1) * 4);
     const uint32_t lat_off = (uint32_t)random_smem_base(N);
     const double *__restrict__ w64 = a.w;
     const uint32_t words = L * WPR;
@@ -111,23 +120,21 @@ __global__ void __launch_bounds__(256) k_sweep_random(const RandomArgs a, uint32
     s2.init(100u * W + 4000u * a.seed, 0x20202041u, 0xbadbad11u, 2u * iter);
     s3.init(1000u * W + 10000u * a.seed, 0x11cafeadu, 0xbadbad11u, 2u * iter);
     // lanes without a chain: an infinite logarithm (or a NaN), so they never
-    // accept, E_Delta stays 1, and they count in the bin after the last, which
-    // the rounded-up size of the histogram has (N + 1 is no multiple of 4)
+    // accept, and E_Delta stays N + 1: they count in the bin after the last,
+    // which the rounded-up sizes of the arrays have (N + 1 is no multiple of 4)
     const float ln2 = active ? kLn2 : -INFINITY;
-    uint32_t e4 = active ? 4u * (uint32_t)a.edel[chain] : 4u;
+    uint32_t e4 = active ? 4u * (uint32_t)a.edel[chain] : 4u * (N + 1u);
     float ej2 = active ? (float)(2 * a.ej[chain]) : 0.0f;
-    unsigned char *hist_lane = reinterpret_cast<unsigned char *>(histS) + (active ? 0u : 4u * N);
 
     unsigned char *const base = LAT_SMEM ? smem : reinterpret_cast<unsigned char *>(a.lat + (size_t)blockIdx.x * words * cpb);
     const uint32_t p4 = 4u * (LAT_SMEM ? pitch : cpb), rs = WPR * p4;  // bytes from a word (row) to the next
     // word q of row r lies at bits(2^23 + r) rs + (bits(2^23 + col) >> 4) p4 + k0
     const uint32_t k0 = (LAT_SMEM ? lat_off : 0u) + 4u * column - 0x4B000000u * rs - 0x04B00000u * p4;
     const float fN = (float)N, fL = (float)L, inv = __frcp_rn(fL), half_inv = 0.5f * inv, magic = 8388608.0f;
-    const float row_last = magic + (fL - 1.0f);
-    const uint32_t col_last = 0x4B000000u + L - 1u, wrap = (L - 1u) * rs;
+    const float last = magic + (fL - 1.0f);
 
     auto word = [&](uint32_t off) -> uint32_t & { return *reinterpret_cast<uint32_t *>(base + off); };
-    auto prep = [&](uint32_t c, RandomAttempt (&at)[4]) {
+    auto prep = [&](uint32_t c, RandomDraw (&at)[4]) {
         uint32_t r1[4], r2[4], r3[4];
         const unsigned long long q = (unsigned long long)kPhiloxM0 * c;
         s1.block(q, r1);
@@ -135,24 +142,34 @@ __global__ void __launch_bounds__(256) k_sweep_random(const RandomArgs a, uint32
         s3.block(q, r3);
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
-            RandomAttempt &x = at[t];
+            RandomDraw &x = at[t];
             x.l = __fmul_rn(lg2_ftz(u01s(r1[t])), ln2);
-            // 2^23 + idx, idx = (unsigned)(u N); row = floor((idx + 1/2) / L)
-            const float ib = __fadd_rz(__fmul_rn(u01s(r2[t]), fN), magic);
-            const float rowb = __fadd_rz(__fmaf_rn(__fsub_rn(ib, magic), inv, half_inv), magic);
-            const float colb = __fmaf_rn(__fsub_rn(rowb, magic), -fL, ib);
-            const uint32_t col = __float_as_uint(colb), row = __float_as_uint(rowb) * rs + k0;
-            const uint32_t cl = colb == magic ? col_last : col - 1u, cr = col == col_last ? 0x4B000000u : col + 1u;
-            x.aC = (col >> 4) * p4 + row;
-            x.aU = x.aC + (rowb == row_last ? 0u - wrap : rs);
-            x.aD = x.aC + (rowb == magic ? wrap : 0u - rs);
-            x.aL = (cl >> 4) * p4 + row;
-            x.aR = (cr >> 4) * p4 + row;
-            x.sC = 2u * col;
-            x.sL = 2u * cl;
-            x.sR = 2u * cr;
+            x.ib = __fadd_rz(__fmul_rn(u01s(r2[t]), fN), magic);  // 2^23 + idx, idx = (unsigned)(u N)
             x.dsel = ((r3[t] >> 29) & 4u) | kRndSel;  // u01fixedpt<float>(r3) < 0.5 <=> top bit clear: s + 1
         }
+    };
+    auto place = [&](const RandomDraw &d) -> RandomAttempt {
+        RandomAttempt x;
+        x.l = d.l;
+        x.dsel = d.dsel;
+        // row = floor((idx + 1/2) / L)
+        const float rowb = __fadd_rz(__fmaf_rn(__fsub_rn(d.ib, magic), inv, half_inv), magic);
+        const float colb = __fmaf_rn(__fsub_rn(rowb, magic), -fL, d.ib);
+        const uint32_t col = __float_as_uint(colb), row = __float_as_uint(rowb) * rs + k0;
+        uint32_t cl = col - 1u, cr = col + 1u;
+        add_if(colb == magic, cl, L);
+        add_if(colb == last, cr, 0u - L);
+        x.aC = (col >> 4) * p4 + row;
+        x.aU = x.aC + rs;
+        x.aD = x.aC - rs;
+        add_if(rowb == last, x.aU, 0u - L * rs);
+        add_if(rowb == magic, x.aD, L * rs);
+        x.aL = (cl >> 4) * p4 + row;
+        x.aR = (cr >> 4) * p4 + row;
+        x.sC = 2u * col;
+        x.sL = 2u * cl;
+        x.sR = 2u * cr;
+        return x;
     };
     // code of the site that the rotation brings to the bottom
     auto code = [](uint32_t w, uint32_t s2x) -> uint32_t { return __funnelshift_r(w, w, s2x) & 3u; };
@@ -177,88 +194,90 @@ __global__ void __launch_bounds__(256) k_sweep_random(const RandomArgs a, uint32
     auto U = [&](uint32_t e) -> float { return *reinterpret_cast<const float *>(uS + e); };
 
     uint32_t c0 = 1;
-    RandomAttempt nx[4];
+    RandomDraw nx[4];
     prep(c0, nx);
-    uint32_t unflushed = 0;
-    auto run = [&](unsigned long long n, auto rec) {
-        constexpr bool REC = decltype(rec)::value;
-        while (n > 0) {
-            const uint32_t len = n < 4ull ? (uint32_t)n : 4u;
-            n -= len;
-            RandomAttempt at[4];
+    auto group = [&](uint32_t len, auto rec, auto part) {
+        constexpr bool REC = decltype(rec)::value, PART = decltype(part)::value;
+        RandomAttempt at[4];
 #pragma unroll
-            for (int t = 0; t < 4; ++t) at[t] = nx[t];
-            if (len < 4u) {
+        for (int t = 0; t < 4; ++t) at[t] = place(nx[t]);
+        if (PART) {
 #pragma unroll
-                for (int t = 1; t < 4; ++t)
-                    if ((uint32_t)t >= len) at[t].l = INFINITY;  // never accepted
+            for (int t = 1; t < 4; ++t)
+                if ((uint32_t)t >= len) at[t].l = INFINITY;  // never accepted
+        }
+        prep(c0 + 1u, nx);
+        const uint32_t e4_0 = e4;
+        const float ej2_0 = ej2;
+        uint32_t old[4], Es[4];
+        bool near = false;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const RandomAttempt &x = at[t];
+            const float um = U(e4 - 4u), up = U(e4);
+            const Move m = decode(x);
+            const float nd = __fsub_rn(__uint_as_float(prmt_var(kRndND_0, kRndND_1, m.sel)), 8388609.0f);
+            // logf(u) - f2 - (w[E + dDel] - w[E]), f2 = -2 dE = dv ns2
+            const float g = __fmaf_rn(nd, nd > 0.0f ? um : up, __fmaf_rn(-m.dv, m.ns2, x.l));
+            const bool acc = g < 0.0f;
+            near |= !(fabsf(g) > band);  // a NaN (differences beyond FP32) is in doubt too
+            old[t] = m.word;
+            const uint32_t step = prmt_var(kRndD4_0, kRndD4_1, m.sel) - 4u, changed = m.word ^ moved(x, m);
+            if (acc) {
+                word(x.aC) = changed;
+                ej2 = __fmaf_rn(-m.dv, m.ns2, ej2);
             }
-            prep(c0 + 1u, nx);
-            const uint32_t e4_0 = e4;
-            const float ej2_0 = ej2;
-            uint32_t old[4], Es[4];
-            bool near = false;
+            add_if(acc, e4, step);
+            Es[t] = e4;
+        }
+        if (near) {
+            // in doubt: the group again, with the reference's FP64
+            // difference and exact log
+            uint32_t r1[4];
+            s1.block((unsigned long long)kPhiloxM0 * c0, r1);
+            e4 = e4_0;
+            ej2 = ej2_0;
+            if (store) {
+#pragma unroll
+                for (int t = 3; t >= 0; --t) word(at[t].aC) = old[t];
+            }
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
-                const RandomAttempt &x = at[t];
-                const float um = U(e4 - 4u), up = U(e4);
-                const Move m = decode(x);
-                const float nd = __fsub_rn(__uint_as_float(prmt_var(kRndND_0, kRndND_1, m.sel)), 8388609.0f);
-                // logf(u) - f2 - (w[E + dDel] - w[E]), f2 = -2 dE = dv ns2
-                const float g = __fmaf_rn(nd, nd > 0.0f ? um : up, __fmaf_rn(-m.dv, m.ns2, x.l));
-                const bool acc = g < 0.0f;
-                near |= !(fabsf(g) > band);  // a NaN (differences beyond FP32) is in doubt too
-                old[t] = m.word;
-                const uint32_t next = e4 + prmt_var(kRndD4_0, kRndD4_1, m.sel) - 4u;
-                const uint32_t changed = m.word ^ (acc ? moved(x, m) : 0u);
-                if (store) word(x.aC) = changed;
-                if (acc) ej2 = __fmaf_rn(-m.dv, m.ns2, ej2);
-                e4 = acc ? next : e4;
+                const Move m = decode(at[t]);
+                const int E = (int)(e4 >> 2), d4 = (int)prmt_var(kRndD4_0, kRndD4_1, m.sel) - 4;
+                if (active && (uint32_t)t < len) {
+                    const double diff = __dsub_rn(__dadd_rn((double)__fmul_rn(m.dv, m.ns2), w64[E + d4 / 4]), w64[E]);
+                    bool acc = diff >= 0.0;
+                    if (!acc) {
+                        const float lg = a.logf_tab ? __ldg(a.logf_tab + (r1[t] >> 9)) : logf(u01s(r1[t]));
+                        acc = (double)lg < diff;
+                    }
+                    if (acc) {
+                        word(at[t].aC) = m.word ^ moved(at[t], m);
+                        ej2 = __fmaf_rn(-m.dv, m.ns2, ej2);
+                        e4 += (uint32_t)d4;
+                    }
+                }
                 Es[t] = e4;
             }
-            if (near) {
-                // in doubt: the group again, with the reference's FP64
-                // difference and exact log
-                uint32_t r1[4];
-                s1.block((unsigned long long)kPhiloxM0 * c0, r1);
-                e4 = e4_0;
-                ej2 = ej2_0;
-                if (store) {
-#pragma unroll
-                    for (int t = 3; t >= 0; --t) word(at[t].aC) = old[t];
-                }
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    const Move m = decode(at[t]);
-                    const int E = (int)(e4 >> 2), d4 = (int)prmt_var(kRndD4_0, kRndD4_1, m.sel) - 4;
-                    if (active && (uint32_t)t < len) {
-                        const double diff = __dsub_rn(__dadd_rn((double)__fmul_rn(m.dv, m.ns2), w64[E + d4 / 4]), w64[E]);
-                        bool acc = diff >= 0.0;
-                        if (!acc) {
-                            const float lg = a.logf_tab ? __ldg(a.logf_tab + (r1[t] >> 9)) : logf(u01s(r1[t]));
-                            acc = (double)lg < diff;
-                        }
-                        if (acc) {
-                            word(at[t].aC) = m.word ^ moved(at[t], m);
-                            ej2 = __fmaf_rn(-m.dv, m.ns2, ej2);
-                            e4 += (uint32_t)d4;
-                        }
-                    }
-                    Es[t] = e4;
-                }
-            }
-            ++c0;
-            if (REC) {
-#pragma unroll
-                for (int t = 0; t < 4; ++t)
-                    if (t == 0 || (uint32_t)t < len) atomicAdd(reinterpret_cast<uint32_t *>(hist_lane + Es[t]), 1u);
-                // no more than 256 lanes x 4 x 2^20 = 2^30 entries between two flushes
-                if (++unflushed == (1u << 20)) {
-                    flush_hist<kModeWeight>(histS, a.hist, N);
-                    unflushed = 0;
-                }
-            }
         }
+        ++c0;
+        if (REC) {
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+                if (!PART || (uint32_t)t < len) atomicAdd(reinterpret_cast<uint32_t *>(smem + hist_off + Es[t]), 1u);
+        }
+    };
+    auto run = [&](unsigned long long n, auto rec) {
+        while (n >= 4ull) {
+            const uint32_t m = n < 1ull << 22 ? (uint32_t)n / 4u : 1u << 20;
+#pragma unroll 2
+            for (uint32_t i = 0; i < m; ++i) group(4u, rec, std::false_type{});
+            n -= 4ull * m;
+            // no more than 256 lanes x 4 x 2^20 = 2^30 entries between two flushes
+            if (decltype(rec)::value && n >= 4ull) flush_hist<kModeWeight>(histS, a.hist, N);
+        }
+        if (n > 0) group((uint32_t)n, rec, std::true_type{});
     };
     run(a.therm, std::false_type{});
     run(nup, std::true_type{});
