@@ -9,22 +9,24 @@
 // m = -i, -i+2, ..., i at (i^2 + 2i + m)/2 = i(i+1)/2 + (m+i)/2.
 //
 // The sums stream the u64 histogram once (HBM bound at 8 B per bin), one
-// warp per row, with exact integer moments per row (see k_observables);
+// warp per row, with exact integer moments per row (see row_moments);
 // the per-row FP64 terms are combined per warp, per block and then in a
 // fixed-order second pass, so the result is deterministic and agrees with
 // the long-double host sum to ~1e-15.
 #include "muca_device.cuh"
 #include "muca_internal.h"
 
+#include <algorithm>
 #include <mutex>
 
 namespace muca {
 
-constexpr int kObsThreads = 256;
-// 2 blocks per SM are resident (96 registers per thread), so the grid is one
-// wave of them over the 152 SMs of GB300 (measured: 12 % faster at L=96 than
-// two waves of 608 blocks)
-constexpr int kObsBlocks = 152 * 2;
+constexpr int kObsThreads = 512;
+// One block for each of the 152 SMs of GB300, 16 warps with 32 loads of 256 B
+// each in flight.  L = 128: 169 us a pass; 24 warps with 16 loads each 174.
+constexpr int kObsBlocks = 152;
+constexpr int kObsRows = 8;  // rows of a warp at most
+static_assert(kObsBlocks * (kObsThreads / 32) * kObsRows >= 16385, "rows of the largest lattice");
 
 __global__ void k_weight_shift(double *lnw, uint32_t N, double beta, double delta)
 {
@@ -51,14 +53,22 @@ __global__ void k_weight_shift(double *lnw, uint32_t N, double beta, double delt
 }
 
 // One warp per row of the triangle at a time (row i = E_Delta holds the i+1
-// bins m = -i, -i+2, ..., i from b = i(i+1)/2): the lanes stream the row's
-// u64 counts with coalesced loads, 2 kObsUnroll independent loads per lane
-// in flight (double-buffered).  Within a row boltz_i is a common factor, so the lanes sum
-// H, |m| H, m^2 H and m^4 H exactly in 128-bit integers (integer pipes; FP64
-// issues slowly on this GPU), the warp reduces them, and lane 0 adds
-// sum_k(i) * boltz_i to its FP64 accumulators: one FP64 product per row and
-// moment instead of one per bin.  Warp w takes rows w, w + W, w + 2W, ...
-// (W warps in the grid), which spreads the long rows evenly.
+// bins m = -i, -i+2, ..., i from b = i(i+1)/2).  Within a row boltz_i is a
+// common factor, so H, |m| H, m^2 H and m^4 H are summed exactly in integers
+// (row_moments), and one FP64 product per row and moment follows.
+//
+// HBM bounds it: the histogram is read once.  To stay there a bin may cost
+// about 44 issue cycles of a warp (152 SMs, 6.7 TB/s); with 128-bit products
+// per bin it took 96.  So the moments are formed without a product:
+//   * the bins of m and -m are folded, since every moment is one of |m|;
+//   * lane l takes |m| = b + 64 k, b = (i & 1) + 2 l, for k = K-1 ... 0 and runs
+//     five nested sums, c0 += G, c1 += c0, ... c4 += c3, which end as
+//     e_p = sum_k C(k+p, p) G_k: ten additions for two bins;
+//   * the sums of k^p G and of |m|^p G follow from them once per row.
+// They are 64-bit: G < 2^30 and K <= 256 keep e4 <= 2^30 C(260, 5) < 2^64.  A
+// row with a bin of 2^29 or more is summed again with 128-bit products, bin by
+// bin; both give the exact sums.
+// L = 128 (1.07 GB): 169 us a pass (6.4 TB/s), 351 with products for every bin.
 constexpr int kObsUnroll = 8;
 
 typedef unsigned __int128 u128;
@@ -76,88 +86,196 @@ __device__ __forceinline__ double u128_to_double(u128 v)
                      (double)(unsigned long long)v);
 }
 
-__global__ void __launch_bounds__(kObsThreads) k_observables(const unsigned long long *__restrict__ hist,
+// A sum of terms >= 0 with the error of its additions beside it (the larger
+// operand first, so three operations give it): chi subtracts <m>^2 from <m^2>,
+// which magnifies what the sums lose to rounding.
+struct DoubleSum {
+    double h = 0.0, l = 0.0;
+    __device__ __forceinline__ void add(double x)
+    {
+        const bool swap = __double_as_longlong(h) < __double_as_longlong(x);
+        const double a = swap ? x : h, b = swap ? h : x, t = __dadd_rn(a, b);
+        l = __dadd_rn(l, __dsub_rn(b, __dsub_rn(t, a)));
+        h = t;
+    }
+    __device__ __forceinline__ void join_xor(int o)
+    {
+        const double oh = __shfl_xor_sync(0xffffffffu, h, o), ol = __shfl_xor_sync(0xffffffffu, l, o);
+        l = __dadd_rn(l, ol);
+        add(oh);
+    }
+    // (of an overflowed sum the error is a NaN)
+    __device__ __forceinline__ double value() const { return l == l ? __dadd_rn(h, l) : h; }
+};
+
+struct RowMoments {
+    u128 a0, a1, a2, a4;  // sums of H, |m| H, m^2 H, m^4 H
+};
+
+// A lane's part of row i with bins of any size: j = lane, lane + 32, ...
+__device__ __forceinline__ RowMoments row_moments_wide(const unsigned long long *row, uint32_t i, uint32_t lane)
+{
+    RowMoments r{0, 0, 0, 0};
+#pragma unroll 1
+    for (uint32_t j = lane; j <= i; j += 32u) {
+        const unsigned long long H = row[j];
+        const int m = 2 * (int)j - (int)i;
+        const uint32_t am = (uint32_t)(m < 0 ? -m : m);  // <= N <= 16384
+        const uint32_t am2 = am * am;                    // < 2^29
+        // 64 x 32-bit products; H m^4 = (H m^2) m^2 with H m^2 < 2^93
+        const u128 t = (u128)H * am2;
+        const unsigned long long tl = (unsigned long long)t, th = (unsigned long long)(t >> 64);
+        r.a0 += H;
+        r.a1 += (u128)H * am;
+        r.a2 += t;
+        r.a4 += (u128)tl * am2 + ((u128)(th * am2) << 64);
+    }
+    return r;
+}
+
+// A lane's part of row i by nested sums (above); bins past 2^29 are reported
+// in `big`.
+__device__ __forceinline__ RowMoments row_moments(const unsigned long long *row, uint32_t i, uint32_t lane, bool &big)
+{
+    typedef unsigned long long u64;
+    // |m| = (i & 1) + 2 n, n = 0 .. i/2: bins (i+1)/2 + n and i/2 - n
+    const uint32_t half = i / 2 + 1;
+    const u64 *up = row + (i + 1) / 2, *dn = row + i / 2;
+    constexpr int U = kObsUnroll;
+    int k = (int)((half + 32u * U - 1) / (32u * U)) * U - 1;  // K - 1, K a multiple of U
+    u64 hu[U], hd[U], nu[U], ndn[U];
+    auto load = [&](int k0, u64 (&a)[U], u64 (&b)[U]) {
+#pragma unroll
+        for (int t = 0; t < U; ++t) {
+            const uint32_t n = lane + 32u * (uint32_t)(k0 - t);
+            const bool in = k0 - t >= 0 && n < half;
+            a[t] = in ? __ldcs(up + n) : 0ull;
+            b[t] = in ? __ldcs(dn - (int)n) : 0ull;
+        }
+    };
+    load(k, hu, hd);
+    u64 c0 = 0, c1 = 0, c2 = 0, c3 = 0, c4 = 0;
+    uint32_t any_hi = 0, any_lo = 0;
+    for (; k >= 0; k -= U) {
+        load(k - U, nu, ndn);
+#pragma unroll
+        for (int t = 0; t < U; ++t) {
+            any_hi |= (uint32_t)(hu[t] >> 32) | (uint32_t)(hd[t] >> 32);
+            any_lo |= (uint32_t)hu[t] | (uint32_t)hd[t];
+            c0 += (uint32_t)hu[t] + (uint32_t)hd[t];
+            c1 += c0;
+            c2 += c1;
+            c3 += c2;
+            c4 += c3;
+        }
+#pragma unroll
+        for (int t = 0; t < U; ++t) {
+            hu[t] = nu[t];
+            hd[t] = ndn[t];
+        }
+    }
+    big = any_hi != 0 || (any_lo >> 29) != 0;
+    if ((i & 1u) == 0 && lane == 0) {
+        // the bin m = 0 was folded with itself
+        const u64 z = *dn;
+        c0 -= z;
+        c1 -= z;
+        c2 -= z;
+        c3 -= z;
+        c4 -= z;
+    }
+    // s_p = sum_k k^p G_k from C(k+1,1) = k + 1, 2 C(k+2,2) = k^2 + 3k + 2,
+    // 6 C(k+3,3) = k^3 + 6k^2 + 11k + 6, 24 C(k+4,4) = k^4 + 10k^3 + 35k^2 + 50k + 24
+    const u64 s1 = c1 - c0, s2 = 2 * c2 - 3 * s1 - 2 * c0, s3 = 6 * c3 - 6 * s2 - 11 * s1 - 6 * c0;
+    const u128 s4 = (u128)c4 * 24u - (u128)s3 * 10u - (u128)s2 * 35u - (u128)s1 * 50u - (u128)c0 * 24u;
+    const uint32_t b = (i & 1u) + 2u * lane, b2 = b * b;  // <= 63
+    RowMoments r;
+    r.a0 = c0;
+    r.a1 = (u64)b * c0 + 64u * s1;  // < 2^52
+    r.a2 = (u128)c0 * b2 + (u128)s1 * (128u * b) + (u128)s2 * 4096u;
+    r.a4 = (u128)c0 * (b2 * b2) + (u128)s1 * (256u * b2 * b) + (u128)s2 * (24576u * b2) + (u128)s3 * (1048576u * b) +
+           (s4 << 24);
+    return r;
+}
+
+__global__ void __launch_bounds__(kObsThreads, 1) k_observables(const unsigned long long *__restrict__ hist,
                                                              const double *__restrict__ lnw, uint32_t N,
                                                              double beta, double delta,
                                                              double *__restrict__ partials)
 {
     const double nbd = __dmul_rn(-beta, delta);
-    double s0 = 0, s1 = 0, s2 = 0, s4 = 0;
     const uint32_t ln = threadIdx.x & 31u;
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i <= N; i += nwarps) {
-        const unsigned long long *row = hist + (unsigned long long)i * (i + 1) / 2;
-        u128 a0 = 0, a1 = 0, a2 = 0, a4 = 0;
-        // double-buffered: the next chunk's loads are in flight while this one is summed
-        unsigned long long h[kObsUnroll], hn[kObsUnroll];
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5, w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    // Warp w takes the w-th longest row, then that many from the other end of
+    // the next nwarps rows, and so on, so that all warps read about as much.
+    // Lane s keeps the s-th row's sums: FP64 issues slowly on this GPU, so the
+    // terms of all rows are formed at once.
+    uint32_t first = 0, slot = 0, my_row = 0;
+    RowMoments mine{0, 0, 0, 0};
+    bool turn = false;
+    while (first <= N) {
+        const uint32_t at = first + (turn ? nwarps - 1u - w : w);
+        if (at <= N) {
+            const uint32_t i = N - at;
+            const unsigned long long *row = hist + (unsigned long long)i * (i + 1) / 2;
+            bool big;
+            RowMoments r = row_moments(row, i, ln, big);
+            if (__any_sync(0xffffffffu, big)) r = row_moments_wide(row, i, ln);
 #pragma unroll
-        for (int k = 0; k < kObsUnroll; ++k) {
-            const uint32_t j = ln + 32u * k;
-            h[k] = j <= i ? __ldcs(row + j) : 0ull;
-        }
-        for (uint32_t j0 = 0; j0 <= i; j0 += 32u * kObsUnroll) {
-#pragma unroll
-            for (int k = 0; k < kObsUnroll; ++k) {
-                const uint32_t j = j0 + 32u * kObsUnroll + ln + 32u * k;
-                hn[k] = j <= i ? __ldcs(row + j) : 0ull;
+            for (int o = 16; o > 0; o >>= 1) {
+                r.a0 += shfl_xor_u128(r.a0, o);
+                r.a1 += shfl_xor_u128(r.a1, o);
+                r.a2 += shfl_xor_u128(r.a2, o);
+                r.a4 += shfl_xor_u128(r.a4, o);
             }
-#pragma unroll
-            for (int k = 0; k < kObsUnroll; ++k) {
-                const unsigned long long H = h[k];
-                const int m = 2 * (int)(j0 + ln + 32u * k) - (int)i;
-                const uint32_t am = (uint32_t)(m < 0 ? -m : m);  // <= N <= 16384
-                const uint32_t am2 = am * am;                    // < 2^29
-                // 64 x 32-bit products; H m^4 = (H m^2) m^2 with H m^2 < 2^93
-                const u128 t = (u128)H * am2;
-                const unsigned long long tl = (unsigned long long)t, th = (unsigned long long)(t >> 64);
-                a0 += H;
-                a1 += (u128)H * am;
-                a2 += t;
-                a4 += (u128)tl * am2 + ((u128)(th * am2) << 64);
+            if (ln == slot) {
+                mine = r;
+                my_row = i;
             }
-#pragma unroll
-            for (int k = 0; k < kObsUnroll; ++k) h[k] = hn[k];
+            ++slot;
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            a0 += shfl_xor_u128(a0, o);
-            a1 += shfl_xor_u128(a1, o);
-            a2 += shfl_xor_u128(a2, o);
-            a4 += shfl_xor_u128(a4, o);
-        }
-        if (ln == 0 && a0 != 0) {
-            const double bz = exp(__dsub_rn(__dmul_rn(nbd, (double)i), lnw[i]));
-            s0 = __dadd_rn(s0, __dmul_rn(u128_to_double(a0), bz));
-            s1 = __dadd_rn(s1, __dmul_rn(u128_to_double(a1), bz));
-            s2 = __dadd_rn(s2, __dmul_rn(u128_to_double(a2), bz));
-            s4 = __dadd_rn(s4, __dmul_rn(u128_to_double(a4), bz));
-        }
+        first += nwarps;
+        turn = !turn;
     }
-    __shared__ double sh[4][kObsThreads / 32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-        s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-        s4 += __shfl_xor_sync(0xffffffffu, s4, o);
+    __shared__ double terms[4][kObsThreads / 32][kObsRows];
+    if (ln < (uint32_t)kObsRows) {
+        double t0 = 0.0, t1 = 0.0, t2 = 0.0, t4 = 0.0;
+        if (ln < slot && mine.a0 != 0) {
+            const double bz = exp(__dsub_rn(__dmul_rn(nbd, (double)my_row), lnw[my_row]));
+            t0 = __dmul_rn(u128_to_double(mine.a0), bz);
+            t1 = __dmul_rn(u128_to_double(mine.a1), bz);
+            t2 = __dmul_rn(u128_to_double(mine.a2), bz);
+            t4 = __dmul_rn(u128_to_double(mine.a4), bz);
+        }
+        const uint32_t wid = threadIdx.x >> 5;
+        terms[0][wid][ln] = t0;
+        terms[1][wid][ln] = t1;
+        terms[2][wid][ln] = t2;
+        terms[3][wid][ln] = t4;
     }
-    if (lane == 0) { sh[0][wid] = s0; sh[1][wid] = s1; sh[2][wid] = s2; sh[3][wid] = s4; }
     __syncthreads();
-    if (threadIdx.x < 4) {
-        double t = 0;
-        for (int w = 0; w < kObsThreads / 32; ++w) t += sh[threadIdx.x][w];
-        partials[(size_t)blockIdx.x * 4 + threadIdx.x] = t;
+    if (threadIdx.x < 128) {
+        const uint32_t q = threadIdx.x >> 5;
+        const double *of_q = &terms[q][0][0];
+        DoubleSum v;
+#pragma unroll
+        for (int k = 0; k < kObsThreads / 32 * kObsRows; k += 32) v.add(of_q[k + ln]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v.join_xor(o);
+        if (ln == 0) partials[(size_t)blockIdx.x * 4 + q] = v.value();
     }
 }
 
+// Warp q sums the blocks' partials of moment q.  (An FP64 instruction takes a
+// warp 64 cycles here, so the partials are few: one block per SM.)
 __global__ void k_observables_final(const double *partials, int nblocks, double *out)
 {
-    if (threadIdx.x < 4) {
-        double t = 0;
-        for (int b = 0; b < nblocks; ++b) t += partials[(size_t)b * 4 + threadIdx.x];
-        out[threadIdx.x] = t;
-    }
+    const uint32_t q = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    DoubleSum v;
+    for (int b = (int)lane; b < nblocks; b += 32) v.add(partials[(size_t)b * 4 + q]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v.join_xor(o);
+    if (lane == 0) out[q] = v.value();
 }
 
 // jakknife (muca_delta_multigpu.cu:620-635), one thread, same order.
@@ -189,8 +307,10 @@ size_t observables_partials(uint32_t) { return (size_t)kObsBlocks * 4; }
 cudaError_t launch_observables(const unsigned long long *hist2d, const double *lnw, uint32_t N, double beta,
                                double delta, double *partials, double *out, cudaStream_t s)
 {
-    k_observables<<<kObsBlocks, kObsThreads, 0, s>>>(hist2d, lnw, N, beta, delta, partials);
-    k_observables_final<<<1, 32, 0, s>>>(partials, kObsBlocks, out);
+    // no more warps than rows
+    const int blocks = std::min(kObsBlocks, (int)(N / (kObsThreads / 32)) + 1);
+    k_observables<<<blocks, kObsThreads, 0, s>>>(hist2d, lnw, N, beta, delta, partials);
+    k_observables_final<<<1, 128, 0, s>>>(partials, blocks, out);
     return cudaGetLastError();
 }
 
@@ -211,8 +331,8 @@ cudaError_t launch_jackknife(const double *x, uint32_t n, double *out2, cudaStre
 // them, the two kernels above run with their block partials in the
 // file-scope array below instead of context memory.
 //
-// The array holds the partials of the fixed kObsBlocks-block grid,
-// kObsBlocks x 4 doubles (9,728 bytes), whatever L is.  Each block
+// The array holds the partials of the largest grid, kObsBlocks blocks:
+// kObsBlocks x 4 doubles (4,864 bytes), whatever L is.  Each block
 // overwrites its own four entries before the final pass reads them, so
 // nothing in it has to start at zero, and no state carries from one call to
 // the next.  There is one array per device, shared by every caller in the
