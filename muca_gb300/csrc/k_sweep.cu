@@ -544,6 +544,15 @@ SweepPlan plan_sweep(int mode, int rounds, uint32_t L, uint32_t nchains, size_t 
     p.row_ring = !p.lat_smem && p.kernel == kKernelWindowed && L % 8 == 0 && front + ring_bytes(L, cpb) <= optin;
     p.smem = front + (p.kernel == kKernelSpecialized ? smem_ring_bytes(warps) : 0) +
              (p.lat_smem ? per_chain * cpb : 0) + (p.row_ring ? ring_bytes(L, cpb) : 0);
+    // Up to two warps of chains per SM leave two sub-partitions idle, which draw
+    // for them (1.2 to 1.3 times as fast, see window.cuh); a third warp of chains
+    // would have to share its sub-partition with a drawing one.
+    const size_t fed = front + align16(per_chain * cpb) + warps * kFeedBytes;
+    if (p.kernel == kKernelWindowed && p.lat_smem && warps <= 2 && fed <= optin) {
+        p.feed = true;
+        p.threads = 2u * warps * 32u;
+        p.smem = fed;
+    }
     return p;
 }
 

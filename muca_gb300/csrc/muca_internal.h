@@ -59,6 +59,7 @@ struct SweepPlan {
     int rounds;
     int kernel;      // SweepKernel
     bool many;       // windowed kernel with more than one warp of chains per SM sub-partition
+    bool feed;       // windowed kernel with warps that draw for those that walk
     bool lat_smem;   // lattice resident in shared memory
     bool row_ring;   // lattice in global memory behind a four-row ring per lane (windowed kernel)
     uint32_t cpb;    // chains per block (lane stride of the packed lattice)

@@ -202,6 +202,127 @@ __device__ __forceinline__ Ahead next8(const AheadAny &a)
     return x;
 }
 
+// ---------------------------------------------------------------------------
+// Draws from another warp.  With no more chains than fill two of an SM's four
+// sub-partitions the idle ones draw: a warp per 32 chains writes their groups
+// into a ring in shared memory, and the warp that walks reads them.  Draws do
+// not depend on the lattice, so the two meet only once per kFeedGroups groups,
+// at a named barrier of the 64 threads that both sides pass equally often
+// (feed_halves).  Cycles per attempt at L = 72, 4000 chains: 70.5 and 76.1
+// (thermalising and recording) for 90.7 and 94.6 in one warp; production 80.5
+// and 137 for 95.6 and 150.  Halves of 8 groups: 72.1; two drawing warps for
+// one: no gain.
+constexpr uint32_t kFeedGroups = 16, kFeedSlots = 2 * kFeedGroups;  // a half of the ring; the ring
+constexpr uint32_t kFeedLogs = kFeedSlots * 32 * 16, kFeedBytes = kFeedLogs + kFeedSlots * 32 * 4;  // per warp
+// halves drawn and read in a launch: the groups of both phases and two ahead
+__device__ __forceinline__ unsigned long long feed_halves(unsigned long long therm, unsigned long long nup)
+{
+    return ((therm + 3ull) / 4ull + (nup + 3ull) / 4ull + 2ull + kFeedGroups - 1ull) / kFeedGroups;
+}
+__device__ __forceinline__ void named_sync(uint32_t id, uint32_t threads)
+{
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void named_arrive(uint32_t id, uint32_t threads)
+{
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+// the drawing warp
+template <int R>
+__device__ __forceinline__ void feed_draw(const Draws<R> &d, unsigned char *ring, uint32_t lane, uint32_t bar,
+                                          unsigned long long halves)
+{
+    for (unsigned long long t = 0; t < halves; ++t) {
+        const uint32_t h = (uint32_t)t & 1u;
+        if (t >= 2ull) named_sync(bar + 2u + h, 64u);
+        float4 *logs = reinterpret_cast<float4 *>(ring) + h * kFeedGroups * 32u + lane;
+        uint32_t *dirs = reinterpret_cast<uint32_t *>(ring + kFeedLogs) + h * kFeedGroups * 32u + lane;
+        const uint32_t c = (uint32_t)t * kFeedGroups + 1u;
+#pragma unroll 2
+        for (uint32_t g = 0; g < kFeedGroups; ++g) {
+            uint32_t r1[4], r3[4];
+            d.group(c + g, r1, r3);
+            logs[g * 32u] = make_float4(d.log_u(r1[0]), d.log_u(r1[1]), d.log_u(r1[2]), d.log_u(r1[3]));
+            dirs[g * 32u] = direction4(r3);
+        }
+        named_arrive(bar + h, 64u);
+    }
+}
+// the reader's side
+struct Feed {
+    const unsigned char *ring;  // this lane's
+    uint32_t bar, b, off;       // first group of the coming window (from 0) and its attempts used up
+    uint32_t ev, avail;         // the next event; groups that may be read
+    unsigned long long t, halves;
+    bool rel;                   // the next event gives a half back
+    __device__ __forceinline__ void init(const unsigned char *r, uint32_t lane, uint32_t id, unsigned long long n)
+    {
+        ring = r + 16u * lane;
+        bar = id;
+        b = off = ev = avail = 0;
+        t = 0;
+        halves = n;
+        rel = false;
+    }
+    // before the groups of the window at (b, off) are read: up to three from b
+    template <bool ALIGNED>
+    __device__ __forceinline__ void ready()
+    {
+        const uint32_t end = b + (ALIGNED || off == 0 ? 2u : 3u);
+        if ((int32_t)(end - ev) > 0) {  // uniform
+            __syncwarp();
+            if (rel) {
+                // every group before end - 3 has been read: half t - 2, which
+                // the producer waits for if it has a half t to draw
+                if (t < halves) named_arrive(bar + 2u + ((uint32_t)t & 1u), 64u);
+                rel = false;
+                ev = avail;
+            } else {
+                named_sync(bar + ((uint32_t)t & 1u), 64u);
+                rel = t > 0;
+                ev = rel ? avail + 2u : kFeedGroups;
+                avail += kFeedGroups;
+                ++t;
+            }
+        }
+    }
+    template <bool ALIGNED>
+    __device__ __forceinline__ void read(Ahead &a) const
+    {
+        const uint32_t s0 = b % kFeedSlots, s1 = (b + 1u) % kFeedSlots;
+        const unsigned char *dirs = ring + kFeedLogs - 12u * (threadIdx.x & 31u);
+        auto dir = [&](uint32_t s) { return *reinterpret_cast<const uint32_t *>(dirs + s * 128u); };
+        const uint32_t d = dir(s0) | dir(s1) << 16;
+        if (ALIGNED) {
+            const float4 x = *reinterpret_cast<const float4 *>(ring + s0 * 512u);
+            const float4 y = *reinterpret_cast<const float4 *>(ring + s1 * 512u);
+            a.l[0] = x.x; a.l[1] = x.y; a.l[2] = x.z; a.l[3] = x.w;
+            a.l[4] = y.x; a.l[5] = y.y; a.l[6] = y.z; a.l[7] = y.w;
+            a.dn = d;
+        } else {
+#pragma unroll
+            for (uint32_t i = 0; i < 8; ++i) {
+                const uint32_t k = (b % kFeedSlots) * 4u + off + i;
+                a.l[i] = *reinterpret_cast<const float *>(ring + (k / 4u % kFeedSlots) * 512u + k % 4u * 4u);
+            }
+            a.dn = __funnelshift_r(d, dir((b + 2u) % kFeedSlots), 4u * off) & 0x11111111u;
+        }
+    }
+};
+// flush_hist by the block's first `threads` threads
+__device__ __forceinline__ void flush_hist_of(uint32_t *histS, unsigned long long *histG, uint32_t N, uint32_t threads)
+{
+    named_sync(15u, threads);
+    for (uint32_t b = threadIdx.x; b <= N; b += threads) {
+        const uint32_t v = histS[b];
+        if (v) {
+            atomicAdd(&histG[b], (unsigned long long)v);
+            histS[b] = 0;
+        }
+    }
+    named_sync(15u, threads);
+}
+
 // Tables over the 3-bit code (s + 1) | direction << 2, direction 0: s + 1,
 // 1: s - 1 (cyclic): codes 0, 1, 2 and 4, 5, 6 (3 and 7 do not occur).
 //   code   s -> s_new   dDel   s_new - s_old
@@ -608,7 +729,8 @@ __device__ __forceinline__ uint32_t *win_prologue(const SweepArgs &a, unsigned c
 
 // The windowed sweep of chain block `blk` (cpb chains, lanes >= cpb are
 // padding): every lane draws its own Philox numbers one window ahead, so that
-// this work fills the latency of the scan.  Ends with the block synchronised
+// this work fills the latency of the scan; with FEED another warp draws them
+// (the block has twice as many threads).  Ends with the block synchronised
 // and, with HS, the shared histogram drained.
 // RING (with LAT_SMEM false): the lattice stays in global memory and each
 // lane keeps a four-row ring of its chain in shared memory (RowRing), at the
@@ -622,7 +744,7 @@ __device__ __forceinline__ uint32_t *win_prologue(const SweepArgs &a, unsigned c
 // index stays inside the weights.
 constexpr int kIdleE = 3;
 template <int MODE, int R, bool LAT_SMEM, bool HS = true, bool BT = false, bool RING = false,
-          bool ALIGNED = true, bool MANY = false>
+          bool ALIGNED = true, bool MANY = false, bool FEED = false>
 __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned char *smem, uint32_t cpb, uint32_t blk,
                                                 uint32_t iter, unsigned long long nup,
                                                 const float *__restrict__ btab = nullptr)
@@ -645,8 +767,12 @@ __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned cha
     constexpr uint32_t rmask = RING ? 3u : ~0u;
     __syncthreads();
     const double *wG = reinterpret_cast<const double *>(a.w);
-    const uint32_t chain = blk * cpb + lane;
-    const bool active = own && chain < a.nchains;
+    // the warps that walk, and with FEED as many behind them that draw for them
+    const uint32_t walkers = FEED ? blockDim.x / 2u : blockDim.x;
+    const bool draws = FEED && threadIdx.x >= walkers;
+    const uint32_t clane = draws ? threadIdx.x - walkers : lane, of_warp = clane / 32u;
+    const uint32_t chain = blk * cpb + clane;
+    const bool active = clane < cpb && chain < a.nchains;
     Draws<R> dr;
     {
         const uint32_t dev = chain / a.chains_per_dev, W = chain - dev * a.chains_per_dev;
@@ -654,6 +780,18 @@ __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned cha
         dr.s1.init(a.k1_mul * W + a.k1_add, a.k1_hi, seed, iter);
         dr.s3.init(a.k3_mul * W + a.k3_add, a.k3_hi, seed, iter);
         dr.ln2 = active ? kLn2 : -INFINITY;
+    }
+    Feed feed;
+    if constexpr (FEED) {
+        unsigned char *ring_of = smem + lat_off + align16((size_t)a.L * a.WPR * 4u * cpb) + of_warp * kFeedBytes;
+        const unsigned long long halves = feed_halves(a.therm, nup);
+        if (draws) {
+            feed_draw(dr, ring_of, threadIdx.x & 31u, 1u + 4u * of_warp, halves);
+            __syncthreads();
+            if (HS && !PROD) drain_hist<MODE>(histS, a.hist, a.N);
+            return;
+        }
+        feed.init(ring_of, threadIdx.x & 31u, 1u + 4u * of_warp, halves);
     }
     // lanes without a chain write their word and count their bin here, so that
     // the windows need no test for them
@@ -673,9 +811,13 @@ __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned cha
     const uint32_t W8 = L >> 4, per_row = L >> 1, tail = per_row & 7u;
     const uint32_t last_sites = L - 16u * (WPR - 1u);  // sites of a row's last word
     // the draws ahead: groups cc - 1 and cc (not ALIGNED: cc - 2 .. cc)
-    std::conditional_t<ALIGNED, Ahead, AheadAny> ah;
+    std::conditional_t<ALIGNED || FEED, Ahead, AheadAny> ah;
     uint32_t cc;
-    if constexpr (ALIGNED) {
+    if constexpr (FEED) {
+        feed.ready<ALIGNED>();
+        feed.read<ALIGNED>(ah);
+        cc = 0;
+    } else if constexpr (ALIGNED) {
         draw8(dr, 1u, ah);
         cc = 2;
     } else {
@@ -695,7 +837,19 @@ __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned cha
         constexpr bool REC = decltype(rc)::value, MASKED = decltype(mc)::value;
         Win<S> w;
         uint32_t c0, off = 0;
-        if constexpr (ALIGNED) {
+        if constexpr (FEED) {
+            c0 = feed.b + 1u;
+            off = feed.off;
+            if (ALIGNED) {
+                feed.b += S == 4 || (MASKED && len <= 4u) ? 1u : 2u;
+            } else {
+                feed.b += (feed.off + len) >> 2;
+                feed.off = (feed.off + len) & 3u;
+            }
+            feed.ready<ALIGNED>();
+            decode<S, HALF, BT>(Cm, Uw, Dw, side, ah, btab, w);
+            feed.read<ALIGNED>(ah);
+        } else if constexpr (ALIGNED) {
             decode<S, HALF, BT>(Cm, Uw, Dw, side, ah, btab, w);
             c0 = cc - 1u;
             // the next window's draws, independent of the scan below
@@ -821,7 +975,8 @@ __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned cha
             if (RING) ring.row_start(row, L, cpb, WPR, own);
             if (HS && !PROD && REC) {
                 if ((since + per_row) * cpb > 0xFFFFFFFFull || (a.hooks & kHookFlushRows)) {  // uniform
-                    flush_hist<MODE>(histS, a.hist, a.N);
+                    if (FEED) flush_hist_of(histS, a.hist, a.N, walkers);
+                    else      flush_hist<MODE>(histS, a.hist, a.N);
                     since = 0;
                 }
                 since += per_row;
@@ -843,7 +998,14 @@ __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned cha
             else           row_half(H1{}, rc, std::true_type{}, row, (uint32_t)n);
         }
         // a phase's draws start at a new group
-        if constexpr (!ALIGNED) {
+        if constexpr (FEED && !ALIGNED) {
+            if (feed.off) {
+                feed.off = 0;
+                ++feed.b;
+                feed.ready<ALIGNED>();
+                feed.read<ALIGNED>(ah);
+            }
+        } else if constexpr (!ALIGNED) {
             if (ah.off) {
                 shift_in(dr, ++cc, ah);
                 ah.off = 0;

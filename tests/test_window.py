@@ -190,3 +190,33 @@ def test_update_over_a_cluster(muca, orc, L, rule):
     assert (s.start, s.end) == orc.hist_range(h)
     assert s.events == int(h.sum()) and s.visited == int((h > 0).sum()) and s.min_count == int(h.min())
     np.testing.assert_allclose(s.d_kl, orc.kull_leibler(h), rtol=1e-11)
+
+
+# one and two walking warps per SM with warps that draw for them, and the first
+# chain count past that; launches that end at, before and after a half of the
+# ring (64 attempts), one half, several, none in one of the phases
+@pytest.mark.gpu
+@pytest.mark.parametrize("nch", [31, 5000, 9728, 9729])
+@pytest.mark.parametrize("L", [8, 10])
+@pytest.mark.parametrize("produce", [False, True])
+def test_draws_from_other_warps(muca, orc, L, nch, produce):
+    N = L * L
+    lnw = np.cumsum(np.random.default_rng(L + nch).normal(-0.3, 0.6, N + 1))
+    with muca.Engine(L, nchains=nch, mode=muca.MODE_PRODUCE if produce else muca.MODE_WEIGHT) as e:
+        e.set_weights(lnw)
+        e.init_chains(muca.INIT_GRADED, 0)
+        lat = e.get_lattice()
+        state = [np.ascontiguousarray(x, np.int32).copy() for x in e.chain_state()]
+        for it, (therm, nup) in enumerate([(0, 1), (52, 1), (56, 0), (53, 4), (64, 57), (N, 3 * N), (127, 65), (0, 121)]):
+            e.sweep(it, 100, 1000, therm, nup)
+            if produce:
+                lat, h = orc.produce_sweep(L, lat, *state, lnw, it, 100, therm, nup, nthreads=8)
+            else:
+                lat, h = orc.weight_sweep(L, lat, *state[:2], lnw.astype(np.float32), it, 100, therm, nup, nthreads=8)
+            np.testing.assert_array_equal(e.get_lattice(), lat)
+            ej, ed, mg = e.chain_state()
+            np.testing.assert_array_equal(ej, state[0])
+            np.testing.assert_array_equal(ed, state[1])
+            if produce:
+                np.testing.assert_array_equal(mg, state[2])
+            assert np.array_equal(e.histogram(), h)
