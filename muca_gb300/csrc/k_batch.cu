@@ -33,7 +33,9 @@ __global__ void k_batch_prep(const BatchInst *__restrict__ insts, uint32_t *__re
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) h[i] = 0ull;
 }
 
-template <int R, int LAT, bool HS>
+// FEED (shapes of one or two warps of chains per SM): as many warps more draw
+// for those that walk, see window.cuh; their rings end the shared memory.
+template <int R, int LAT, bool HS, bool FEED = false>
 __global__ void __launch_bounds__(256, 1) k_batch_sweep(const BatchInst *__restrict__ insts,
                                                          const BatchItem *__restrict__ items, uint32_t n_items,
                                                          uint32_t *__restrict__ next_item, uint32_t cpb,
@@ -42,6 +44,7 @@ __global__ void __launch_bounds__(256, 1) k_batch_sweep(const BatchInst *__restr
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint32_t s_item;
     __shared__ float s_btab[kBetaTab];
+    const uint32_t feed_off = smem_bytes - (FEED ? (cpb + 31u) / 32u * kFeedBytes : 0u);
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(next_item, 1u);
         __syncthreads();
@@ -65,12 +68,15 @@ __global__ void __launch_bounds__(256, 1) k_batch_sweep(const BatchInst *__restr
                 // (kLatWhereFits); otherwise it stays in global memory, behind
                 // a four-row ring per lane where that fits
                 const size_t base = smem_weights_bytes(kModeWeight, a.N) + (HS ? smem_hist_bytes(kModeWeight, a.N) : 0);
-                if (LAT == kLatWhereFits && base + (size_t)a.L * a.WPR * 4u * cpb <= smem_bytes)
-                    win_sweep_block<kModeWeight, R, true, HS, true>(a, smem, cpb, item.blk, iter, nup, s_btab);
-                else if (a.L % 4 == 0 && a.WPR <= 8 && base + ring_bytes(a.L, cpb) <= smem_bytes)
-                    win_sweep_block<kModeWeight, R, false, HS, true, true>(a, smem, cpb, item.blk, iter, nup, s_btab);
+                if (LAT == kLatWhereFits && base + (size_t)a.L * a.WPR * 4u * cpb <= feed_off)
+                    win_sweep_block<kModeWeight, R, true, HS, true, false, true, false, FEED>(a, smem, cpb, item.blk, iter, nup,
+                                                                                             s_btab, feed_off);
+                else if (a.L % 4 == 0 && a.WPR <= 8 && base + ring_bytes(a.L, cpb) <= feed_off)
+                    win_sweep_block<kModeWeight, R, false, HS, true, true, true, false, FEED>(a, smem, cpb, item.blk, iter, nup,
+                                                                                             s_btab, feed_off);
                 else
-                    win_sweep_block<kModeWeight, R, false, HS, true>(a, smem, cpb, item.blk, iter, nup, s_btab);
+                    win_sweep_block<kModeWeight, R, false, HS, true, false, true, false, FEED>(a, smem, cpb, item.blk, iter, nup,
+                                                                                              s_btab, feed_off);
             }
         }
         __syncthreads();
@@ -107,8 +113,10 @@ static BatchKernel batch_kernel_r(uint32_t lat, bool hist_smem)
                                 : batch_kernel_lat<R, kLatGlobal>(hist_smem);
 }
 
-static BatchKernel batch_kernel(int rounds, uint32_t lat, bool hist_smem)
+static BatchKernel batch_kernel(int rounds, uint32_t lat, bool hist_smem, bool feed)
 {
+    // where all lattices fit, "where it fits" is "in shared memory"
+    if (feed) return rounds == 10 ? k_batch_sweep<10, kLatWhereFits, true, true> : k_batch_sweep<7, kLatWhereFits, true, true>;
     return rounds == 10 ? batch_kernel_r<10>(lat, hist_smem) : batch_kernel_r<7>(lat, hist_smem);
 }
 
@@ -120,25 +128,34 @@ static cudaError_t raise_smem_limit(BatchKernel k, size_t smem_limit)
     return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_limit);
 }
 
-cudaError_t batch_sweep_occupancy(uint32_t cpb, int rounds, uint32_t lat, bool hist_smem, size_t smem,
+size_t batch_feed_smem(uint32_t cpb) { return (cpb + 31u) / 32u * kFeedBytes; }
+
+static uint32_t batch_threads(uint32_t cpb, bool feed) { return (cpb + 31u) / 32u * 32u * (feed ? 2u : 1u); }
+static bool feed_allowed(uint32_t cpb, uint32_t lat, bool hist_smem)
+{
+    return cpb <= 64 && lat != kLatGlobal && hist_smem;
+}
+
+cudaError_t batch_sweep_occupancy(uint32_t cpb, int rounds, uint32_t lat, bool hist_smem, bool feed, size_t smem,
                                   size_t smem_limit, int *blocks)
 {
-    if (lat > kLatWhereFits) return cudaErrorInvalidValue;
-    const BatchKernel k = batch_kernel(rounds, lat, hist_smem);
+    if (lat > kLatWhereFits || (feed && !feed_allowed(cpb, lat, hist_smem))) return cudaErrorInvalidValue;
+    const BatchKernel k = batch_kernel(rounds, lat, hist_smem, feed);
     const cudaError_t e = raise_smem_limit(k, smem_limit);
     if (e != cudaSuccess) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k, (int)((cpb + 31u) / 32u * 32u), smem);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k, (int)batch_threads(cpb, feed), smem);
 }
 
 cudaError_t launch_batch_sweep(const BatchInst *insts, const BatchItem *items, uint32_t n_items, uint32_t *next_item,
-                               uint32_t cpb, int rounds, uint32_t lat, bool hist_smem, uint32_t grid, size_t smem,
-                               size_t smem_limit, cudaStream_t s)
+                               uint32_t cpb, int rounds, uint32_t lat, bool hist_smem, bool feed, uint32_t grid,
+                               size_t smem, size_t smem_limit, cudaStream_t s)
 {
-    if (cpb == 0 || cpb > 256 || lat > kLatWhereFits) return cudaErrorInvalidValue;
-    const BatchKernel k = batch_kernel(rounds, lat, hist_smem);
+    if (cpb == 0 || cpb > 256 || lat > kLatWhereFits || (feed && !feed_allowed(cpb, lat, hist_smem)))
+        return cudaErrorInvalidValue;
+    const BatchKernel k = batch_kernel(rounds, lat, hist_smem, feed);
     const cudaError_t e = raise_smem_limit(k, smem_limit);
     if (e != cudaSuccess) return e;
-    k<<<grid, (cpb + 31u) / 32u * 32u, smem, s>>>(insts, items, n_items, next_item, cpb, (uint32_t)smem);
+    k<<<grid, batch_threads(cpb, feed), smem, s>>>(insts, items, n_items, next_item, cpb, (uint32_t)smem);
     return cudaGetLastError();
 }
 

@@ -17,7 +17,9 @@ __global__ void __launch_bounds__(MANY ? 512 : 128, 1) k_sweep_win(const SweepAr
     uint32_t iter;
     unsigned long long nup;
     if (!launch_params(a, iter, nup)) return;
-    win_sweep_block<MODE, R, LAT_SMEM, true, false, RING, ALIGNED, MANY, FEED>(a, smem, cpb, blockIdx.x, iter, nup);
+    win_sweep_block<MODE, R, LAT_SMEM, true, false, RING, ALIGNED, MANY, FEED>(
+        a, smem, cpb, blockIdx.x, iter, nup, nullptr,
+        FEED ? (uint32_t)(win_smem_base(MODE, a.N, true) + align16((size_t)a.L * a.WPR * 4u * cpb)) : 0u);
 }
 
 template <int MODE, int R>

@@ -55,6 +55,7 @@ struct muca_batch {
     BatchItem *d_items = nullptr;
     size_t items_cap = 0;
     uint32_t n_items = 0;
+    bool feed = false;  // the shape has drawing warps
     uint32_t *d_counters = nullptr;  // [0] next item, [1] running instances
     uint32_t *h_running = nullptr;
     unsigned int *d_err = nullptr;
@@ -215,31 +216,51 @@ size_t smem_budget(const muca_batch *b) { return b->smem_optin > 1024 ? b->smem_
 // makes the same choice per instance against the launch's size), and a
 // lattice left in global memory with its four-row ring where that fits the
 // budget (the kernel again decides per instance against the launch's size).
-size_t shape_smem(const muca_batch *b, uint32_t cpb, uint32_t lat, bool hist_smem)
+size_t shape_smem(const muca_batch *b, uint32_t cpb, uint32_t lat, bool hist_smem, bool feed = false)
 {
+    const size_t rings = feed ? batch_feed_smem(cpb) : 0, budget = smem_budget(b) > rings ? smem_budget(b) - rings : 0;
     size_t smem = 0;
     for (const muca_instance &m : b->inst) {
         const size_t with = batch_sweep_smem(m.L, cpb, true, hist_smem);
         const size_t ring = batch_sweep_smem(m.L, cpb, false, hist_smem, true);
-        const size_t without = ring <= smem_budget(b) ? ring : batch_sweep_smem(m.L, cpb, false, hist_smem);
-        const bool in = lat == kLatShared || (lat == kLatWhereFits && with <= smem_budget(b));
+        const size_t without = ring <= budget ? ring : batch_sweep_smem(m.L, cpb, false, hist_smem);
+        const bool in = lat == kLatShared || (lat == kLatWhereFits && with <= budget);
         smem = std::max(smem, in ? with : without);
     }
-    return smem;
+    return smem + rings;
 }
 
 muca_status apply_shape(muca_batch *b, const muca_batch_shape &s, uint32_t rule)
 {
     if (muca_status st = set_layout(b, s.chains_per_block, rule)) return st;
-    const size_t smem = shape_smem(b, s.chains_per_block, s.lattice_in_smem, s.hist_in_smem);
+    size_t smem = shape_smem(b, s.chains_per_block, s.lattice_in_smem, s.hist_in_smem);
     int per_sm = 0;
-    BCUDA(b, batch_sweep_occupancy(s.chains_per_block, b->rounds, s.lattice_in_smem, s.hist_in_smem, smem, smem_budget(b),
-                                   &per_sm));
+    BCUDA(b, batch_sweep_occupancy(s.chains_per_block, b->rounds, s.lattice_in_smem, s.hist_in_smem, false, smem,
+                                   smem_budget(b), &per_sm));
+    // No more than two warps of chains per SM leave sub-partitions idle to draw
+    // for them, as in a single simulation.  64 instances of L = 16..128, 256
+    // chains each: 1.44 ms a sweep with 64 chains per block, 1.77 with 128 per
+    // block, which leave none idle.
+    const uint32_t warps = (s.chains_per_block + 31u) / 32u;
+    const uint32_t waves = (b->n_items + (uint32_t)b->sms - 1) / (uint32_t)b->sms;
+    b->feed = false;
+    if (s.hist_in_smem && s.lattice_in_smem != kLatGlobal && std::min((uint32_t)std::max(per_sm, 0), waves) * warps <= 2) {
+        const size_t fed = shape_smem(b, s.chains_per_block, s.lattice_in_smem, true, true);
+        int fed_per_sm = 0;
+        if (fed <= smem_budget(b))
+            BCUDA(b, batch_sweep_occupancy(s.chains_per_block, b->rounds, s.lattice_in_smem, true, true, fed,
+                                           smem_budget(b), &fed_per_sm));
+        if (fed_per_sm >= (int)std::min((uint32_t)std::max(per_sm, 1), waves)) {
+            b->feed = true;
+            smem = fed;
+            per_sm = fed_per_sm;
+        }
+    }
     if (per_sm < 1) return bfail(b, MUCA_ERR_BAD_ARG, "shape does not fit on an SM");
     b->shape = s;
     b->shape.blocks_per_sm = (uint32_t)per_sm;
     b->smem = smem;
-    b->threads = (s.chains_per_block + 31u) / 32u * 32u;
+    b->threads = warps * 32u * (b->feed ? 2u : 1u);
     b->grid = (uint32_t)(b->sms * per_sm);
     if (b->graph) {
         cudaGraphExecDestroy(b->graph);
@@ -322,7 +343,7 @@ muca_status sweep_once(muca_batch *b)
 {
     BCUDA(b, launch_batch_prep(b->d_inst, b->n, b->d_counters, b->d_counters + 1, b->stream));
     BCUDA(b, launch_batch_sweep(b->d_inst, b->d_items, b->n_items, b->d_counters, b->shape.chains_per_block,
-                                b->rounds, b->shape.lattice_in_smem, b->shape.hist_in_smem, b->grid, b->smem,
+                                b->rounds, b->shape.lattice_in_smem, b->shape.hist_in_smem, b->feed, b->grid, b->smem,
                                 smem_budget(b), b->stream));
     return MUCA_OK;
 }
@@ -612,7 +633,7 @@ muca_status muca_batch_run(muca_batch *b, const muca_batch_run_opts *o, muca_bat
             e = launch_batch_prep(b->d_inst, b->n, b->d_counters, b->d_counters + 1, b->stream);
             if (e == cudaSuccess)
                 e = launch_batch_sweep(b->d_inst, b->d_items, b->n_items, b->d_counters, b->shape.chains_per_block,
-                                       b->rounds, b->shape.lattice_in_smem, b->shape.hist_in_smem, b->grid, b->smem,
+                                       b->rounds, b->shape.lattice_in_smem, b->shape.hist_in_smem, b->feed, b->grid, b->smem,
                                        smem_budget(b), b->stream);
             if (e == cudaSuccess) e = launch_batch_update(b->d_inst, b->n, b->max_N, rec, b->d_counters + 1, b->stream);
         }

@@ -228,15 +228,17 @@ enum BatchLattice : uint32_t { kLatGlobal = 0, kLatShared = 1, kLatWhereFits = 2
 // shared-memory placement.  grid blocks of roundup32(cpb) threads and
 // `smem` bytes.
 cudaError_t launch_batch_sweep(const BatchInst *insts, const BatchItem *items, uint32_t n_items, uint32_t *next_item,
-                               uint32_t cpb, int rounds, uint32_t lat, bool hist_smem, uint32_t grid, size_t smem,
-                               size_t smem_limit, cudaStream_t s);
+                               uint32_t cpb, int rounds, uint32_t lat, bool hist_smem, bool feed, uint32_t grid,
+                               size_t smem, size_t smem_limit, cudaStream_t s);
+// Shared memory of the drawing warps' rings, behind the rest of a block's.
+size_t batch_feed_smem(uint32_t cpb);
 // Dynamic shared memory of one batch sweep block for an instance of size L,
 // with its lattice, or without it (then optionally with its four-row ring).
 size_t batch_sweep_smem(uint32_t L, uint32_t cpb, bool lat_smem, bool hist_smem, bool row_ring = false);
 // Blocks of the batch sweep that fit on one SM with `smem` bytes each; also
 // sets the kernel's shared-memory limit to `smem` (call before any capture).
 // The launch with that shape needs no further attribute call.
-cudaError_t batch_sweep_occupancy(uint32_t cpb, int rounds, uint32_t lat, bool hist_smem, size_t smem,
+cudaError_t batch_sweep_occupancy(uint32_t cpb, int rounds, uint32_t lat, bool hist_smem, bool feed, size_t smem,
                                   size_t smem_limit, int *blocks);
 // Sets the update kernels' shared-memory and cluster limits (call before any capture).
 cudaError_t prepare_batch_update(uint32_t max_N);

@@ -730,7 +730,8 @@ __device__ __forceinline__ uint32_t *win_prologue(const SweepArgs &a, unsigned c
 // The windowed sweep of chain block `blk` (cpb chains, lanes >= cpb are
 // padding): every lane draws its own Philox numbers one window ahead, so that
 // this work fills the latency of the scan; with FEED another warp draws them
-// (the block has twice as many threads).  Ends with the block synchronised
+// (the block has twice as many threads, the rings of the draws lie at feed_off).
+// Ends with the block synchronised
 // and, with HS, the shared histogram drained.
 // RING (with LAT_SMEM false): the lattice stays in global memory and each
 // lane keeps a four-row ring of its chain in shared memory (RowRing), at the
@@ -747,7 +748,7 @@ template <int MODE, int R, bool LAT_SMEM, bool HS = true, bool BT = false, bool 
           bool ALIGNED = true, bool MANY = false, bool FEED = false>
 __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned char *smem, uint32_t cpb, uint32_t blk,
                                                 uint32_t iter, unsigned long long nup,
-                                                const float *__restrict__ btab = nullptr)
+                                                const float *__restrict__ btab = nullptr, uint32_t feed_off = 0)
 {
     static_assert(!(RING && LAT_SMEM), "the ring serves lattices in global memory");
     static_assert(ALIGNED || !RING, "the ring serves L % 8 == 0");
@@ -783,7 +784,7 @@ __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned cha
     }
     Feed feed;
     if constexpr (FEED) {
-        unsigned char *ring_of = smem + lat_off + align16((size_t)a.L * a.WPR * 4u * cpb) + of_warp * kFeedBytes;
+        unsigned char *ring_of = smem + feed_off + of_warp * kFeedBytes;
         const unsigned long long halves = feed_halves(a.therm, nup);
         if (draws) {
             feed_draw(dr, ring_of, threadIdx.x & 31u, 1u + 4u * of_warp, halves);

@@ -196,3 +196,22 @@ def test_two_batches_share_a_kernel(muca):
         b.run(**opts)
         for i in range(2):
             np.testing.assert_array_equal(b.get_weights(i), alone[i])
+
+
+# one and two warps of chains per block with warps that draw for them, the
+# lattices in shared memory, where they fit, and behind the row ring (L = 128)
+@pytest.mark.gpu
+@pytest.mark.parametrize("insts,shape", [(INSTANCES, (32, 1, 1)), (INSTANCES, (64, 1, 1)),
+                                         (MIXED, (32, 2, 1)), (MIXED, (64, 2, 1))])
+def test_batch_with_drawing_warps_equals_single_simulations(muca, insts, shape):
+    kw = dict(flat_minmean=1, max_iter=10)
+    with muca.Batch(insts, shape=shape) as b:
+        assert b.info().threads == 2 * shape[0]
+        res, _ = b.run(starting_M=1, graph_iters=4, **kw)
+        ws = [b.get_weights(i) for i in range(len(insts))]
+        hs = [b.histogram(i) for i in range(len(insts))]
+    for i, (L, nc, beta, seed) in enumerate(insts):
+        r, w, h = _single(muca, L, nc, seed, **kw)
+        assert (res[i].iterations, res[i].total_run) == (r.iterations, r.total_run), i
+        np.testing.assert_array_equal(ws[i], w, err_msg="instance %d" % i)
+        np.testing.assert_array_equal(hs[i], h, err_msg="instance %d" % i)
