@@ -106,7 +106,7 @@ typedef struct muca_info {
     uint32_t smem_bytes, sms, weights_in_smem;
     uint64_t device_bytes;
     double log_bracket;  /* bound used by the fast acceptance test: twice the measured
-                            max |__logf(u) - logf(u)| over all u01fixedpt<float> values */
+                            max |fast log(u) - logf(u)| over all u01fixedpt<float> values */
     uint32_t kernel;      /* sweep kernel in use (see muca_params.kernel) */
     uint32_t threads_per_block;
 } muca_info;

@@ -3,13 +3,13 @@
 // Many (L, beta) instances of uneven size advance one weight iteration
 // together: a prep kernel clears the histograms of the instances still
 // running, one persistent sweep kernel works through the list of chain
-// blocks of all instances, and one update block per instance applies the
+// blocks of all instances, and a cluster of blocks per instance applies the
 // statistics, the schedule and the weight update (k_weights.cu).  The three
 // launches of an iteration are captured into a CUDA graph by the host
 // (muca_batch.cu) and replayed.
 //
 // The sweep of a chain block is the single-simulation windowed sweep
-// (sweep_core.cuh) with two differences: the Metropolis term -beta*dE comes
+// (window.cuh) with two differences: the Metropolis term -beta*dE comes
 // from the instance's table (exactly -2 dE for the reference's beta = 2), and
 // the histogram may go straight to the u64 device histogram, which frees the
 // shared memory of the u32 bins for more blocks per SM.  Work is fetched by

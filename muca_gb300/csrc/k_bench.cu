@@ -59,7 +59,7 @@ cudaError_t launch_philox_peak(int rounds, uint32_t grid, uint32_t blocks_per_th
 }
 
 constexpr uint32_t kFloorL = 72, kFloorWPR = 5, kFloorCpb = 128, kFloorN = kFloorL * kFloorL;
-constexpr float kFloorEps = 3.5e-6f;  // twice max |__logf(u) - logf(u)| measured on GB300
+constexpr float kFloorEps = 3.5e-6f;  // twice max |fast_logf(u) - logf(u)| measured on GB300
 
 __device__ __forceinline__ uint32_t floor_hash(uint32_t x)
 {

@@ -10,31 +10,31 @@
 //   diff = (float)(-2 dE) + w[E + dDel] - w[E]        (:810)
 // evaluated without contraction, and the same test diff >= 0 || logf(u) < diff.
 //
-// GB300 layout (windowed kernels, L % 8 == 0):
-//   * the lattice lives in shared memory, 2 bits per spin, rows padded to
-//     16-site words, [word][lane] so the lanes of a warp hit distinct banks;
-//   * the weights (FP32 or FP64) and, in weight mode, a u32 histogram live in
-//     shared memory; the histogram is drained to the u64 device histogram
-//     once per launch (the reference does one global atomic per attempt);
-//   * the sweep is processed in windows of the 8 (or 4) same-parity sites of
-//     one word of one row.  Sites of a window are never neighbours of each
-//     other (their neighbours are the other parity or the rows above/below),
-//     so the whole window's proposals and energy changes are formed from four
-//     word loads with nibble-parallel (SWAR) arithmetic; only the
-//     accept/reject scan over E_Delta is sequential.  The window's new spins
-//     are merged into one word store;
-//   * the acceptance test uses the hardware __logf(u) and falls back to the
-//     exact logf(u) (replaying the window) whenever __logf(u) lies within the
-//     measured worst-case difference of the two functions from diff in any
-//     lane, so every decision equals the reference's logf decision.
+// GB300 layout:
+//   * a lattice takes 2 bits per spin, rows padded to 16-site words, [word][lane]
+//     so the lanes of a warp hit distinct banks; it lives in shared memory, or in
+//     global memory behind a ring of rows;
+//   * the weights (FP32; of FP64 ones their differences) and, in weight mode, a
+//     u32 histogram live in shared memory; the histogram is drained to the u64
+//     device histogram once per launch (the reference does one global atomic per
+//     attempt);
+//   * the sweep is processed in windows of up to 8 same-parity sites of one word
+//     of one row.  Sites of a window are never neighbours of each other (their
+//     neighbours are the other parity or the rows above/below), so the whole
+//     window's proposals and energy changes are formed from four word loads with
+//     nibble-parallel arithmetic; only the accept/reject scan over E_Delta is
+//     sequential.  The window's new spins are merged into one word store;
+//   * the acceptance test uses a fast logarithm and replays the window with the
+//     exact logf(u) whenever the fast one lies within the measured worst-case
+//     difference of the two from deciding otherwise in any lane, so every
+//     decision equals the reference's logf decision.
 // Kernels:
-//   k_sweep_spec  warp-specialised: per 32 chains one producer warp draws the
-//                 Philox numbers and decodes each window into a 2-deep
-//                 shared-memory ring guarded by mbarriers, and one consumer
-//                 warp runs the scan, write-back and histogram; two
-//                 independent instruction streams per 32 chains;
-//   k_sweep_win   the same window core with the Philox numbers drawn by the
-//                 chain's own lane, one window ahead;
+//   k_sweep_win   (k_sweep_win.cuh, window.cuh) every even L >= 8: the numbers
+//                 are drawn by the chain's own lane, one window ahead, or, where
+//                 SM sub-partitions would be idle, by another warp;
+//   k_sweep_spec  only on request, L % 8 == 0: per 32 chains one producer warp
+//                 draws and decodes each window into a shared-memory ring
+//                 guarded by mbarriers, and one consumer warp runs the scan;
 //   k_sweep_generic  the reference step by step on the packed layout, any L.
 #include "window.cuh"
 
@@ -92,7 +92,7 @@ enum SlotWord : uint32_t {
     kSlotDV = 3,    // s_new - s_old + 2 (nibbles; production only)
     kSlotDE = 4,    // dE as signed bytes, sites 0..3 and 4..7 (two words)
     kSlotF2 = 6,    // -beta dE as floats (8 words)
-    kSlotLF = 14,   // __logf(u) (8 words)
+    kSlotLF = 14,   // fast_logf(u) (8 words)
     kSlotP = 22,    // acceptance words for the exact replay, or packed draws of a partial window (8 words)
 };
 static_assert(kSlotP + 8 == kSlotWords, "slot layout");
@@ -150,7 +150,7 @@ __device__ __forceinline__ void get_window(const uint32_t *slot, uint32_t *pc, u
 
 // Per 32 chains one producer warp and one consumer warp.  The producer draws
 // the Philox numbers and decodes each window (proposals, dE, dDelta,
-// __logf(u)) into a ring slot; the consumer runs the scan, the lattice
+// fast_logf(u)) into a ring slot; the consumer runs the scan, the lattice
 // store and the histogram.  Decoding window (row, q) reads the same-parity
 // word of row - 1, written by the consumer WPR windows earlier, so the ring
 // is at most WPR deep; at the start of a half (and of a phase) the producer
@@ -232,11 +232,11 @@ __global__ void __launch_bounds__(256, 1) k_sweep_spec(const SweepArgs a, uint32
                 for (int t = 0; t < 8; ++t) slot[32 * (kSlotP + t)] = pack_draw(r1[t], r3[t]);
             } else if (cnt == 8) {
                 WinDec<MODE> d;
-                decode_window<MODE, 8>(lat, cpb, L, WPR, row, q, half, r1, r3, nullptr, d);
+                decode_window<MODE, 8>(lat, cpb, L, WPR, row, q, half, r1, r3, d);
                 put_window<MODE, 8>(d, slot);
             } else {
                 WinDec<MODE> d;
-                decode_window<MODE, 4>(lat, cpb, L, WPR, row, q, half, r1, r3, nullptr, d);
+                decode_window<MODE, 4>(lat, cpb, L, WPR, row, q, half, r1, r3, d);
                 put_window<MODE, 4>(d, slot);
             }
             if (!silent) mbar_arrive(full + s);
@@ -267,11 +267,11 @@ __global__ void __launch_bounds__(256, 1) k_sweep_spec(const SweepArgs a, uint32
             } else if (cnt == 8) {
                 WinDec<MODE> d;
                 get_window<MODE, 8>(slot, pc, half, d);
-                scan_window<MODE, 8, true>(d, rec, store, checked, wS, histS, a.hist, st, eps, wG, tol);
+                scan_window<MODE, 8>(d, rec, store, checked, wS, histS, a.hist, st, eps, wG, tol);
             } else {
                 WinDec<MODE> d;
                 get_window<MODE, 4>(slot, pc, half, d);
-                scan_window<MODE, 4, true>(d, rec, store, checked, wS, histS, a.hist, st, eps, wG, tol);
+                scan_window<MODE, 4>(d, rec, store, checked, wS, histS, a.hist, st, eps, wG, tol);
             }
             mbar_arrive(empty + s);  // after the store: the producer may read the word
             ++w;
@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(256) k_sweep_generic(const SweepArgs a, uint32
 }
 
 // ---------------------------------------------------------------------------
-// Worst-case |__logf(u) - logf(u)| over every value u01fixedpt<float> can
+// Worst-case |fast_logf(u) - logf(u)| over every value u01fixedpt<float> can
 // return (u = (2k+1) 2^-24, k < 2^23), as the bits of a non-negative float.
 __global__ void k_logf_bracket(unsigned int *maxbits)
 {

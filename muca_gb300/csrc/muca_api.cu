@@ -48,7 +48,7 @@ struct muca_ctx {
     unsigned int *d_err = nullptr, *h_err = nullptr;
     uint64_t device_bytes = 0;
     double log_eps = 0, log_eps_measured = 0;
-    double log_eps_table = 1e30;  // host_logf: twice max |__logf(u) - the host table's log(u)|
+    double log_eps_table = 1e30;  // host_logf: twice max |fast_logf(u) - the host table's log(u)|
     uint32_t algo = 0;
     float *d_logf_tab = nullptr;  // random-site algorithm with host_logf: the host libm's logf
     RecScratch rec{};             // the multi-block recursion's dS_i and pair flags (weight mode)

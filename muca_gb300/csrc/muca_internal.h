@@ -24,7 +24,7 @@ struct SweepArgs {
     uint32_t seed_base, seed_dev_mul, iter;
     unsigned long long therm, nup;
     uint32_t k1_mul, k1_add, k1_hi, k3_mul, k3_add, k3_hi;
-    // bound on |__logf(u) - logf(u)| over all u01fixedpt<float> values
+    // bound on |fast_logf(u) - logf(u)| over all u01fixedpt<float> values
     // (measure_logf_bracket) times a safety factor; 0 disables the fast test
     double log_eps;
     // optional device-resident (iter, nup, skip) for graph-captured loops;
@@ -78,7 +78,7 @@ constexpr uint32_t kSlotWords = 30;
 // `smem_optin` bytes of opt-in shared memory per block and `sms` SMs.
 // kernel: -1 = choose (windowed when L is even and at least 8, else generic), else a SweepKernel.
 SweepPlan plan_sweep(int mode, int rounds, uint32_t L, uint32_t nchains, size_t smem_optin, int sms, int kernel = -1);
-// Worst case of |__logf(u) - logf(u)| over u = (2k+1) 2^-24, k < 2^23 (exhaustive, on the device).
+// Worst case of |fast_logf(u) - logf(u)| over u = (2k+1) 2^-24, k < 2^23 (exhaustive, on the device).
 cudaError_t measure_logf_bracket(float *max_abs_err, cudaStream_t s);
 // The bound of the fast acceptance test for `device` (current): twice the
 // measured worst case, measured once per device and cached; 1e30 (every
@@ -101,11 +101,11 @@ struct RandomArgs {
     unsigned long long therm, nup;
     const float *logf_tab;
     const uint32_t *dyn;  // as SweepArgs::dyn
-    // bound on |__logf(u) - log(u)| over every u01fixedpt<float> value, log
+    // bound on |fast_logf(u) - log(u)| over every u01fixedpt<float> value, log
     // being logf_tab's values (when given) or CUDA's logf, with a safety factor
     double log_eps;
 };
-// Worst case of |__logf(u) - tab[k]| over u = (2k+1) 2^-24, k < 2^23 (exhaustive, on the device).
+// Worst case of |fast_logf(u) - tab[k]| over u = (2k+1) 2^-24, k < 2^23 (exhaustive, on the device).
 cudaError_t measure_table_bracket(const float *tab, float *max_abs_err, cudaStream_t s);
 size_t random_sweep_smem(uint32_t L, uint32_t cpb, bool lat_smem);
 // Block shape of the random-site sweep for (L, nchains) on a device with

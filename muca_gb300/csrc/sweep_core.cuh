@@ -1,8 +1,8 @@
-// sweep_core.cuh -- the per-chain Metropolis machinery shared by the sweep
-// kernels of one simulation (k_sweep.cu) and of a batch of simulations
-// (k_batch.cu): shared-memory layout, Philox draws, the windowed SWAR step,
-// the step-by-step partial window, histogram recording and the walk over the
-// reference's sweep order.  See k_sweep.cu for the design.
+// sweep_core.cuh -- the per-chain Metropolis machinery of the sweep kernels:
+// shared-memory layout, the row ring and histogram flushes that all share, and
+// the window of the warp-specialised kernel with its step-by-step remainder,
+// histogram recording and walk over the reference's sweep order.  (The lean
+// window of the other windowed kernels is in window.cuh.)
 #pragma once
 #include "muca_device.cuh"
 #include "muca_internal.h"
@@ -60,12 +60,10 @@ __device__ __forceinline__ void draw_pair(uint32_t cc, uint32_t seed, uint32_t i
 
 // Histogram entry.  The u32 shared bins are drained into the u64 device
 // histogram by the lane whose increment finds 2^31 counts already there.
-template <int MODE, bool HS = true>
+template <int MODE>
 __device__ __forceinline__ void record(uint32_t *histS, unsigned long long *histG, int E, int M)
 {
-    if (MODE == kModeWeight && !HS) {
-        atomicAdd(&histG[E], 1ull);
-    } else if (MODE == kModeWeight) {
+    if (MODE == kModeWeight) {
         const uint32_t old = atomicAdd(&histS[E], 1u);
         if (old >= 0x80000000u) {
             const uint32_t v = atomicExch(&histS[E], 0u);
@@ -76,32 +74,18 @@ __device__ __forceinline__ void record(uint32_t *histS, unsigned long long *hist
     }
 }
 
-// Histogram entries of one window.  Weight mode with the shared u32
-// histogram: one shared atomic per attempt; `checked` (uniform: the launch
-// can put 2^32 entries into one block's bins) drains a u32 shared bin into
-// the u64 device histogram once it holds 2^31 (the warp-specialised sweep;
-// the windowed sweep flushes all bins between rows instead, flush_hist).
-// Device (u64) histograms: the entries are merged into runs of equal bins
-// per lane first (E_Delta moves by at most one per attempt, so a window's
-// entries cluster), which saves global atomics; HS = false (weight mode)
-// sends the runs straight to the u64 device histogram.
-template <int MODE, int SLOTS, bool HS = true>
+// Histogram entries of one window.  Weight mode: one shared atomic per
+// attempt; `checked` (uniform: the launch can put 2^32 entries into one
+// block's bins) drains a u32 shared bin into the u64 device histogram once it
+// holds 2^31 (the warp-specialised sweep; the windowed sweep flushes all bins
+// between rows instead, flush_hist).  Production: the entries are merged into
+// runs of equal bins per lane first, which saves global atomics.
+template <int MODE, int SLOTS>
 __device__ __forceinline__ void record_window(uint32_t *__restrict__ histS, unsigned long long *__restrict__ histG,
                                               const int (&Es)[SLOTS], const int (&Ms)[SLOTS], bool checked)
 {
     // run lengths are at most SLOTS: 32-bit counts, widened at the atomics
-    if (MODE == kModeWeight && !HS) {
-        int cur = Es[0];
-        uint32_t cnt = 1;
-#pragma unroll
-        for (int t = 1; t < SLOTS; ++t) {
-            const bool same = Es[t] == cur;
-            if (!same) atomicAdd(&histG[cur], (unsigned long long)cnt);
-            cnt = same ? cnt + 1u : 1u;
-            cur = Es[t];
-        }
-        atomicAdd(&histG[cur], (unsigned long long)cnt);
-    } else if (MODE == kModeWeight) {
+    if (MODE == kModeWeight) {
         if (checked) {
 #pragma unroll
             for (int t = 0; t < SLOTS; ++t) {
@@ -138,7 +122,7 @@ struct WinDec {
     uint32_t C, ctr, vnib, hs0;  // the word, old and proposed codes (nibbles), parity shift
     int dE[8], dDel[8], dM[8];
     float f2[8];                // -beta dE (an even integer for beta = 2: exact in FP32 and FP64)
-    float lf[8];                // __logf(u)
+    float lf[8];                // fast_logf(u)
     uint32_t p[8];              // the acceptance words (for the exact replay; bits 31..9 used)
     const uint32_t *pr;         // or, when set, those words in shared memory (pr[32 t])
 };
@@ -149,32 +133,24 @@ struct WinDec {
 // lat points at this lane's word 0 (stride cpb).  The half is a value, not a
 // template branch, so decode and scan of neighbouring windows form one basic
 // block the compiler can interleave.
-// BT: -beta*dE comes from the table btab[dE + 8] (any beta) instead of the
-// reference's literal -2 dE (beta = 2); the table holds (float)(-beta*dE),
-// which for beta = 2 is the same value.
-// rmask: rows are addressed as (row & rmask): ~0u for a whole lattice,
-// 3 for the four-row ring of RowRing (L is a multiple of 4, so the ring's
-// slots follow the periodic rows).
-template <int MODE, int SLOTS, bool BT = false>
+template <int MODE, int SLOTS>
 __device__ __forceinline__ void decode_window(uint32_t *__restrict__ lat, uint32_t cpb, uint32_t L, uint32_t WPR,
                                               uint32_t row, uint32_t q, uint32_t half, const uint32_t *r1,
-                                              const uint32_t *r3, const float *__restrict__ btab, WinDec<MODE> &d,
-                                              uint32_t rmask = ~0u)
+                                              const uint32_t *r3, WinDec<MODE> &d)
 {
     using WT = typename WeightType<MODE>::T;
     constexpr uint32_t M2 = 0x33333333u, N1 = 0x11111111u;
     const uint32_t rup = (row + 1 == L) ? 0u : row + 1;
     const uint32_t rdn = (row == 0) ? L - 1 : row - 1;
-    const uint32_t rw = row & rmask;
-    d.pc = lat + (size_t)(rw * WPR + q) * cpb;
+    d.pc = lat + (size_t)(row * WPR + q) * cpb;
     const uint32_t C = *d.pc;
-    const uint32_t U = lat[(size_t)((rup & rmask) * WPR + q) * cpb];
-    const uint32_t D = lat[(size_t)((rdn & rmask) * WPR + q) * cpb];
+    const uint32_t U = lat[(size_t)(rup * WPR + q) * cpb];
+    const uint32_t D = lat[(size_t)(rdn * WPR + q) * cpb];
     // the one neighbour outside word q: left of the first even site, or
     // right of the last odd site (wrapping along the row)
     const uint32_t sq = half ? ((16 * q + 16 < L) ? q + 1 : 0u) : (q ? q - 1 : (L - 1) >> 4);
     const uint32_t sb = half ? 0u : (q ? 15u : ((L - 1) & 15u));
-    const uint32_t sv = spin_code(lat[(size_t)(rw * WPR + sq) * cpb], sb);
+    const uint32_t sv = spin_code(lat[(size_t)(row * WPR + sq) * cpb], sb);
 
     // Nibble t of `ctr` holds the spin code (s+1) of the window's site t;
     // nibble t of `nbs` the sum of its four neighbours' codes (0..8, no
@@ -210,24 +186,18 @@ __device__ __forceinline__ void decode_window(uint32_t *__restrict__ lat, uint32
         d.dDel[t] = (int)((ddb >> (4 * t)) & 3u) - 1;
         d.dE[t] = dv * (4 - (int)((nbs >> (4 * t)) & 15u));  // -(s_new - s_old) * (sum of neighbour spins)
         d.dM[t] = dv;
-        if (BT) d.f2[t] = btab[d.dE[t] + 8];
-        else    d.f2[t] = small_int_to_float(-2 * d.dE[t]);
+        d.f2[t] = small_int_to_float(-2 * d.dE[t]);
         d.lf[t] = fast_logf(u01f(r1[t]));
         d.p[t] = r1[t];
     }
 }
 
 // The accept/reject scan of a decoded window, its lattice write and its
-// histogram entries.  ONEBAND (weight mode): decide each attempt with the
-// one-band test of the production scan instead of the two tests.  AHEAD2
-// (weight mode): fetch each attempt's weight three attempts ahead, for the
-// four outcomes of the two decisions between, instead of one attempt ahead
-// for two outcomes.  Both forms decide every attempt identically; which is
-// faster depends on the kernel around the scan (measured per kernel).
+// histogram entries.
 // `store` is false for padding lanes: they read another lane's spins, never
 // accept (so their E stays at 3 and every weight index E + dDel_t + dDel_t+1
 // + dDel_t+2 stays in [0, 6]) and never write.
-template <int MODE, int SLOTS, bool HS = true, bool ONEBAND = false, bool AHEAD2 = false>
+template <int MODE, int SLOTS>
 __device__ __forceinline__ void scan_window(const WinDec<MODE> &d, bool rec, bool store, bool checked,
                                             const typename WeightType<MODE>::T *__restrict__ wS,
                                             uint32_t *__restrict__ histS, unsigned long long *__restrict__ histG,
@@ -260,8 +230,8 @@ __device__ __forceinline__ void scan_window(const WinDec<MODE> &d, bool rec, boo
             // logf(u) < 0 for every u = (1|(r>>8)) 2^-24 <= 1 - 2^-24, so the
             // reference's  diff >= 0 || logf(u) < diff  is  logf(u) < diff.
             // With |fast - diff| <= tol (any dDel, a zero difference
-            // included) and |__logf(u) - logf(u)| <= eps, the sign of
-            // g = __logf(u) - fast is that of logf(u) - diff whenever
+            // included) and |fast_logf(u) - logf(u)| <= eps, the sign of
+            // g = fast_logf(u) - fast is that of logf(u) - diff whenever
             // |g| > tol + eps; otherwise the window is replayed.
             const float g = __fsub_rn(d.lf[t], fast);
             const bool acc = store && (g < 0.0f);
@@ -298,13 +268,13 @@ __device__ __forceinline__ void scan_window(const WinDec<MODE> &d, bool rec, boo
         }
         const uint32_t merged = (d.ctr & ~accm) | (d.vnib & accm);
         if (store) *d.pc = (d.C & (d.hs0 ? M2 : ~M2)) | (merged << d.hs0);
-        if (rec) record_window<MODE, SLOTS, HS>(histS, histG, Es, Ms, checked);
+        if (rec) record_window<MODE, SLOTS>(histS, histG, Es, Ms, checked);
         return;
     }
     // Sequential accept/reject over E_Delta:
     //   accept  <=>  diff >= 0  ||  logf(u) < diff,
     //   diff = (float)(-2 dE) + w[E + dDel] - w[E]   (muca_delta_multigpu.cu:810-816)
-    // decided with __logf(u) unless it lies within eps of diff in some lane;
+    // decided with fast_logf(u) unless it lies within eps of diff in some lane;
     // then the window is replayed with the exact logf(u).  The weight of the
     // next attempt is fetched one attempt ahead for both outcomes (c0: this
     // attempt rejected, c1: accepted), so no shared-memory load sits on the
@@ -315,110 +285,36 @@ __device__ __forceinline__ void scan_window(const WinDec<MODE> &d, bool rec, boo
     uint32_t accm = 0;
     bool near = false;
     int Es[SLOTS], Ms[SLOTS];
-    if constexpr (AHEAD2) {
-        // P[u][2a + b]: the weight at attempt u's proposed E_Delta when the
-        // attempts u-2 and u-1 decide a and b, loaded after attempt u-3
-        WT P[SLOTS][4];
-        bool av[SLOTS];
-        P[0][0] = wS[st.E + d.dDel[0]];
-        if (SLOTS > 1) {
-            P[1][0] = wS[st.E + d.dDel[1]];
-            P[1][1] = wS[st.E + d.dDel[0] + d.dDel[1]];
-        }
-        if (SLOTS > 2) {
-            P[2][0] = wS[st.E + d.dDel[2]];
-            P[2][1] = wS[st.E + d.dDel[1] + d.dDel[2]];
-            P[2][2] = wS[st.E + d.dDel[0] + d.dDel[2]];
-            P[2][3] = wS[st.E + d.dDel[0] + d.dDel[1] + d.dDel[2]];
-        }
+    WT A = wS[st.E + d.dDel[0]];
+    WT c0 = A, c1 = A;
+    if (SLOTS > 1) {
+        c0 = wS[st.E + d.dDel[1]];
+        c1 = wS[st.E + d.dDel[0] + d.dDel[1]];
+    }
 #pragma unroll
-        for (int t = 0; t < SLOTS; ++t) {
-            WT A;
-            if (t == 0) {
-                A = P[0][0];
-            } else if (t == 1) {
-                A = av[0] ? P[1][1] : P[1][0];
-            } else {
-                const WT q0 = av[t - 2] ? P[t][2] : P[t][0];
-                const WT q1 = av[t - 2] ? P[t][3] : P[t][1];
-                A = av[t - 1] ? q1 : q0;
-            }
-            WT diff;
-            if (MODE == kModeWeight)
-                diff = __fsub_rn(__fadd_rn((float)d.f2[t], (float)A), (float)wE);
-            else
-                diff = __dsub_rn(__dadd_rn((double)d.f2[t], (double)A), (double)wE);
-            const WT l = (WT)d.lf[t];
-            bool acc;
-            if (ONEBAND) {
-                const WT g = l - diff;
-                acc = store && (g < (WT)0);
-                near |= fabs(g) <= eps;
-            } else {
-                acc = store && ((diff >= (WT)0) || (l < diff));
-                near |= (diff < (WT)0) && (fabs(l - diff) <= eps);
-            }
-            av[t] = acc;
-            if (acc) {
-                st.E += d.dDel[t];
-                st.EJ += d.dE[t];
-                st.M += d.dM[t];
-                wE = A;
-                accm |= 0xFu << (4 * t);
-            }
-            Es[t] = st.E;
-            Ms[t] = st.M;
-            if (t + 3 < SLOTS) {
-                const int e = st.E + d.dDel[t + 3];
-                P[t + 3][0] = wS[e];
-                P[t + 3][1] = wS[e + d.dDel[t + 2]];
-                P[t + 3][2] = wS[e + d.dDel[t + 1]];
-                P[t + 3][3] = wS[e + d.dDel[t + 1] + d.dDel[t + 2]];
-            }
+    for (int t = 0; t < SLOTS; ++t) {
+        WT diff;
+        if (MODE == kModeWeight)
+            diff = __fsub_rn(__fadd_rn((float)d.f2[t], (float)A), (float)wE);
+        else
+            diff = __dsub_rn(__dadd_rn((double)d.f2[t], (double)A), (double)wE);
+        const WT l = (WT)d.lf[t];
+        const bool acc = store && ((diff >= (WT)0) || (l < diff));
+        near |= (diff < (WT)0) && (fabs(l - diff) <= eps);
+        if (acc) {
+            st.E += d.dDel[t];
+            st.EJ += d.dE[t];
+            st.M += d.dM[t];
+            wE = A;
+            accm |= 0xFu << (4 * t);
         }
-    } else {
-        WT A = wS[st.E + d.dDel[0]];
-        WT c0 = A, c1 = A;
-        if (SLOTS > 1) {
-            c0 = wS[st.E + d.dDel[1]];
-            c1 = wS[st.E + d.dDel[0] + d.dDel[1]];
-        }
-#pragma unroll
-        for (int t = 0; t < SLOTS; ++t) {
-            WT diff;
-            if (MODE == kModeWeight)
-                diff = __fsub_rn(__fadd_rn((float)d.f2[t], (float)A), (float)wE);
-            else
-                diff = __dsub_rn(__dadd_rn((double)d.f2[t], (double)A), (double)wE);
-            const WT l = (WT)d.lf[t];
-            bool acc;
-            if (ONEBAND) {
-                // logf(u) < 0 for every u <= 1 - 2^-24, so  diff >= 0 || logf(u) < diff
-                // is  logf(u) < diff;  g = __logf(u) - diff has its sign unless |g| <= eps
-                const WT g = l - diff;
-                acc = store && (g < (WT)0);
-                near |= fabs(g) <= eps;
-            } else {
-                // two tests: the one-band form measured 11 % slower in the
-                // single-instance kernel (and 1 % faster in the batch kernel)
-                acc = store && ((diff >= (WT)0) || (l < diff));
-                near |= (diff < (WT)0) && (fabs(l - diff) <= eps);
-            }
-            if (acc) {
-                st.E += d.dDel[t];
-                st.EJ += d.dE[t];
-                st.M += d.dM[t];
-                wE = A;
-                accm |= 0xFu << (4 * t);
-            }
-            Es[t] = st.E;
-            Ms[t] = st.M;
-            if (t + 1 < SLOTS) {
-                A = acc ? c1 : c0;
-                if (t + 2 < SLOTS) {
-                    c0 = wS[st.E + d.dDel[t + 2]];
-                    c1 = wS[st.E + d.dDel[t + 1] + d.dDel[t + 2]];
-                }
+        Es[t] = st.E;
+        Ms[t] = st.M;
+        if (t + 1 < SLOTS) {
+            A = acc ? c1 : c0;
+            if (t + 2 < SLOTS) {
+                c0 = wS[st.E + d.dDel[t + 2]];
+                c1 = wS[st.E + d.dDel[t + 1] + d.dDel[t + 2]];
             }
         }
     }
@@ -450,56 +346,34 @@ __device__ __forceinline__ void scan_window(const WinDec<MODE> &d, bool rec, boo
     }
     const uint32_t merged = (d.ctr & ~accm) | (d.vnib & accm);
     if (store) *d.pc = (d.C & (d.hs0 ? M2 : ~M2)) | (merged << d.hs0);
-    if (rec) record_window<MODE, SLOTS, HS>(histS, histG, Es, Ms, checked);
-}
-
-// One full window: decode, then scan.
-template <int MODE, int SLOTS, int HALF, bool HS = true, bool BT = false, bool AHEAD2 = false>
-__device__ __forceinline__ void window_core(uint32_t *__restrict__ lat, uint32_t cpb, uint32_t L, uint32_t WPR,
-                                            uint32_t row, uint32_t q, bool rec, bool store, bool checked,
-                                            const typename WeightType<MODE>::T *__restrict__ wS,
-                                            uint32_t *__restrict__ histS, unsigned long long *__restrict__ histG,
-                                            ChainState &st, const uint32_t (&r1)[SLOTS], const uint32_t (&r3)[SLOTS],
-                                            typename WeightType<MODE>::T eps, const float *__restrict__ btab = nullptr,
-                                            uint32_t hrt = 0, const double *__restrict__ wG = nullptr,
-                                            float tol = 0.0f, uint32_t rmask = ~0u)
-{
-    WinDec<MODE> d;
-    decode_window<MODE, SLOTS, BT>(lat, cpb, L, WPR, row, q, HALF < 0 ? hrt : (uint32_t)HALF, r1, r3, btab, d,
-                                   rmask);
-    // the batch kernel (the one user of the beta table) and the scan with
-    // weights fetched three attempts ahead decide weight-mode attempts with
-    // the one-band test
-    scan_window<MODE, SLOTS, HS, BT || AHEAD2, AHEAD2>(d, rec, store, checked, wS, histS, histG, st, eps, wG, tol);
+    if (rec) record_window<MODE, SLOTS>(histS, histG, Es, Ms, checked);
 }
 
 // The first `len` (< window size) attempts of a window, one at a time as
 // the reference writes them; only the last window of a phase is partial.
-template <int MODE, bool HS = true, bool BT = false>
+template <int MODE>
 __device__ __noinline__ void partial_core(uint32_t *__restrict__ lat, uint32_t cpb, uint32_t L, uint32_t WPR,
                                           uint32_t row, uint32_t q, uint32_t half, uint32_t len, bool rec,
                                           bool store, const typename WeightType<MODE>::T *__restrict__ wS,
                                           uint32_t *__restrict__ histS, unsigned long long *__restrict__ histG,
-                                          ChainState &st, const uint32_t *p, const float *__restrict__ btab = nullptr,
-                                          uint32_t rmask = ~0u)
+                                          ChainState &st, const uint32_t *p)
 {
     using WT = typename WeightType<MODE>::T;
-    const uint32_t rup = ((row + 1 == L) ? 0u : row + 1) & rmask;
-    const uint32_t rdn = ((row == 0) ? L - 1 : row - 1) & rmask;
-    const uint32_t rw = row & rmask;
+    const uint32_t rup = (row + 1 == L) ? 0u : row + 1;
+    const uint32_t rdn = (row == 0) ? L - 1 : row - 1;
     for (uint32_t t = 0; t < len; ++t) {
         const uint32_t col = 16u * q + 2u * t + half;
         const uint32_t cl = col ? col - 1 : L - 1, cr = (col + 1 == L) ? 0u : col + 1;
-        uint32_t *pw = lat + (size_t)(rw * WPR + (col >> 4)) * cpb;
+        uint32_t *pw = lat + (size_t)(row * WPR + (col >> 4)) * cpb;
         const int os = (int)spin_code(*pw, col) - 1;
         int ns = os + ((p[t] & 1u) ? -1 : 1);
         ns = ns - 3 * (ns == 2) + 3 * (ns == -2);
-        const int nb = (int)spin_code(lat[(size_t)(rw * WPR + (cl >> 4)) * cpb], cl) +
-                       (int)spin_code(lat[(size_t)(rw * WPR + (cr >> 4)) * cpb], cr) +
+        const int nb = (int)spin_code(lat[(size_t)(row * WPR + (cl >> 4)) * cpb], cl) +
+                       (int)spin_code(lat[(size_t)(row * WPR + (cr >> 4)) * cpb], cr) +
                        (int)spin_code(lat[(size_t)(rup * WPR + (col >> 4)) * cpb], col) +
                        (int)spin_code(lat[(size_t)(rdn * WPR + (col >> 4)) * cpb], col) - 4;
         const int dE = -(ns - os) * nb, dDel = ns * ns - os * os, dM = ns - os;
-        const WT f2 = BT ? (WT)btab[dE + 8] : (WT)(-2 * dE);
+        const WT f2 = (WT)(-2 * dE);
         WT diff;
         if (MODE == kModeWeight)
             diff = __fsub_rn(__fadd_rn((float)f2, (float)wS[st.E + dDel]), (float)wS[st.E]);
@@ -514,7 +388,7 @@ __device__ __noinline__ void partial_core(uint32_t *__restrict__ lat, uint32_t c
             st.EJ += dE;
             st.M += dM;
         }
-        if (rec) record<MODE, HS>(histS, histG, st.E, st.M);
+        if (rec) record<MODE>(histS, histG, st.E, st.M);
     }
 }
 
