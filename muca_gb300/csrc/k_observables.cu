@@ -10,8 +10,8 @@
 //
 // The sums stream the u64 histogram once (HBM bound at 8 B per bin), one
 // warp per row, with exact integer moments per row (see row_moments);
-// the per-row FP64 terms are combined per warp, per block and then in a
-// fixed-order second pass, so the result is deterministic and agrees with
+// the per-row FP64 terms are combined per block and then in a fixed-order
+// second pass, so the result is deterministic and agrees with
 // the long-double host sum to ~1e-15.
 #include "muca_device.cuh"
 #include "muca_internal.h"

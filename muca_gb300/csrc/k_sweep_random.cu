@@ -37,7 +37,7 @@
 //     the float 2^23 + entry;
 //   * lattice columns in shared memory lie a multiple of 32 lanes apart where
 //     that fits, so that lanes at different sites meet no bank conflict.
-// L = 72, 16384 chains, 85 M attempts: 0.56 ms (205 cycles an attempt and
+// L = 72, 16384 chains, 85 M attempts: 0.56 ms (224 cycles an attempt and
 // warp); 0.68 with the addresses too kept from one group to the next (a move for
 // each), selects instead of predicated additions and stores, and a group's
 // length tested in its loop; 0.79 with tables of a row's and a column's

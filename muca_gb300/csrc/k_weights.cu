@@ -4,8 +4,9 @@
 // program (muca_delta_multigpu.cu:422-476): hist_range (:573-596), the
 // Kullback-Leibler divergence against a uniform distribution over visited
 // bins (:598-618), the trivial update lnW -= ln H for H > 1 followed by
-// lnW -= lnW[0] (:466-476), and weight_recursion (:833-859).  One block
-// serves one histogram of N+1 <= 16385 bins.  Element-wise steps use the
+// lnW -= lnW[0] (:466-476), and weight_recursion (:833-859).  One cluster,
+// a few launches or one block serve one histogram of N+1 <= 16385 bins (see
+// launch_weight_update and the batch's update).  Element-wise steps use the
 // reference's operation order with explicitly rounded FP64 operations, so
 // the updated weights equal the host's up to the last-bit differences of the
 // device and host log(); the divergence is a tree sum and agrees to ~1e-15.
