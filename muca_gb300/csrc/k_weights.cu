@@ -209,6 +209,9 @@ __host__ __device__ __forceinline__ uint32_t next_nupdates(uint32_t nup, bool fu
     return (uint32_t)nx;
 }
 
+// Whether an update clears the histogram for the run's next iteration.
+__device__ __forceinline__ bool clears_hist(const RunCtl *ctl) { return ctl && !ctl->st.stop && !ctl->keep_hist; }
+
 // The statistics' consumers, one thread: the stats record, and in a
 // device-driven run the running width, convergence, record and NUPDATES of
 // the next iteration (muca_delta_multigpu.cu:431-447,464-466).  Returns
@@ -282,8 +285,8 @@ __device__ __forceinline__ unsigned char recursion_increment(const unsigned long
 }
 
 // `dyn`: dynamic shared memory of update_smem(N, rule) bytes.
-// clear: in a device-driven run, zero the histogram for the next iteration
-// unless this was the last.
+// CLEAR: in a device-driven run, zero the histogram for the next iteration
+// (clears_hist).
 template <bool CLEAR = false>
 __device__ __forceinline__ void weight_update_body(unsigned long long *__restrict__ hist, uint32_t N,
                                                    double *__restrict__ lnw, float *__restrict__ w32,
@@ -322,7 +325,7 @@ __device__ __forceinline__ void weight_update_body(unsigned long long *__restric
     kl = block_reduce(kl, AddD(), shd);
     if (tid == 0) {
         const int upd = bookkeep(start, end, vis, ev, mn, kl, N, rule, stats, ctl);
-        do_update = upd | (CLEAR && ctl && !ctl->st.stop ? 2 : 0);
+        do_update = upd | (CLEAR && clears_hist(ctl) ? 2 : 0);
     }
     __syncthreads();
     const bool clear = CLEAR && (do_update & 2);
@@ -480,7 +483,7 @@ __global__ void __launch_bounds__(kUpdMultiThreads) k_upd_kl(const unsigned long
     int start = lo, end = hi < 0 ? 0 : hi;
     if (start > end) { start = 0; end = 0; }
     sc->upd = bookkeep(start, end, vis, ev, mn, klt, N, rule, stats, ctl);
-    sc->clear = ctl && !ctl->st.stop;  // the next iteration's histogram
+    sc->clear = clears_hist(ctl);
     sc->start = start;
     sc->end = end;
     // lnW[0] after its ln H subtraction (:469), from the weights before any write
@@ -540,7 +543,7 @@ __device__ __forceinline__ unsigned long long cluster_load(const void *p, uint32
 
 // The update by this block's cluster (kClusterBlocks successive blocks), PER
 // bins per thread at most.  CLEAR: in a device-driven run, zero the histogram
-// for the next iteration unless this was the last.  Returns whether this
+// for the next iteration (clears_hist).  Returns whether this
 // thread (one of the cluster) has seen the run go on.
 template <int PER, bool CLEAR>
 __device__ __forceinline__ bool cluster_update(unsigned long long *__restrict__ hist, uint32_t N,
@@ -614,7 +617,7 @@ __device__ __forceinline__ bool cluster_update(unsigned long long *__restrict__ 
             int start = v.lo, end = v.hi < 0 ? 0 : v.hi;
             if (start > end) { start = 0; end = 0; }
             const int upd = bookkeep(start, end, v.vis, v.ev, v.mn, klt, N, rule, stats, ctl ? &s_ctl : nullptr);
-            s_do = (upd ? 1u : 0u) | (ctl && !s_ctl.st.stop ? 2u : 0u);
+            s_do = (upd ? 1u : 0u) | (ctl && !s_ctl.st.stop ? 2u : 0u) | (ctl && clears_hist(&s_ctl) ? 4u : 0u);
             if (ctl) ctl->st = s_ctl.st;
         }
     }
@@ -638,7 +641,7 @@ __device__ __forceinline__ bool cluster_update(unsigned long long *__restrict__ 
                 lnw[i] = x[k];
                 w32[i] = (float)x[k];
             }
-            if (CLEAR && (todo & 2u)) hist[i] = 0ull;
+            if (CLEAR && (todo & 4u)) hist[i] = 0ull;
         }
     }
     cluster_sync();  // no block leaves while another may read its shared memory

@@ -715,9 +715,12 @@ static muca_status run_impl(muca_ctx *c, const muca_run_opts *o, muca_run_result
     h.recs = need ? c->d_recs : nullptr;
     h.rec_cap = (uint32_t)need;
     h.rec_ring = cb ? 1u : 0u;
+    h.keep_hist = cb ? 1u : 0u;
     CUDA_TRY(c, cudaMemcpyAsync(c->d_ctl, &h, sizeof h, cudaMemcpyHostToDevice, c->stream));
-    // each iteration's update clears the histogram for the next one
-    CUDA_TRY(c, cudaMemsetAsync(c->d_hist, 0, c->hist_len * 8, c->stream));
+    // without a callback each iteration's update clears the histogram for the
+    // next one; a callback may read it, or leave something else there, so then
+    // every sweep starts with a clear of its own
+    if (!cb) CUDA_TRY(c, cudaMemsetAsync(c->d_hist, 0, c->hist_len * 8, c->stream));
     // therm_coeff * N (:315-316); the CPU program's random-site runs thermalise 0 (muca_mag.cpp:140)
     const uint64_t therm = o->therm ? o->therm : (c->algo == MUCA_ALGO_RANDOM_SITE ? 0 : c->N);
     SweepArgs a = sweep_args(c, 0, 100u, 1000u, therm, 0);  // seed SEED+1000*l (:393)
@@ -775,7 +778,8 @@ static muca_status run_impl(muca_ctx *c, const muca_run_opts *o, muca_run_result
     while (!graph_mode) {
         // one iteration per host round trip, like the reference loop; the
         // device decides the schedule and convergence
-        cudaError_t e = cudaEventRecord(e0, c->stream);
+        cudaError_t e = cb ? cudaMemsetAsync(c->d_hist, 0, c->hist_len * 8, c->stream) : cudaSuccess;
+        if (e == cudaSuccess) e = cudaEventRecord(e0, c->stream);
         if (e == cudaSuccess)
             e = c->algo == MUCA_ALGO_RANDOM_SITE
                     ? launch_sweep_random(ra, c->plan.cpb, c->plan.blocks, (int)c->rounds, c->smem_optin, c->stream)

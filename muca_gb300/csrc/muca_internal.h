@@ -194,6 +194,8 @@ struct RunCtl {
     uint32_t N, nchains_total, rule, hold, flat_minmean, max_iter, sched, rec_cap;
     uint32_t rec_ring;  // 1: records go to recs[k % rec_cap] (streaming), else recs[k] for k < rec_cap
     uint32_t nup_max;   // cap of NUPDATES (0: none for schedule 0, 2^30 for the doubling ones)
+    uint32_t keep_hist; // 1: an iteration's counts stay for a callback to read (the host clears them before the
+                        // next sweep), else the update clears them once it has used them
     double mom_thr, dkl_max;
     IterRecordDev *recs;
 };
