@@ -208,11 +208,17 @@ muca_status muca_set_wait_limit(muca_ctx *ctx, uint64_t cycles);
  * never signal a filled ring slot, so the consumers' bounded waits run out.
  * Nothing faults and every wait stays bounded.
  * MUCA_HOOK_FLUSH_ROWS: the windowed sweep flushes its shared u32 histogram
- * bins into the device histogram before every row it records, the path a
- * launch takes when its bins could otherwise reach 2^32 (results are the
- * same bit for bit). */
+ * bins (production: sends the chains' 32-bit counts) into the device histogram
+ * before every row it records, the path a launch takes when one could otherwise
+ * reach 2^32 (results are the same bit for bit).
+ * MUCA_HOOK_AGED_RUN: the windowed sweep of production records as if every
+ * chain had already spent MUCA_AGED_RUN attempts in the bin it starts
+ * recording in, close to where a 32-bit count ends; the histogram has that many
+ * entries more in those bins. */
 #define MUCA_HOOK_SILENT_PRODUCER 1u
 #define MUCA_HOOK_FLUSH_ROWS 2u
+#define MUCA_HOOK_AGED_RUN 8u
+#define MUCA_AGED_RUN 0xFFFFFC00u
 muca_status muca_set_test_hooks(muca_ctx *ctx, uint32_t hooks);
 
 /* Chains.  Replaces the host lattice init (muca_delta_multigpu.cu:340-354,

@@ -46,9 +46,15 @@ constexpr long long kWaitCyclesDefault = 1ll << 34;
 // launch ends with the error word set (a test of the timeout path; it faults
 // nothing and every wait stays bounded)
 constexpr uint32_t kHookSilentProducer = 1u;
-// kHookFlushRows: the windowed sweep flushes its shared u32 bins before every
-// recorded row, as a launch that could fill a bin does
+// kHookFlushRows: the windowed sweep flushes its shared u32 bins (production:
+// sends the chains' 32-bit counts) before every recorded row, as a launch that
+// could fill one does
 constexpr uint32_t kHookFlushRows = 2u;
+// kHookAgedRun: a windowed production launch records as if every chain had
+// already spent kAgedRun attempts in its bin: its histogram has that many
+// entries more in each chain's starting bin
+constexpr uint32_t kHookAgedRun = 8u;
+constexpr uint32_t kAgedRun = 0xFFFFFC00u;  // 2^32 - 1024
 
 enum SweepMode { kModeWeight = 0, kModeProduce = 1 };
 

@@ -533,6 +533,9 @@ struct PState {
     uint32_t bin;
     int since;
 };
+// Attempts a chain may spend in one bin before its count is sent (at a row's
+// start): far below 2^32, and too seldom to cost anything.
+constexpr uint32_t kRunAttempts = 1u << 30;
 
 // An accepted attempt leaves the chain's bin of the 2D histogram: the attempts
 // since it came there go to the bin as one reduction, and the chain moves on
@@ -969,6 +972,13 @@ __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned cha
     // Recorded attempts per lane since the shared u32 bins were last flushed:
     // no bin can reach 2^32 while cpb * since stays below it
     unsigned long long since = 0;
+    // production: rows until the attempts in the chains' bins (PState::since) are sent
+    const uint32_t run_rows = (a.hooks & kHookFlushRows) ? 0u : kRunAttempts / per_row;
+    uint32_t rows_left = run_rows;
+    auto send_run = [&]() {
+        if (active && ps.since) atomicAdd(a.hist + (ps.bin >> 3), (unsigned long long)(uint32_t)-ps.since);
+        ps.since = 0;
+    };
     auto phase = [&](auto rc, unsigned long long n) {
         constexpr bool REC = decltype(rc)::value;
         uint32_t row = 0, half = 0;
@@ -981,6 +991,13 @@ __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned cha
                     since = 0;
                 }
                 since += per_row;
+            }
+            // a chain that stays in its bin for 2^32 attempts would wrap its count
+            if (PROD && REC) {
+                if (rows_left-- == 0) {  // uniform
+                    send_run();
+                    rows_left = run_rows;
+                }
             }
         };
         while (n >= per_row) {
@@ -1017,9 +1034,13 @@ __device__ __forceinline__ void win_sweep_block(const SweepArgs &a, unsigned cha
     if (PROD) {
         const uint32_t E = ps.e4 >> 2;
         ps.bin = ((uint32_t)((int)ps.mag + (int)(E * E + 2u * E)) >> 1) * 8u;
+        if (a.hooks & kHookAgedRun) {
+            ps.since = (int)(0u - kAgedRun);
+            rows_left = 0;
+        }
     }
     phase(std::true_type{}, nup);
-    if (PROD && active && ps.since) atomicAdd(a.hist + (ps.bin >> 3), (unsigned long long)(uint32_t)-ps.since);
+    if (PROD) send_run();
     if (LAT_SMEM && own) {
         const uint32_t words = L * WPR;
         for (uint32_t w = 0; w < words; ++w) gl[(size_t)w * cpb] = lat[(size_t)w * cpb];
