@@ -13,6 +13,8 @@
 #include "muca_device.cuh"
 #include "muca_internal.h"
 
+#include <algorithm>
+
 #include <cfloat>
 
 namespace muca {
@@ -655,10 +657,9 @@ __global__ void __launch_bounds__(kClusterThreads) k_upd_cluster(unsigned long l
     cluster_update<kClusterPer, true>(hist, N, lnw, w32, rule, stats, ctl);
 }
 
-// One iteration's tail for every instance of a batch without the recursion
-// (a cluster per instance, up to 16385 bins), and the count of the instances
-// still running.  The FP64 work spreads over the whole chip; a block per
-// instance left the largest one's 16385 bins to one SM (378 us at L = 128).
+// One iteration's tail for every instance of a batch without the recursion, a
+// cluster per instance (up to 16385 bins), and the count of the instances still
+// running: the form of few and large instances (batch_update_by_cluster).
 constexpr int kBatchPer = 5;
 static_assert(kClusterBlocks * kClusterThreads * kBatchPer >= 16385, "bins of the largest instance");
 __global__ void __launch_bounds__(kClusterThreads) k_batch_update(const BatchInst *__restrict__ insts,
@@ -743,8 +744,9 @@ static cudaError_t launch_update_multi(unsigned long long *hist, uint32_t N, dou
     return cudaGetLastError();
 }
 
-// The tail of a batch's iteration with the recursion: block i = instance i.
-__global__ void __launch_bounds__(kUpdThreads) k_batch_update_rec(const BatchInst *__restrict__ insts,
+// The tail of a batch's iteration by a block per instance: the recursion, and
+// the trivial updates of many or small instances.
+__global__ void __launch_bounds__(kUpdThreads) k_batch_update_block(const BatchInst *__restrict__ insts,
                                                                    uint32_t *__restrict__ running)
 {
     extern __shared__ __align__(16) unsigned char dyn[];
@@ -808,20 +810,37 @@ cudaError_t prepare_batch_update(uint32_t max_N)
     // the limit of the largest size, whatever this batch's: another batch of the
     // process shares the kernel
     if (e == cudaSuccess && update_smem(max_N, 2) > 48 * 1024)
-        return cudaFuncSetAttribute(k_batch_update_rec, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        return cudaFuncSetAttribute(k_batch_update_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)update_smem(16384, 2));
     return e;
 }
 
-cudaError_t launch_batch_update(const BatchInst *insts, uint32_t n_inst, uint32_t max_N, int recursion,
+// Clusters spread an instance's FP64 work over sixteen SMs but run some twenty at
+// a time, blocks run one per SM, so which is faster follows from the sizes.
+// Microseconds by cluster / by block, every bin visited:
+//   instances      1          16          64          200         1000
+//   L = 8       14.4/20.8   30.7/22.6   69.3/22.6  185.8/41.0   852/133
+//   L = 32      18.5/45.2   40.1/47.2    104/47.1   278/90.1   1309/307
+//   L = 64      20.5/116    42.5/117     117/117    314/229    1472/794
+//   L = 128     38.0/395    94.0/396     282/396    793/788    3852/2788
+//   L = 16..128             65.2/395     153/395    440/395    2130/1099
+// The two estimates below are fitted to these.
+bool batch_update_by_cluster(uint64_t sum_N, uint32_t max_N, uint32_t n_inst, int sms)
+{
+    const double cluster = 14.0 + 1.15 * n_inst + 0.00017 * (double)sum_N;
+    const double block = std::max(20.0 + 0.023 * max_N, (20.0 * n_inst + 0.023 * (double)sum_N) / sms);
+    return cluster < block;
+}
+
+cudaError_t launch_batch_update(const BatchInst *insts, uint32_t n_inst, uint32_t max_N, int recursion, bool cluster,
                                 uint32_t *running, cudaStream_t s)
 {
-    if (!recursion) {
+    if (!recursion && cluster) {
         cudaLaunchAttribute at;
         const cudaLaunchConfig_t cfg = cluster_config(&at, n_inst, s);
         return cudaLaunchKernelEx(&cfg, k_batch_update, insts, running);
     }
-    k_batch_update_rec<<<n_inst, kUpdThreads, update_smem(max_N, 2), s>>>(insts, running);
+    k_batch_update_block<<<n_inst, kUpdThreads, recursion ? update_smem(max_N, 2) : 0, s>>>(insts, running);
     return cudaGetLastError();
 }
 

@@ -56,6 +56,7 @@ struct muca_batch {
     size_t items_cap = 0;
     uint32_t n_items = 0;
     bool feed = false;  // the shape has drawing warps
+    bool upd_cluster = false;  // the trivial updates take a cluster per instance
     uint32_t *d_counters = nullptr;  // [0] next item, [1] running instances
     uint32_t *h_running = nullptr;
     unsigned int *d_err = nullptr;
@@ -494,6 +495,7 @@ muca_status muca_batch_create(const muca_batch_params *p, const muca_instance *i
     BTRY(cudaMemsetAsync(b->d_err, 0, sizeof(unsigned int), b->stream));
     BTRY(device_log_eps(b->device, b->stream, &b->log_eps));
     BTRY(prepare_batch_update(b->max_N));
+    b->upd_cluster = batch_update_by_cluster(b->total_w - n, b->max_N, n, b->sms);
     muca_status st;
     if (p->shape_chains_per_block) {
         muca_batch_shape s{};
@@ -635,7 +637,8 @@ muca_status muca_batch_run(muca_batch *b, const muca_batch_run_opts *o, muca_bat
                 e = launch_batch_sweep(b->d_inst, b->d_items, b->n_items, b->d_counters, b->shape.chains_per_block,
                                        b->rounds, b->shape.lattice_in_smem, b->shape.hist_in_smem, b->feed, b->grid, b->smem,
                                        smem_budget(b), b->stream);
-            if (e == cudaSuccess) e = launch_batch_update(b->d_inst, b->n, b->max_N, rec, b->d_counters + 1, b->stream);
+            if (e == cudaSuccess) e = launch_batch_update(b->d_inst, b->n, b->max_N, rec, b->upd_cluster,
+                                                          b->d_counters + 1, b->stream);
         }
         cudaGraph_t g = nullptr;
         const cudaError_t e2 = cudaStreamEndCapture(b->stream, &g);

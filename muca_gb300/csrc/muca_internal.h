@@ -250,8 +250,11 @@ cudaError_t batch_sweep_occupancy(uint32_t cpb, int rounds, uint32_t lat, bool h
                                   size_t smem_limit, int *blocks);
 // Sets the update kernels' shared-memory and cluster limits (call before any capture).
 cudaError_t prepare_batch_update(uint32_t max_N);
+// Whether the trivial updates of n_inst instances (N = L^2: their sum and the
+// largest) take a cluster each, rather than a block each.
+bool batch_update_by_cluster(uint64_t sum_N, uint32_t max_N, uint32_t n_inst, int sms);
 // The update step of every instance; *running += instances not stopped.
-cudaError_t launch_batch_update(const BatchInst *insts, uint32_t n_inst, uint32_t max_N, int recursion,
+cudaError_t launch_batch_update(const BatchInst *insts, uint32_t n_inst, uint32_t max_N, int recursion, bool cluster,
                                 uint32_t *running, cudaStream_t s);
 
 // One iteration's tail: statistics, width/convergence bookkeeping, weight

@@ -215,3 +215,39 @@ def test_batch_with_drawing_warps_equals_single_simulations(muca, insts, shape):
         assert (res[i].iterations, res[i].total_run) == (r.iterations, r.total_run), i
         np.testing.assert_array_equal(ws[i], w, err_msg="instance %d" % i)
         np.testing.assert_array_equal(hs[i], h, err_msg="instance %d" % i)
+
+
+# enough small instances that the trivial updates take a block each
+@pytest.mark.gpu
+@pytest.mark.parametrize("rule", [0, 1])
+def test_batch_of_many_small_instances_equals_single_simulations(muca, rule):
+    insts = [(8 * (1 + k % 3), 32, 2.0, k) for k in range(40)]
+    kw = dict(rule=rule, flat_minmean=1, max_iter=12)
+    with muca.Batch(insts, shape=(32, 1, 1)) as b:
+        res, _ = b.run(starting_M=1, graph_iters=4, **kw)
+        ws = [b.get_weights(i) for i in range(len(insts))]
+    for i in (0, 1, 2, 20, 39):
+        L, nc, _, seed = insts[i]
+        r, w, _ = _single(muca, L, nc, seed, **kw)
+        assert (res[i].iterations, res[i].total_run) == (r.iterations, r.total_run), i
+        np.testing.assert_array_equal(ws[i], w, err_msg="instance %d" % i)
+
+
+@pytest.mark.gpu
+def test_batch_trivial_update_costs_no_more_than_the_recursion(muca):
+    """An iteration of many small instances with a trivial update: its work per
+    bin is part of the recursion's, so it must not take longer (a quarter more
+    for the clock's noise)."""
+    insts = [(8, 32, 2.0, k) for k in range(512)]
+    with muca.Batch(insts, shape=(32, 1, 1)) as b:
+        def per_iteration(rule):
+            best = []
+            for n in (64, 320):
+                t = []
+                for _ in range(5):
+                    _, sec = b.run(starting_M=64, rule=rule, max_iter=n, graph_iters=32, d_kl_max=1e-30)
+                    t.append(sec)
+                best.append(min(t))
+            return (best[1] - best[0]) / 256
+        trivial, recursion = per_iteration(muca.UPDATE_TRIVIAL), per_iteration(muca.UPDATE_RECURSION)
+    assert trivial <= 1.25 * recursion, (trivial, recursion)
