@@ -521,12 +521,14 @@ __global__ void __launch_bounds__(kUpdMultiThreads) k_upd_apply(unsigned long lo
 // between them, the partial results read from the other blocks' shared memory
 // and the bins held in registers, and forms the updated weights while one
 // thread keeps the books.  What bounds it is the latency of its FP64 divisions
-// and logarithms (FP64 issues slowly on this GPU) and of the barriers.  Back to
-// back, N = 256: 14.5 us against 22.6 for the three launches (whose cost does
-// not depend on the size); N = 4096: 16.4; N = 5184: 20.6; above 8191 bins, two
-// per thread, the three launches with their 64 SMs stay.
+// and logarithms (FP64 issues slowly on this GPU) and of the barriers.  Every bin
+// visited, back to back in a stream / in a graph, against the three launches
+// (whose cost does not depend on the size): N = 256: 16.4/14.7 us for 22.5/15.7,
+// N = 3969: 17.4/15.1 for 22.5/15.9, N = 4096: 20.5/17.8, N = 4356..8100:
+// 22.6..23.5/21.1: a second bin per thread costs more than the launches saved, so
+// from 4097 bins the three launches with their 64 SMs serve.
 constexpr uint32_t kClusterBlocks = 16, kClusterThreads = 256;
-constexpr int kClusterPer = 2;  // bins per thread at most
+constexpr int kClusterPer = 1;  // bins per thread
 constexpr uint32_t kClusterBins = kClusterBlocks * kClusterThreads * kClusterPer;
 
 __device__ __forceinline__ void cluster_sync()
