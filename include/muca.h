@@ -214,10 +214,14 @@ muca_status muca_set_wait_limit(muca_ctx *ctx, uint64_t cycles);
  * MUCA_HOOK_AGED_RUN: the windowed sweep of production records as if every
  * chain had already spent MUCA_AGED_RUN attempts in the bin it starts
  * recording in, close to where a 32-bit count ends; the histogram has that many
- * entries more in those bins. */
+ * entries more in those bins.
+ * MUCA_HOOK_NO_CLUSTER: the weight updates run as on a device (or a partition
+ * of one) that has no place for a thread-block cluster of sixteen blocks: the
+ * same weights, the divergence summed in another order. */
 #define MUCA_HOOK_SILENT_PRODUCER 1u
 #define MUCA_HOOK_FLUSH_ROWS 2u
 #define MUCA_HOOK_AGED_RUN 8u
+#define MUCA_HOOK_NO_CLUSTER 16u
 #define MUCA_AGED_RUN 0xFFFFFC00u
 muca_status muca_set_test_hooks(muca_ctx *ctx, uint32_t hooks);
 

@@ -782,10 +782,26 @@ static cudaError_t prep_update(uint32_t N, int rule)
     return cudaSuccess;
 }
 
-cudaError_t launch_weight_update(unsigned long long *hist, uint32_t N, double *lnw, float *w32, double *p_acc,
-                                 int rule, HistStatsDev *stats, cudaStream_t s, UpdScratch *sc, const RecScratch *rs)
+// Sixteen blocks of a cluster need SMs of one GPC: a partition of the device (or
+// an SM-restricted context) may have none to place them on.
+bool update_cluster_fits(cudaStream_t s, bool batch)
 {
-    if (rule != 2 && N < kClusterBins) return launch_update_cluster(hist, N, lnw, w32, rule, stats, nullptr, s);
+    const void *kern = batch ? (const void *)k_batch_update : (const void *)k_upd_cluster;
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg = cluster_config(&at, 1, s);
+    int clusters = 0;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess && clusters > 0;
+}
+
+cudaError_t launch_weight_update(unsigned long long *hist, uint32_t N, double *lnw, float *w32, double *p_acc,
+                                 int rule, HistStatsDev *stats, cudaStream_t s, bool cluster, UpdScratch *sc,
+                                 const RecScratch *rs)
+{
+    if (cluster && rule != 2 && N < kClusterBins)
+        return launch_update_cluster(hist, N, lnw, w32, rule, stats, nullptr, s);
     if (sc && (rule != 2 || rs))
         return launch_update_multi(hist, N, lnw, w32, p_acc, rule, stats, nullptr, sc, rs, s);
     cudaError_t e = prep_update(N, rule);
@@ -795,9 +811,11 @@ cudaError_t launch_weight_update(unsigned long long *hist, uint32_t N, double *l
 }
 
 cudaError_t launch_run_update(unsigned long long *hist, double *lnw, float *w32, double *p_acc, RunCtl *ctl,
-                              cudaStream_t s, uint32_t N, int rule, UpdScratch *sc, const RecScratch *rs)
+                              cudaStream_t s, uint32_t N, int rule, bool cluster, UpdScratch *sc,
+                              const RecScratch *rs)
 {
-    if (rule != 2 && N < kClusterBins) return launch_update_cluster(hist, N, lnw, w32, rule, nullptr, ctl, s);
+    if (cluster && rule != 2 && N < kClusterBins)
+        return launch_update_cluster(hist, N, lnw, w32, rule, nullptr, ctl, s);
     if (sc && (rule != 2 || rs))
         return launch_update_multi(hist, N, lnw, w32, p_acc, rule, nullptr, ctl, sc, rs, s);
     cudaError_t e = prep_update(N, rule);
@@ -808,13 +826,12 @@ cudaError_t launch_run_update(unsigned long long *hist, double *lnw, float *w32,
 
 cudaError_t prepare_batch_update(uint32_t max_N)
 {
-    const cudaError_t e = cudaFuncSetAttribute(k_batch_update, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     // the limit of the largest size, whatever this batch's: another batch of the
     // process shares the kernel
-    if (e == cudaSuccess && update_smem(max_N, 2) > 48 * 1024)
+    if (update_smem(max_N, 2) > 48 * 1024)
         return cudaFuncSetAttribute(k_batch_update_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)update_smem(16384, 2));
-    return e;
+    return cudaSuccess;
 }
 
 // Clusters spread an instance's FP64 work over sixteen SMs but run some twenty at

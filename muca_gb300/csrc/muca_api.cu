@@ -37,6 +37,7 @@ struct muca_ctx {
     // the statistics and, behind them, the error word: one copy brings both
     HistStatsDev *d_stats = nullptr, *h_stats = nullptr;
     UpdScratch *d_upd = nullptr;  // the multi-block weight update
+    bool cluster_fits = false;    // the one-launch weight update can be placed
     RunCtl *d_ctl = nullptr, *h_ctl = nullptr;
     IterRecordDev *d_recs = nullptr;
     size_t recs_cap = 0;
@@ -129,6 +130,8 @@ muca_status recompute_energies(muca_ctx *c)
                                 c->stream));
     return MUCA_OK;
 }
+
+bool by_cluster(const muca_ctx *c) { return c->cluster_fits && !(c->hooks & kHookNoCluster); }
 
 // Synchronises and reports a wait that gave up; h_stats has the statistics
 // of the last update afterwards.
@@ -318,6 +321,7 @@ muca_status muca_create(const muca_params *p, muca_ctx **out)
     c->d_err = reinterpret_cast<unsigned int *>(c->d_stats + 1);
     CREATE_TRY(dmalloc(c, &c->d_upd, 1));
     CREATE_TRY(cudaMemsetAsync(c->d_upd, 0, sizeof(UpdScratch), c->stream));
+    c->cluster_fits = c->mode == MUCA_MODE_WEIGHT && update_cluster_fits(c->stream, false);
     if (c->mode == MUCA_MODE_WEIGHT) {
         CREATE_TRY(dmalloc(c, &c->rec.ds, (size_t)N));
         CREATE_TRY(dmalloc(c, &c->rec.valid, (size_t)N));
@@ -430,10 +434,12 @@ muca_status muca_set_wait_limit(muca_ctx *c, uint64_t cycles)
 muca_status muca_set_test_hooks(muca_ctx *c, uint32_t hooks)
 {
     if (!c) return fail(nullptr, MUCA_ERR_BAD_ARG, "ctx is NULL");
-    if (hooks & ~(uint32_t)(MUCA_HOOK_SILENT_PRODUCER | MUCA_HOOK_FLUSH_ROWS | MUCA_HOOK_AGED_RUN))
+    if (hooks & ~(uint32_t)(MUCA_HOOK_SILENT_PRODUCER | MUCA_HOOK_FLUSH_ROWS | MUCA_HOOK_AGED_RUN |
+                            MUCA_HOOK_NO_CLUSTER))
         return fail(c, MUCA_ERR_BAD_ARG, "unknown hook bits 0x%x", hooks);
     static_assert(MUCA_HOOK_SILENT_PRODUCER == kHookSilentProducer && MUCA_HOOK_FLUSH_ROWS == kHookFlushRows &&
-                      MUCA_HOOK_AGED_RUN == kHookAgedRun && MUCA_AGED_RUN == kAgedRun,
+                      MUCA_HOOK_AGED_RUN == kHookAgedRun && MUCA_AGED_RUN == kAgedRun &&
+                      MUCA_HOOK_NO_CLUSTER == kHookNoCluster,
                   "hook bits");
     c->hooks = hooks;
     return MUCA_OK;
@@ -612,8 +618,8 @@ static muca_status update_impl(muca_ctx *c, int rule, muca_hist_stats *st)
     if (!c) return fail(nullptr, MUCA_ERR_BAD_ARG, "ctx is NULL");
     if (c->mode != MUCA_MODE_WEIGHT) return fail(c, MUCA_ERR_STATE, "weight statistics need a weight-mode context");
     CUDA_TRY(c, cudaSetDevice(c->device));
-    CUDA_TRY(c, launch_weight_update(c->d_hist, c->N, c->d_lnw, c->d_w32, c->d_pacc, rule, c->d_stats, c->stream, c->d_upd,
-                                     &c->rec));
+    CUDA_TRY(c, launch_weight_update(c->d_hist, c->N, c->d_lnw, c->d_w32, c->d_pacc, rule, c->d_stats, c->stream,
+                                     by_cluster(c), c->d_upd, &c->rec));
     if (!st) return MUCA_OK;  // enqueue only
     if (muca_status e = check_err(c)) return e;
     stats_out(*c->h_stats, st);
@@ -651,7 +657,7 @@ muca_status muca_iterate_host(muca_ctx *c, const double *lnw_in, uint32_t iter, 
     }
     if (muca_status e = do_sweep(c, iter, seed_base, seed_dev_mul, therm, nup, !lnw_in)) return e;
     CUDA_TRY(c, launch_weight_update(c->d_hist, c->N, c->d_lnw, c->d_w32, c->d_pacc, (int)rule, c->d_stats, c->stream,
-                                     c->d_upd, &c->rec));
+                                     by_cluster(c), c->d_upd, &c->rec));
     if (lnw_out) CUDA_TRY(c, cudaMemcpyAsync(lnw_out, c->d_lnw, n * 8, cudaMemcpyDeviceToHost, c->stream));
     if (hist_out) CUDA_TRY(c, cudaMemcpyAsync(hist_out, c->d_hist, n * 8, cudaMemcpyDeviceToHost, c->stream));
     if (muca_status e = check_err(c)) return e;  // the one synchronisation
@@ -750,7 +756,7 @@ static muca_status run_impl(muca_ctx *c, const muca_run_opts *o, muca_run_result
                         ? launch_sweep_random(ra, c->plan.cpb, c->plan.blocks, (int)c->rounds, c->smem_optin, c->stream)
                         : launch_sweep(c->plan, a, c->stream);
             if (e == cudaSuccess) e = launch_run_update(c->d_hist, c->d_lnw, c->d_w32, c->d_pacc, c->d_ctl, c->stream,
-                                                        c->N, (int)o->rule, c->d_upd, &c->rec);
+                                                        c->N, (int)o->rule, by_cluster(c), c->d_upd, &c->rec);
         }
         if (capturing) {
             const cudaError_t ec = cudaStreamEndCapture(c->stream, &graph);
@@ -787,7 +793,7 @@ static muca_status run_impl(muca_ctx *c, const muca_run_opts *o, muca_run_result
                     : launch_sweep(c->plan, a, c->stream);
         if (e == cudaSuccess) e = cudaEventRecord(e1, c->stream);
         if (e == cudaSuccess) e = launch_run_update(c->d_hist, c->d_lnw, c->d_w32, c->d_pacc, c->d_ctl, c->stream,
-                                                        c->N, (int)o->rule, c->d_upd, &c->rec);
+                                                        c->N, (int)o->rule, by_cluster(c), c->d_upd, &c->rec);
         if (e == cudaSuccess) e = cudaEventRecord(m0, c->stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(&h.st, &c->d_ctl->st, sizeof(IterState), cudaMemcpyDeviceToHost, c->stream);
         if (e == cudaSuccess) e = cudaEventRecord(m1, c->stream);

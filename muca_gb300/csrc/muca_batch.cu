@@ -495,7 +495,7 @@ muca_status muca_batch_create(const muca_batch_params *p, const muca_instance *i
     BTRY(cudaMemsetAsync(b->d_err, 0, sizeof(unsigned int), b->stream));
     BTRY(device_log_eps(b->device, b->stream, &b->log_eps));
     BTRY(prepare_batch_update(b->max_N));
-    b->upd_cluster = batch_update_by_cluster(b->total_w - n, b->max_N, n, b->sms);
+    b->upd_cluster = batch_update_by_cluster(b->total_w - n, b->max_N, n, b->sms) && update_cluster_fits(b->stream, true);
     muca_status st;
     if (p->shape_chains_per_block) {
         muca_batch_shape s{};

@@ -50,6 +50,9 @@ constexpr uint32_t kHookSilentProducer = 1u;
 // sends the chains' 32-bit counts) before every recorded row, as a launch that
 // could fill one does
 constexpr uint32_t kHookFlushRows = 2u;
+// kHookNoCluster: the weight updates run as on a device that has no place for a
+// cluster
+constexpr uint32_t kHookNoCluster = 16u;
 // kHookAgedRun: a windowed production launch records as if every chain had
 // already spent kAgedRun attempts in its bin: its histogram has that many
 // entries more in each chain's starting bin
@@ -177,9 +180,14 @@ struct RecScratch {
 // (zero-initialised once) rules -1, 0 and 1 spread their FP64 work over
 // kUpdBlocks blocks, and so does rule 2 when `rs` is given too (its prefix
 // then runs as one block's segmented scan); otherwise one block does all.
+// `cluster` (update_cluster_fits): rules -1, 0 and 1 of up to 4096 bins may run
+// as one cluster launch.
 cudaError_t launch_weight_update(unsigned long long *hist, uint32_t N, double *lnw, float *w32,
-                                 double *p_acc, int rule, HistStatsDev *stats, cudaStream_t s,
+                                 double *p_acc, int rule, HistStatsDev *stats, cudaStream_t s, bool cluster,
                                  UpdScratch *sc = nullptr, const RecScratch *rs = nullptr);
+// Whether the device can place a cluster of the update (batch: of a batch's) on
+// behalf of stream s; call before any capture.
+bool update_cluster_fits(cudaStream_t s, bool batch);
 
 // Device-resident state of a weight-estimation run (the loop of
 // muca_delta_multigpu.cu:374-477).  The first three words are what the
@@ -248,7 +256,7 @@ size_t batch_sweep_smem(uint32_t L, uint32_t cpb, bool lat_smem, bool hist_smem,
 // The launch with that shape needs no further attribute call.
 cudaError_t batch_sweep_occupancy(uint32_t cpb, int rounds, uint32_t lat, bool hist_smem, bool feed, size_t smem,
                                   size_t smem_limit, int *blocks);
-// Sets the update kernels' shared-memory and cluster limits (call before any capture).
+// Sets the update kernels' shared-memory limit (call before any capture).
 cudaError_t prepare_batch_update(uint32_t max_N);
 // Whether the trivial updates of n_inst instances (N = L^2: their sum and the
 // largest) take a cluster each, rather than a block each.
@@ -260,8 +268,8 @@ cudaError_t launch_batch_update(const BatchInst *insts, uint32_t n_inst, uint32_
 // One iteration's tail: statistics, width/convergence bookkeeping, weight
 // update, schedule of the next NUPDATES; a no-op once st.stop is set.
 cudaError_t launch_run_update(unsigned long long *hist, double *lnw, float *w32, double *p_acc,
-                              RunCtl *ctl, cudaStream_t s, uint32_t N, int rule, UpdScratch *sc = nullptr,
-                              const RecScratch *rs = nullptr);
+                              RunCtl *ctl, cudaStream_t s, uint32_t N, int rule, bool cluster,
+                              UpdScratch *sc = nullptr, const RecScratch *rs = nullptr);
 // After FP64 weights have arrived in lnw[0..n): the FP32 shadow, the copy obs
 // (unless NULL), and the histogram's first n_hist bins cleared.
 cudaError_t launch_weights_in(const double *lnw, float *w32, double *obs, uint32_t n, unsigned long long *hist,
