@@ -286,21 +286,18 @@ __device__ __forceinline__ unsigned char recursion_increment(const unsigned long
     return 1;
 }
 
-// `dyn`: dynamic shared memory of update_smem(N, rule) bytes.
-// CLEAR: in a device-driven run, zero the histogram for the next iteration
-// (clears_hist).
-template <bool CLEAR = false>
-__device__ __forceinline__ void weight_update_body(unsigned long long *__restrict__ hist, uint32_t N,
+// One block's statistics and update of an instance of a batch.  `dyn`: dynamic
+// shared memory of update_smem(N, rule) bytes.
+__device__ __forceinline__ void weight_update_body(const unsigned long long *__restrict__ hist, uint32_t N,
                                                    double *__restrict__ lnw, float *__restrict__ w32,
-                                                   double *__restrict__ p_acc, int rule,
-                                                   HistStatsDev *__restrict__ stats, RunCtl *__restrict__ ctl,
+                                                   double *__restrict__ p_acc, int rule, RunCtl *__restrict__ ctl,
                                                    unsigned char *dyn)
 {
     __shared__ HistSum shs[32];
     __shared__ double shd[32];
     __shared__ int do_update;
     const uint32_t tid = threadIdx.x, bs = blockDim.x;
-    if (ctl && ctl->st.stop) return;
+    if (ctl->st.stop) return;
 
     // values needed before anything is written (normalisation constant)
     const unsigned long long h0 = hist[0];
@@ -325,17 +322,9 @@ __device__ __forceinline__ void weight_update_body(unsigned long long *__restric
         }
     }
     kl = block_reduce(kl, AddD(), shd);
-    if (tid == 0) {
-        const int upd = bookkeep(start, end, vis, ev, mn, kl, N, rule, stats, ctl);
-        do_update = upd | (CLEAR && clears_hist(ctl) ? 2 : 0);
-    }
+    if (tid == 0) do_update = bookkeep(start, end, vis, ev, mn, kl, N, rule, nullptr, ctl);
     __syncthreads();
-    const bool clear = CLEAR && (do_update & 2);
-    if (!(do_update & 1)) {
-        if (clear)
-            for (uint32_t i = tid; i <= N; i += bs) hist[i] = 0ull;
-        return;
-    }
+    if (!do_update) return;
 
     if (rule == 0 || rule == 1) {
         // tmp = lnW[0] after the ln H subtraction (:469), computed from the
@@ -349,7 +338,6 @@ __device__ __forceinline__ void weight_update_body(unsigned long long *__restric
             if (rule == 0 || h > 0) v = __dsub_rn(v, tmp);
             lnw[i] = v;
             w32[i] = (float)v;
-            if (clear) hist[i] = 0ull;
         }
         return;
     }
@@ -369,18 +357,7 @@ __device__ __forceinline__ void weight_update_body(unsigned long long *__restric
         v = __dsub_rn(v, lnw0);
         lnw[i] = v;
         w32[i] = (float)v;
-        if (clear) hist[i] = 0ull;
     }
-}
-
-__global__ void __launch_bounds__(kUpdThreads) k_weight_update(unsigned long long *__restrict__ hist, uint32_t N,
-                                                                double *__restrict__ lnw, float *__restrict__ w32,
-                                                                double *__restrict__ p_acc, int rule,
-                                                                HistStatsDev *__restrict__ stats,
-                                                                RunCtl *__restrict__ ctl)
-{
-    extern __shared__ __align__(16) unsigned char dyn[];
-    weight_update_body<true>(hist, N, lnw, w32, p_acc, rule, stats, ctl, dyn);
 }
 
 // ---- the same statistics and update over kUpdBlocks blocks ---------------
@@ -753,7 +730,7 @@ __global__ void __launch_bounds__(kUpdThreads) k_batch_update_block(const BatchI
 {
     extern __shared__ __align__(16) unsigned char dyn[];
     const BatchInst &I = insts[blockIdx.x];
-    weight_update_body(I.a.hist, I.a.N, I.lnw, I.w32, I.p_acc, (int)I.rule, nullptr, I.ctl, dyn);
+    weight_update_body(I.a.hist, I.a.N, I.lnw, I.w32, I.p_acc, (int)I.rule, I.ctl, dyn);
     if (threadIdx.x == 0 && !I.ctl->st.stop) atomicAdd(running, 1u);
 }
 
@@ -773,14 +750,6 @@ __global__ void k_weights_in(const double *__restrict__ lnw, float *__restrict__
 }
 
 static size_t update_smem(uint32_t N, int rule) { return rule == 2 ? (size_t)N * (sizeof(double) + 1) : 0; }
-
-static cudaError_t prep_update(uint32_t N, int rule)
-{
-    if (update_smem(N, rule) > 48 * 1024)
-        return cudaFuncSetAttribute(k_weight_update, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)update_smem(16384, 2));
-    return cudaSuccess;
-}
 
 // Sixteen blocks of a cluster need SMs of one GPC: a partition of the device (or
 // an SM-restricted context) may have none to place them on.
@@ -802,12 +771,7 @@ cudaError_t launch_weight_update(unsigned long long *hist, uint32_t N, double *l
 {
     if (cluster && rule != 2 && N < kClusterBins)
         return launch_update_cluster(hist, N, lnw, w32, rule, stats, nullptr, s);
-    if (sc && (rule != 2 || rs))
-        return launch_update_multi(hist, N, lnw, w32, p_acc, rule, stats, nullptr, sc, rs, s);
-    cudaError_t e = prep_update(N, rule);
-    if (e != cudaSuccess) return e;
-    k_weight_update<<<1, kUpdThreads, update_smem(N, rule), s>>>(hist, N, lnw, w32, p_acc, rule, stats, nullptr);
-    return cudaGetLastError();
+    return launch_update_multi(hist, N, lnw, w32, p_acc, rule, stats, nullptr, sc, rs, s);
 }
 
 cudaError_t launch_run_update(unsigned long long *hist, double *lnw, float *w32, double *p_acc, RunCtl *ctl,
@@ -816,12 +780,7 @@ cudaError_t launch_run_update(unsigned long long *hist, double *lnw, float *w32,
 {
     if (cluster && rule != 2 && N < kClusterBins)
         return launch_update_cluster(hist, N, lnw, w32, rule, nullptr, ctl, s);
-    if (sc && (rule != 2 || rs))
-        return launch_update_multi(hist, N, lnw, w32, p_acc, rule, nullptr, ctl, sc, rs, s);
-    cudaError_t e = prep_update(N, rule);
-    if (e != cudaSuccess) return e;
-    k_weight_update<<<1, kUpdThreads, update_smem(N, rule), s>>>(hist, N, lnw, w32, p_acc, rule, nullptr, ctl);
-    return cudaGetLastError();
+    return launch_update_multi(hist, N, lnw, w32, p_acc, rule, nullptr, ctl, sc, rs, s);
 }
 
 cudaError_t prepare_batch_update(uint32_t max_N)

@@ -146,7 +146,7 @@ cudaError_t launch_energies(const uint32_t *lat, int32_t *ej, int32_t *edel, int
 // Checks that every value of an int8 lattice is in {-1,0,1}; *bad gets the count of others.
 cudaError_t launch_validate(const int8_t *src, size_t n, unsigned long long *bad, cudaStream_t s);
 
-// Weight math (k_weights.cu), FP64, one block per instance.
+// Weight math (k_weights.cu), FP64.
 struct HistStatsDev {
     int32_t start, end;
     uint32_t width, visited;
@@ -176,15 +176,13 @@ struct RecScratch {
     unsigned char *valid;
 };
 // stats of hist[0..N]; if rule >= 0 also updates lnw (FP64) / w32 (FP32 shadow)
-// (rule: 0 trivial, 1 trivial-cpu, 2 recursion with p_acc).  With `sc`
-// (zero-initialised once) rules -1, 0 and 1 spread their FP64 work over
-// kUpdBlocks blocks, and so does rule 2 when `rs` is given too (its prefix
-// then runs as one block's segmented scan); otherwise one block does all.
-// `cluster` (update_cluster_fits): rules -1, 0 and 1 of up to 4096 bins may run
-// as one cluster launch.
+// (rule: 0 trivial, 1 trivial-cpu, 2 recursion with p_acc), the FP64 work over
+// kUpdBlocks blocks (the recursion's prefix as one block's segmented scan), or,
+// with `cluster` (update_cluster_fits), of up to 4096 bins and rules -1, 0 and 1
+// as one cluster launch.  `sc`: zero-initialised once.
 cudaError_t launch_weight_update(unsigned long long *hist, uint32_t N, double *lnw, float *w32,
                                  double *p_acc, int rule, HistStatsDev *stats, cudaStream_t s, bool cluster,
-                                 UpdScratch *sc = nullptr, const RecScratch *rs = nullptr);
+                                 UpdScratch *sc, const RecScratch *rs);
 // Whether the device can place a cluster of the update (batch: of a batch's) on
 // behalf of stream s; call before any capture.
 bool update_cluster_fits(cudaStream_t s, bool batch);
@@ -269,7 +267,7 @@ cudaError_t launch_batch_update(const BatchInst *insts, uint32_t n_inst, uint32_
 // update, schedule of the next NUPDATES; a no-op once st.stop is set.
 cudaError_t launch_run_update(unsigned long long *hist, double *lnw, float *w32, double *p_acc,
                               RunCtl *ctl, cudaStream_t s, uint32_t N, int rule, bool cluster,
-                              UpdScratch *sc = nullptr, const RecScratch *rs = nullptr);
+                              UpdScratch *sc, const RecScratch *rs);
 // After FP64 weights have arrived in lnw[0..n): the FP32 shadow, the copy obs
 // (unless NULL), and the histogram's first n_hist bins cleared.
 cudaError_t launch_weights_in(const double *lnw, float *w32, double *obs, uint32_t n, unsigned long long *hist,
