@@ -65,10 +65,13 @@ __global__ void k_weight_shift(double *lnw, uint32_t N, double beta, double delt
 //     five nested sums, c0 += G, c1 += c0, ... c4 += c3, which end as
 //     e_p = sum_k C(k+p, p) G_k: ten additions for two bins;
 //   * the sums of k^p G and of |m|^p G follow from them once per row.
-// They are 64-bit: G < 2^30 and K <= 256 keep e4 <= 2^30 C(260, 5) < 2^64.  A
-// row with a bin of 2^29 or more is summed again with 128-bit products, bin by
-// bin; both give the exact sums.
-// L = 128 (1.07 GB): 169 us a pass (6.4 TB/s), 351 with products for every bin.
+// They are 64-bit: G < 2^30 and K <= 257 keep e4 <= 2^30 C(261, 5) < 2^64.  A
+// row with a bin of 2^29 or more is summed again in two parts (row_moments_wide),
+// and so are a warp's next rows from the start while they have such bins; both
+// give the exact sums.
+// L = 128 (1.07 GB): 169 us a pass (6.4 TB/s), 351 with products for every bin;
+// every bin 2^30: 229 us, 351 with products at once, 997 with them after a first
+// reading.
 constexpr int kObsUnroll = 8;
 
 typedef unsigned __int128 u128;
@@ -112,29 +115,98 @@ struct RowMoments {
     u128 a0, a1, a2, a4;  // sums of H, |m| H, m^2 H, m^4 H
 };
 
-// A lane's part of row i with bins of any size: j = lane, lane + 32, ...
-__device__ __forceinline__ RowMoments row_moments_wide(const unsigned long long *row, uint32_t i, uint32_t lane)
+// The moments from nested sums: s_p = sum_k k^p G_k from C(k+1,1) = k + 1,
+// 2 C(k+2,2) = k^2 + 3k + 2, 6 C(k+3,3) = k^3 + 6k^2 + 11k + 6 and
+// 24 C(k+4,4) = k^4 + 10k^3 + 35k^2 + 50k + 24, then (b + 64 k)^p term by term.
+__device__ __noinline__ RowMoments moments_of_nested(u128 c0, u128 c1, u128 c2, u128 c3, u128 c4, uint32_t b)
 {
-    RowMoments r{0, 0, 0, 0};
-#pragma unroll 1
-    for (uint32_t j = lane; j <= i; j += 32u) {
-        const unsigned long long H = row[j];
-        const int m = 2 * (int)j - (int)i;
-        const uint32_t am = (uint32_t)(m < 0 ? -m : m);  // <= N <= 16384
-        const uint32_t am2 = am * am;                    // < 2^29
-        // 64 x 32-bit products; H m^4 = (H m^2) m^2 with H m^2 < 2^93
-        const u128 t = (u128)H * am2;
-        const unsigned long long tl = (unsigned long long)t, th = (unsigned long long)(t >> 64);
-        r.a0 += H;
-        r.a1 += (u128)H * am;
-        r.a2 += t;
-        r.a4 += (u128)tl * am2 + ((u128)(th * am2) << 64);
-    }
+    const u128 s1 = c1 - c0, s2 = 2 * c2 - 3 * s1 - 2 * c0, s3 = 6 * c3 - 6 * s2 - 11 * s1 - 6 * c0;
+    const u128 s4 = 24 * c4 - 10 * s3 - 35 * s2 - 50 * s1 - 24 * c0;
+    const uint32_t b2 = b * b;  // b <= 63
+    RowMoments r;
+    r.a0 = c0;
+    r.a1 = c0 * b + s1 * 64u;
+    r.a2 = c0 * b2 + s1 * (128u * b) + s2 * 4096u;
+    r.a4 = c0 * (b2 * b2) + s1 * (256u * b2 * b) + s2 * (24576u * b2) + s3 * (1048576u * b) + (s4 << 24);
     return r;
 }
 
-// A lane's part of row i by nested sums (above); bins past 2^29 are reported
-// in `big`.
+// A lane's part of row i with bins of any size: the nested sums of their low 29
+// bits and of the rest beside each other (the rest is below 2^35, so its fourth
+// sum may reach 2^70 and takes 96 bits).  Twice the additions keep it near HBM's
+// pace where a 128-bit product per bin did not; `big`: some bin needs it.
+__device__ __forceinline__ RowMoments row_moments_wide(const unsigned long long *row, uint32_t i, uint32_t lane,
+                                                       bool &big)
+{
+    typedef unsigned long long u64;
+    const uint32_t half = i / 2 + 1;
+    const u64 *up = row + (i + 1) / 2, *dn = row + i / 2;
+    constexpr int U = kObsUnroll / 2;
+    constexpr uint32_t low = (1u << 29) - 1u;
+    int k = (int)((half + 32u * U - 1) / (32u * U)) * U - 1;
+    u64 hu[U], hd[U], nu[U], ndn[U];
+    auto load = [&](int k0, u64 (&a)[U], u64 (&b)[U]) {
+#pragma unroll
+        for (int t = 0; t < U; ++t) {
+            const uint32_t n = lane + 32u * (uint32_t)(k0 - t);
+            const bool in = k0 - t >= 0 && n < half;
+            a[t] = in ? __ldcs(up + n) : 0ull;
+            b[t] = in ? __ldcs(dn - (int)n) : 0ull;
+        }
+    };
+    load(k, hu, hd);
+    u64 c0 = 0, c1 = 0, c2 = 0, c3 = 0, c4 = 0, g0 = 0, g1 = 0, g2 = 0, g3 = 0, g4 = 0;
+    uint32_t g5 = 0;
+    for (; k >= 0; k -= U) {
+        load(k - U, nu, ndn);
+#pragma unroll
+        for (int t = 0; t < U; ++t) {
+            c0 += ((uint32_t)hu[t] & low) + ((uint32_t)hd[t] & low);
+            c1 += c0;
+            c2 += c1;
+            c3 += c2;
+            c4 += c3;
+            g0 += (hu[t] >> 29) + (hd[t] >> 29);
+            g1 += g0;
+            g2 += g1;
+            g3 += g2;
+            g4 += g3;
+            g5 += g4 < g3;
+        }
+#pragma unroll
+        for (int t = 0; t < U; ++t) {
+            hu[t] = nu[t];
+            hd[t] = ndn[t];
+        }
+    }
+    big = g0 != 0;
+    u128 g4w = ((u128)g5 << 64) | g4;
+    if ((i & 1u) == 0 && lane == 0) {
+        // the bin m = 0 was folded with itself
+        const u64 z = *dn & low, y = *dn >> 29;
+        c0 -= z;
+        c1 -= z;
+        c2 -= z;
+        c3 -= z;
+        c4 -= z;
+        g0 -= y;
+        g1 -= y;
+        g2 -= y;
+        g3 -= y;
+        g4w -= y;
+    }
+    const uint32_t b = (i & 1u) + 2u * lane;
+    RowMoments r = moments_of_nested(c0, c1, c2, c3, c4, b);
+    const RowMoments q = moments_of_nested(g0, g1, g2, g3, g4w, b);
+    r.a0 += q.a0 << 29;
+    r.a1 += q.a1 << 29;
+    r.a2 += q.a2 << 29;
+    r.a4 += q.a4 << 29;
+    return r;
+}
+
+// A lane's part of row i by nested sums (above); bins from 2^29 are reported in
+// `big` (the sums are then wrong).
 __device__ __forceinline__ RowMoments row_moments(const unsigned long long *row, uint32_t i, uint32_t lane, bool &big)
 {
     typedef unsigned long long u64;
@@ -184,8 +256,7 @@ __device__ __forceinline__ RowMoments row_moments(const unsigned long long *row,
         c3 -= z;
         c4 -= z;
     }
-    // s_p = sum_k k^p G_k from C(k+1,1) = k + 1, 2 C(k+2,2) = k^2 + 3k + 2,
-    // 6 C(k+3,3) = k^3 + 6k^2 + 11k + 6, 24 C(k+4,4) = k^4 + 10k^3 + 35k^2 + 50k + 24
+    // as moments_of_nested, in 64 bits where they suffice
     const u64 s1 = c1 - c0, s2 = 2 * c2 - 3 * s1 - 2 * c0, s3 = 6 * c3 - 6 * s2 - 11 * s1 - 6 * c0;
     const u128 s4 = (u128)c4 * 24u - (u128)s3 * 10u - (u128)s2 * 35u - (u128)s1 * 50u - (u128)c0 * 24u;
     const uint32_t b = (i & 1u) + 2u * lane, b2 = b * b;  // <= 63
@@ -213,14 +284,22 @@ __global__ void __launch_bounds__(kObsThreads, 1) k_observables(const unsigned l
     uint32_t first = 0, slot = 0, my_row = 0;
     RowMoments mine{0, 0, 0, 0};
     bool turn = false;
+    bool wide = false;  // (uniform) the last row had bins of 2^29 or more
     while (first <= N) {
         const uint32_t at = first + (turn ? nwarps - 1u - w : w);
         if (at <= N) {
             const uint32_t i = N - at;
             const unsigned long long *row = hist + (unsigned long long)i * (i + 1) / 2;
-            bool big;
-            RowMoments r = row_moments(row, i, ln, big);
-            if (__any_sync(0xffffffffu, big)) r = row_moments_wide(row, i, ln);
+            bool big = false;
+            RowMoments r;
+            if (!wide) {
+                r = row_moments(row, i, ln, big);
+                wide = __any_sync(0xffffffffu, big);
+                if (wide) r = row_moments_wide(row, i, ln, big);
+            } else {
+                r = row_moments_wide(row, i, ln, big);
+                wide = __any_sync(0xffffffffu, big);
+            }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 r.a0 += shfl_xor_u128(r.a0, o);
