@@ -244,8 +244,12 @@ __global__ void __launch_bounds__(256, 1) k_sweep_spec(const SweepArgs a, uint32
             return true;
         });
     } else {
-        // lanes without a chain never accept (their E_Delta stays 3)
-        const bool store = cs.active;
+        // Lanes without a chain never accept (their E_Delta stays 3).  The compiler
+        // must not see that this is cs.active: it then splits the scan by it
+        // (L = 72, 16384 chains: 1.40 ms a launch instead of 1.31).
+        uint32_t on = cs.active;
+        asm("" : "+r"(on));
+        const bool store = on != 0;
         ChainState st;
         st.E = cs.active ? a.edel[cs.chain] : 3;
         st.EJ = cs.active ? a.ej[cs.chain] : 0;
