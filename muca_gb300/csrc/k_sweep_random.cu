@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(256) k_sweep_random(const RandomArgs a, uint32
         }
     }
     const float band = stage_differences(w64, N, u) + (float)a.log_eps;
-    if (tid == 0) u[-1] = 0.0f;
+    if (tid == 0) u[-1] = u[N + 1] = 0.0f;  // (u[N + 1]: read by lanes without a chain)
     for (uint32_t i = tid; i <= N; i += nt) histS[i] = 0u;
     if (LAT_SMEM) asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();

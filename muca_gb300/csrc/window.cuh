@@ -305,7 +305,8 @@ struct Feed {
                 const uint32_t k = (b % kFeedSlots) * 4u + off + i;
                 a.l[i] = *reinterpret_cast<const float *>(ring + (k / 4u % kFeedSlots) * 512u + k % 4u * 4u);
             }
-            a.dn = __funnelshift_r(d, dir((b + 2u) % kFeedSlots), 4u * off) & 0x11111111u;
+            // the third group only where it is used (and so drawn, see ready)
+            a.dn = __funnelshift_r(d, off ? dir((b + 2u) % kFeedSlots) : 0u, 4u * off) & 0x11111111u;
         }
     }
 };
