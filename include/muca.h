@@ -209,8 +209,9 @@ muca_status muca_set_wait_limit(muca_ctx *ctx, uint64_t cycles);
  * Nothing faults and every wait stays bounded.
  * MUCA_HOOK_FLUSH_ROWS: the windowed sweep flushes its shared u32 histogram
  * bins (production: sends the chains' 32-bit counts) into the device histogram
- * before every row it records, the path a launch takes when one could otherwise
- * reach 2^32 (results are the same bit for bit).
+ * before every row it records, and the random-site sweep every eight attempts:
+ * the path a launch takes when one could otherwise reach 2^32 (results are the
+ * same bit for bit).
  * MUCA_HOOK_AGED_RUN: the windowed sweep of production records as if every
  * chain had already spent MUCA_AGED_RUN attempts in the bin it starts
  * recording in, close to where a 32-bit count ends; the histogram has that many

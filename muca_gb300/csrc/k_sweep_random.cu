@@ -75,7 +75,9 @@ constexpr uint32_t kRndD4_0 = 0x00040800u, kRndD4_1 = 0x00000804u;  // 4 dDel + 
 constexpr uint32_t kRndVX_0 = 0x00020301u, kRndVX_1 = 0x00030102u;  // old code ^ new code
 constexpr uint32_t kRndSel = 0x7330u;
 
-template <int R, bool LAT_SMEM>
+// SEGMENT: groups between two flushes of the u32 bins (a constant: read from the
+// arguments it cost 3 % of the sweep).
+template <int R, bool LAT_SMEM, uint32_t SEGMENT>
 __global__ void __launch_bounds__(256) k_sweep_random(const RandomArgs a, uint32_t cpb, uint32_t pitch)
 {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -270,7 +272,7 @@ __global__ void __launch_bounds__(256) k_sweep_random(const RandomArgs a, uint32
     };
     auto run = [&](unsigned long long n, auto rec) {
         while (n >= 4ull) {
-            const uint32_t m = n < 1ull << 22 ? (uint32_t)n / 4u : 1u << 20;
+            const uint32_t m = n < 4ull * SEGMENT ? (uint32_t)n / 4u : SEGMENT;
 #pragma unroll 2
             for (uint32_t i = 0; i < m; ++i) group(4u, rec, std::false_type{});
             n -= 4ull * m;
@@ -298,10 +300,12 @@ template <int R, bool LS>
 static cudaError_t launch_random_one(const RandomArgs &a, uint32_t cpb, uint32_t pitch, uint32_t blocks, size_t smem,
                                      size_t smem_limit, cudaStream_t s)
 {
-    const cudaError_t e = cudaFuncSetAttribute(k_sweep_random<R, LS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem_limit);
+    // (the test hook's short segments)
+    void (*const kern)(const RandomArgs, uint32_t, uint32_t) =
+        (a.hooks & kHookFlushRows) ? k_sweep_random<R, LS, 2u> : k_sweep_random<R, LS, 1u << 20>;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_limit);
     if (e != cudaSuccess) return e;
-    k_sweep_random<R, LS><<<blocks, (cpb + 31u) / 32u * 32u, smem, s>>>(a, cpb, pitch);
+    kern<<<blocks, (cpb + 31u) / 32u * 32u, smem, s>>>(a, cpb, pitch);
     return cudaGetLastError();
 }
 

@@ -208,6 +208,7 @@ RandomArgs random_args(muca_ctx *c, uint32_t iter, uint32_t seed, uint64_t therm
     a.nup = nup;
     a.logf_tab = c->d_logf_tab;
     a.dyn = nullptr;
+    a.hooks = c->hooks;
     // muca_set_log_bracket widens either bound
     a.log_eps = c->d_logf_tab ? (c->log_eps_table > c->log_eps ? c->log_eps_table : c->log_eps) : c->log_eps;
     return a;

@@ -48,7 +48,7 @@ constexpr long long kWaitCyclesDefault = 1ll << 34;
 constexpr uint32_t kHookSilentProducer = 1u;
 // kHookFlushRows: the windowed sweep flushes its shared u32 bins (production:
 // sends the chains' 32-bit counts) before every recorded row, as a launch that
-// could fill one does
+// could fill one does; the random-site sweep flushes its bins every two groups
 constexpr uint32_t kHookFlushRows = 2u;
 // kHookNoCluster: the weight updates run as on a device that has no place for a
 // cluster
@@ -113,6 +113,7 @@ struct RandomArgs {
     // bound on |fast_logf(u) - log(u)| over every u01fixedpt<float> value, log
     // being logf_tab's values (when given) or CUDA's logf, with a safety factor
     double log_eps;
+    uint32_t hooks;  // as SweepArgs::hooks
 };
 // Worst case of |fast_logf(u) - tab[k]| over u = (2k+1) 2^-24, k < 2^23 (exhaustive, on the device).
 cudaError_t measure_table_bracket(const float *tab, float *max_abs_err, cudaStream_t s);
