@@ -23,8 +23,10 @@ INCLUDE = os.path.join(ROOT, "include")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2", "-I", INCLUDE,
                      "--expt-relaxed-constexpr", "-Xptxas", "-warn-spills"]
-CU_SOURCES = ["k_batch.cu", "k_win_weight.cu", "k_win_produce.cu", "k_sweep.cu", "k_sweep_random.cu", "k_lattice.cu", "k_weights.cu", "k_observables.cu", "k_bench.cu",
-              "k_mlp.cu", "muca_api.cu", "muca_batch.cu", "muca_mlp.cu"]
+# the longest compilations first
+CU_SOURCES = ["k_win_produce.cu", "k_batch_fits7.cu", "k_batch_fits10.cu", "k_win_weight.cu", "k_batch_place7.cu",
+              "k_batch_place10.cu", "k_sweep_random.cu", "k_sweep.cu", "k_bench.cu", "k_batch.cu", "k_lattice.cu",
+              "k_weights.cu", "k_observables.cu", "k_mlp.cu", "muca_api.cu", "muca_batch.cu", "muca_mlp.cu"]
 CLI_SOURCES = {"multigpu_weight": "multigpu_weight.cpp", "produce_gpu": "produce_gpu.cpp"}
 
 

@@ -3,7 +3,7 @@
 // Many (L, beta) instances of uneven size advance one weight iteration
 // together: a prep kernel clears the histograms of the instances still
 // running, one persistent sweep kernel works through the list of chain
-// blocks of all instances, and a cluster of blocks per instance applies the
+// blocks of all instances, and a cluster or a block per instance applies the
 // statistics, the schedule and the weight update (k_weights.cu).  The three
 // launches of an iteration are captured into a CUDA graph by the host
 // (muca_batch.cu) and replayed.
@@ -14,8 +14,9 @@
 // the histogram may go straight to the u64 device histogram, which frees the
 // shared memory of the u32 bins for more blocks per SM.  Work is fetched by
 // an atomic counter over items sorted by decreasing cost, so the large
-// lattices start first and the small ones fill the tail.
-#include "window.cuh"
+// lattices start first and the small ones fill the tail.  The kernel is in
+// k_batch_sweep.cuh, its instances in k_batch_fits*.cu and k_batch_place*.cu.
+#include "k_batch_sweep.cuh"
 
 namespace muca {
 
@@ -33,56 +34,6 @@ __global__ void k_batch_prep(const BatchInst *__restrict__ insts, uint32_t *__re
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) h[i] = 0ull;
 }
 
-// FEED (shapes of one or two warps of chains per SM): as many warps more draw
-// for those that walk, see window.cuh; their rings end the shared memory.
-template <int R, int LAT, bool HS, bool FEED = false>
-__global__ void __launch_bounds__(256, 1) k_batch_sweep(const BatchInst *__restrict__ insts,
-                                                         const BatchItem *__restrict__ items, uint32_t n_items,
-                                                         uint32_t *__restrict__ next_item, uint32_t cpb,
-                                                         uint32_t smem_bytes)
-{
-    extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ uint32_t s_item;
-    __shared__ float s_btab[kBetaTab];
-    const uint32_t feed_off = smem_bytes - (FEED ? (cpb + 31u) / 32u * kFeedBytes : 0u);
-    for (;;) {
-        if (threadIdx.x == 0) s_item = atomicAdd(next_item, 1u);
-        __syncthreads();
-        const uint32_t it = s_item;
-        if (it >= n_items) return;  // uniform: every thread read the same item
-        const BatchItem item = items[it];
-        const BatchInst *I = insts + item.inst;
-        const SweepArgs a = I->a;
-        uint32_t iter;
-        unsigned long long nup;
-        if (launch_params(a, iter, nup)) {  // the instance is still running
-            // -beta dE by dE + 8, then beta times the neighbour spin sum by code sum
-            if (threadIdx.x < kBetaTab)
-                s_btab[threadIdx.x] = I->btab[threadIdx.x < 17 ? threadIdx.x : 29 - threadIdx.x];
-            // s_btab is read only after the block barrier inside the sweep's prologue
-            if (LAT == kLatShared) {
-                win_sweep_block<kModeWeight, R, true, HS, true>(a, smem, cpb, item.blk, iter, nup, s_btab);
-            } else {
-                // uniform per item: the lattice joins the weights (and bins) in
-                // shared memory when all fit in the launch's allocation
-                // (kLatWhereFits); otherwise it stays in global memory, behind
-                // a four-row ring per lane where that fits
-                const size_t base = smem_weights_bytes(kModeWeight, a.N) + (HS ? smem_hist_bytes(kModeWeight, a.N) : 0);
-                if (LAT == kLatWhereFits && base + (size_t)a.L * a.WPR * 4u * cpb <= feed_off)
-                    win_sweep_block<kModeWeight, R, true, HS, true, false, true, false, FEED>(a, smem, cpb, item.blk, iter, nup,
-                                                                                             s_btab, feed_off);
-                else if (a.L % 4 == 0 && a.WPR <= 8 && base + ring_bytes(a.L, cpb) <= feed_off)
-                    win_sweep_block<kModeWeight, R, false, HS, true, true, true, false, FEED>(a, smem, cpb, item.blk, iter, nup,
-                                                                                             s_btab, feed_off);
-                else
-                    win_sweep_block<kModeWeight, R, false, HS, true, false, true, false, FEED>(a, smem, cpb, item.blk, iter, nup,
-                                                                                              s_btab, feed_off);
-            }
-        }
-        __syncthreads();
-    }
-}
-
 cudaError_t launch_batch_prep(const BatchInst *insts, uint32_t n_inst, uint32_t *next_item, uint32_t *running,
                               cudaStream_t s)
 {
@@ -97,27 +48,19 @@ size_t batch_sweep_smem(uint32_t L, uint32_t cpb, bool lat_smem, bool hist_smem,
            (lat_smem ? (size_t)L * WPR * 4 * cpb : (row_ring ? ring_bytes(L, cpb) : 0));
 }
 
-using BatchKernel = void (*)(const BatchInst *, const BatchItem *, uint32_t, uint32_t *, uint32_t, uint32_t);
-
-template <int R, int LAT>
-static BatchKernel batch_kernel_lat(bool hist_smem)
-{
-    return hist_smem ? k_batch_sweep<R, LAT, true> : k_batch_sweep<R, LAT, false>;
-}
-
 template <int R>
-static BatchKernel batch_kernel_r(uint32_t lat, bool hist_smem)
+static BatchKernel batch_kernel_r(uint32_t lat, bool hist_smem, bool feed)
 {
-    return lat == kLatWhereFits ? batch_kernel_lat<R, kLatWhereFits>(hist_smem)
-         : lat == kLatShared    ? batch_kernel_lat<R, kLatShared>(hist_smem)
-                                : batch_kernel_lat<R, kLatGlobal>(hist_smem);
+    return lat == kLatWhereFits ? batch_kernel_of<R, kLatWhereFits>(hist_smem, feed)
+         : lat == kLatShared    ? batch_kernel_of<R, kLatShared>(hist_smem, false)
+                                : batch_kernel_of<R, kLatGlobal>(hist_smem, false);
 }
 
 static BatchKernel batch_kernel(int rounds, uint32_t lat, bool hist_smem, bool feed)
 {
     // where all lattices fit, "where it fits" is "in shared memory"
-    if (feed) return rounds == 10 ? k_batch_sweep<10, kLatWhereFits, true, true> : k_batch_sweep<7, kLatWhereFits, true, true>;
-    return rounds == 10 ? batch_kernel_r<10>(lat, hist_smem) : batch_kernel_r<7>(lat, hist_smem);
+    if (feed) lat = kLatWhereFits;
+    return rounds == 10 ? batch_kernel_r<10>(lat, hist_smem, feed) : batch_kernel_r<7>(lat, hist_smem, feed);
 }
 
 // Every launch raises the kernel's limit to all that a block may have: a limit
