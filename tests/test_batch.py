@@ -251,3 +251,18 @@ def test_batch_trivial_update_costs_no_more_than_the_recursion(muca):
             return (best[1] - best[0]) / 256
         trivial, recursion = per_iteration(muca.UPDATE_TRIVIAL), per_iteration(muca.UPDATE_RECURSION)
     assert trivial <= 1.25 * recursion, (trivial, recursion)
+
+
+@pytest.mark.gpu
+def test_global_bins_cost_about_as_much_as_shared_ones(muca):
+    """One warp of chains per SM sub-partition, lattices behind the row ring: a
+    window's reductions to the device histogram fill the latency of its scan, so
+    they may cost a third of an iteration, not more."""
+    insts = [(72, 256, 1.5, k) for k in range(64)]
+    t = []
+    for hist in (1, 0):
+        with muca.Batch(insts, shape=(128, 0, hist)) as b:
+            def run(n):
+                return min(b.run(starting_sweeps=1, max_iter=n, graph_iters=2, d_kl_max=1e-30)[1] for _ in range(3))
+            t.append((run(10) - run(2)) / 8)
+    assert t[1] <= 1.33 * t[0], t
