@@ -498,14 +498,17 @@ __global__ void __launch_bounds__(kUpdMultiThreads) k_upd_apply(unsigned long lo
 // between them, the partial results read from the other blocks' shared memory
 // and the bins held in registers, and forms the updated weights while one
 // thread keeps the books.  What bounds it is the latency of its FP64 divisions
-// and logarithms (FP64 issues slowly on this GPU) and of the barriers.  Every bin
-// visited, back to back in a stream / in a graph, against the three launches
-// (whose cost does not depend on the size): N = 256: 16.4/14.7 us for 22.5/15.7,
-// N = 3969: 17.4/15.1 for 22.5/15.9, N = 4096: 20.5/17.8, N = 4356..8100:
-// 22.6..23.5/21.1: a second bin per thread costs more than the launches saved, so
-// from 4097 bins the three launches with their 64 SMs serve.
+// and logarithms (FP64 issues slowly on this GPU) and of the barriers.  Whole
+// iterations of 4096 chains with few attempts, against the three launches (a
+// third of the bins visited): host-buffer calls 90 us for 102 at N = 4096, 103
+// for 113 at 5184, 124 for 129 at 8100; runs in a graph 55.7 for 58.4, 66.2 for
+// 68.4 and 88.7 for 89.0 an iteration.  The update alone back to back, every bin
+// visited: 16.4 for 22.5 us at N = 256, 17.4 at 3969, 23.0 at 5184, 23.5 at 8100
+// (and in a graph 21.1 for 15.9 from two bins per thread on, where nothing lies
+// between the updates).  Above 8191 bins the three launches with their 64 SMs
+// stay.
 constexpr uint32_t kClusterBlocks = 16, kClusterThreads = 256;
-constexpr int kClusterPer = 1;  // bins per thread
+constexpr int kClusterPer = 2;  // bins per thread at most
 constexpr uint32_t kClusterBins = kClusterBlocks * kClusterThreads * kClusterPer;
 
 __device__ __forceinline__ void cluster_sync()

@@ -179,7 +179,7 @@ struct RecScratch {
 // stats of hist[0..N]; if rule >= 0 also updates lnw (FP64) / w32 (FP32 shadow)
 // (rule: 0 trivial, 1 trivial-cpu, 2 recursion with p_acc), the FP64 work over
 // kUpdBlocks blocks (the recursion's prefix as one block's segmented scan), or,
-// with `cluster` (update_cluster_fits), of up to 4096 bins and rules -1, 0 and 1
+// with `cluster` (update_cluster_fits), of up to 8191 bins and rules -1, 0 and 1
 // as one cluster launch.  `sc`: zero-initialised once.
 cudaError_t launch_weight_update(unsigned long long *hist, uint32_t N, double *lnw, float *w32,
                                  double *p_acc, int rule, HistStatsDev *stats, cudaStream_t s, bool cluster,

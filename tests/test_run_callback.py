@@ -33,8 +33,8 @@ def _stream(muca, e, rule, starting_M, max_iter, seen):
     return res
 
 
-# every form of the update: one cluster (L = 16, 63), several launches (L = 64,
-# 96), the recursion; and the random-site algorithm's sweep
+# every form of the update: one cluster (L = 16, 63, 64), several launches
+# (L = 96), the recursion; and the random-site algorithm's sweep
 @pytest.mark.parametrize("L,rule,algo", [(16, 0, 0), (16, 1, 0), (16, 2, 0), (63, 0, 0), (64, 0, 0), (96, 0, 0),
                                          (96, 2, 0), (12, 1, 1)])
 def test_callback_sees_the_iterations_counts(muca, L, rule, algo):
