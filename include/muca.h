@@ -286,7 +286,9 @@ muca_status muca_iterate_host(muca_ctx *ctx, const double *lnw_in, uint32_t iter
 muca_status muca_weight_run(muca_ctx *ctx, const muca_run_opts *opts, muca_run_result *res,
                             muca_iter_record *recs, size_t cap);
 /* Same, calling cb(record, user) on the host after every iteration (the
- * per-iteration log line of :439). */
+ * per-iteration log line of :439).  While cb runs the context's histogram holds
+ * that iteration's counts; it is cleared before the next sweep, whatever cb
+ * leaves there. */
 typedef void (*muca_iter_callback)(const muca_iter_record *rec, void *user);
 muca_status muca_weight_run_stream(muca_ctx *ctx, const muca_run_opts *opts, muca_run_result *res,
                                    muca_iter_callback cb, void *user);
@@ -307,8 +309,8 @@ muca_status muca_compute_observables(muca_ctx *ctx, double beta, double delta, m
  * device buffers owned by the caller; no context.  The call allocates
  * nothing: for callers that must not see a device allocation (a scheduler
  * owning HBM through its own pool and budget; a process that only reweights
- * histograms it holds).  Its scratch is a fixed device array of 304 x 4
- * doubles inside the library (the partials of a fixed 304-block grid; the
+ * histograms it holds).  Its scratch is a fixed device array of 152 x 4
+ * doubles inside the library (the partials of a grid of at most 152 blocks; the
  * size does not depend on L), whose address is looked up on the first call
  * per device and cached; make that first call before any stream capture,
  * since it may load the module.  The cached address belongs to the device's

@@ -240,8 +240,9 @@ cudaError_t launch_batch_prep(const BatchInst *insts, uint32_t n_inst, uint32_t 
 enum BatchLattice : uint32_t { kLatGlobal = 0, kLatShared = 1, kLatWhereFits = 2 };
 // Persistent sweep over `items` (fetched through *next_item) with chain
 // blocks of cpb chains; lat (BatchLattice) / hist_smem select the
-// shared-memory placement.  grid blocks of roundup32(cpb) threads and
-// `smem` bytes.
+// shared-memory placement.  grid blocks of roundup32(cpb) threads (with `feed`,
+// drawing warps, twice that) and `smem` bytes; the kernel's limit is raised to
+// smem_limit.
 cudaError_t launch_batch_sweep(const BatchInst *insts, const BatchItem *items, uint32_t n_items, uint32_t *next_item,
                                uint32_t cpb, int rounds, uint32_t lat, bool hist_smem, bool feed, uint32_t grid,
                                size_t smem, size_t smem_limit, cudaStream_t s);
@@ -251,8 +252,7 @@ size_t batch_feed_smem(uint32_t cpb);
 // with its lattice, or without it (then optionally with its four-row ring).
 size_t batch_sweep_smem(uint32_t L, uint32_t cpb, bool lat_smem, bool hist_smem, bool row_ring = false);
 // Blocks of the batch sweep that fit on one SM with `smem` bytes each; also
-// sets the kernel's shared-memory limit to `smem` (call before any capture).
-// The launch with that shape needs no further attribute call.
+// raises the kernel's shared-memory limit to smem_limit, as every launch does.
 cudaError_t batch_sweep_occupancy(uint32_t cpb, int rounds, uint32_t lat, bool hist_smem, bool feed, size_t smem,
                                   size_t smem_limit, int *blocks);
 // Sets the update kernels' shared-memory limit (call before any capture).
